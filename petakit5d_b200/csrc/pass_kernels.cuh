@@ -6,6 +6,7 @@
 // registers between the inverse and the forward transform.
 #pragma once
 #include "fft_ct.cuh"
+#include "gen_engine.cuh"
 #include "pk_internal.h"
 
 #define PK_EPS_F 2.220446049250313e-16f  // single(eps) = 2^-52
@@ -348,8 +349,14 @@ __host__ __device__ inline int y_aux_arrays(int mode) {
     }
 }
 
-template <int P, int MODE, int TP = PK_TILE_POINTS>
-__global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
+// Slots of one buffer of a row tile of the mixed-radix engine: `lines` complex lines of up to `len` points
+// (even, so that what follows stays on a 16-byte boundary).
+__host__ __device__ inline int gen_y_slots(int lines, int len) { return (lines * len + 1) & ~1; }
+
+// GEN (P = 0): 1 and 2 run lengths without a plan on the mixed-radix / chirp engine (gen_engine.cuh; 2: with
+// its radices above 16), 0 on the in-place run-time engine.
+template <int P, int MODE, int TP = PK_TILE_POINTS, int GEN = 0>
+__global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
                                                      int nvol, int) {
     constexpr int mode = MODE;   // one kernel per mode: only that mode's code is in the kernel
     extern __shared__ float2 smem[];
@@ -363,18 +370,34 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
     const int L = P == 0 ? d.Ly : plan_lines_y(kPlans[P].n, TP);
     const bool odd = d.odd;
     const int Py = d.Py, ny = d.ny;
-    // shared memory: tw[tw_slots(M)] | twrc[M+1] (even ny) | buf[padded L*M] | nyq[L] | aux0[L*M] | aux1[L*M]
+    // lengths without a plan run the mixed-radix / chirp engine on two buffers of its L points a line
+    const GenAxis* const G = P == 0 ? A.gen : nullptr;
+    // odd ny: the odd rows of a pair travel as the imaginary part of the even ones (two real transforms in one)
+    const bool pairs = GEN && odd;
+    const int lines = pairs ? (L + 1) / 2 : L;   // complex lines of a full tile
+    const int bufn = GEN ? gen_y_slots(lines, odd ? max(G->L, M + 1) : G->L) : padded_size(L * M);
+    const pkgen::FastDiv divM(M), divPy(Py);
+    auto line_of = [&](int idx) { return P == 0 ? divM(idx) : idx / M; };
+    auto slot = [](int a) { return GEN ? a : pad(a); };   // the tile's word of element a
+    // shared memory: tw[tw_slots(M)] (not with G) | twrc[M+1] (even ny) | buf[padded L*M] | second buf (G) | nyq[L]
+    // | aux0[L*M] | aux1[L*M]
     float2* tw = smem;
-    float2* twrc = smem + tw_slots(M);
+    float2* twrc = smem + (G ? 0 : tw_slots(M));
     float2* buf = twrc + (odd ? 0 : M + 1);
-    float2* nyq = buf + padded_size(L * M);
+    float2* const gb0 = buf;
+    float2* const gb1 = buf + bufn;
+    float2* nyq = buf + (G ? 2 : 1) * bufn;
     float2* aux0 = nyq + L;
-    float2* aux1 = aux0 + L * M;
+    const int auxn = pairs ? gen_y_slots(L, M) / 2 : L * M;   // pairs of odd rows: one float a voxel
+    float2* aux1 = aux0 + auxn;
+    auto aux = [&](const float2* p, int idx) {
+        return pairs ? make_float2(reinterpret_cast<const float*>(p)[idx], 0.f) : p[idx];
+    };
     const long long row0 = (long long)lb * L;
     const int Lc = (int)min((long long)L, d.nrows - row0);
     const bool spec_in = mode_from_spec(mode), spec_out = mode_to_spec(mode);
-    if (!PK_SMEM_OK(d, sizeof(float2) * (tw_slots(M) + (odd ? 0 : M + 1) + padded_size(L * M) + L +
-                                         (size_t)y_aux_arrays(mode) * L * M), 1) ||
+    if (!PK_SMEM_OK(d, sizeof(float2) * ((G ? 0 : tw_slots(M)) + (odd ? 0 : M + 1) + (G ? 2 : 1) * bufn + L +
+                                         (size_t)y_aux_arrays(mode) * auxn), 1) ||
         !PK_IN(d, row0 < d.nrows && Lc >= 1, 2))
         return;   // uniform over the CTA, before any barrier
     if constexpr (mode == Y_FINAL || mode == Y_RLFINAL) {
@@ -388,17 +411,17 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
         if (P > 0 && !odd) {
             // Py = M + 1: bins 0..M-1 of each row into the tile, bin M (Nyquist) aside
             for (int idx = tid; idx < Lc * M; idx += NT) {
-                const int l = idx / M, k = idx - l * M;
-                if (PK_IN(d, k < Pp, 11)) cp8(&buf[pad(idx)], S0 + l * Pp + k);
+                const int l = line_of(idx), k = idx - l * M;
+                if (PK_IN(d, k < Pp, 11)) cp8(&buf[slot(idx)], S0 + l * Pp + k);
             }
             for (int l = tid; l < Lc; l += NT)
                 if (PK_IN(d, M < Pp, 11)) cp8(&nyq[l], S0 + l * Pp + M);
         } else {
             const int nin = Lc * Py;
             for (int idx = tid; idx < nin; idx += NT) {
-                const int l = idx / Py, k = idx - l * Py;
+                const int l = divPy(idx), k = idx - l * Py;
                 if (!odd && k == M) cp8(&nyq[l], S0 + l * Pp + k);
-                else cp8(&buf[pad(l * M + k)], S0 + l * Pp + k);
+                else cp8(pairs ? &gb1[idx] : &buf[slot(l * M + k)], S0 + l * Pp + k);
             }
         }
     }
@@ -424,21 +447,21 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
     if (mode == Y_PRE && !raw_sync) {
         if (d.raw_type == PK_F32 && wide_ok && (reinterpret_cast<uintptr_t>(d.raw) & 15) == 0) {
             for (int idx = 2 * tid; idx < nvox; idx += 2 * NT) {
-                const int l = idx / M, k = idx - l * M;
+                const int l = line_of(idx), k = idx - l * M;
                 cp16(&aux0[idx], (const float*)d.raw + v0 + (long long)l * ny + 2 * k);
             }
         } else {
             for (int idx = tid; idx < nvox; idx += NT) {
-                const int l = idx / M, k = idx - l * M;
+                const int l = line_of(idx), k = idx - l * M;
                 const long long vi = v0 + (long long)l * ny + (odd ? k : 2 * k);
                 if (d.raw_type == PK_U16) cp4(&aux0[idx], (const uint16_t*)d.raw + vi);
                 else if (!odd) cp8(&aux0[idx], (const float*)d.raw + vi);
-                else cp4(&aux0[idx], (const float*)d.raw + vi);
+                else cp4(pairs ? (float*)aux0 + idx : (float*)&aux0[idx], (const float*)d.raw + vi);
             }
         }
     } else if (pa0 && wide_ok && ((reinterpret_cast<uintptr_t>(pa0) | reinterpret_cast<uintptr_t>(pa1)) & 15) == 0) {
         for (int idx = 2 * tid; idx < nvox; idx += 2 * NT) {
-            const int l = idx / M, k = idx - l * M;
+            const int l = line_of(idx), k = idx - l * M;
             const long long vi = v0 + (long long)l * ny + 2 * k;
             if (!PK_IN(d, vi + 3 < d.nrows * (long long)ny, 12)) continue;
             cp16(&aux0[idx], pa0 + vi);
@@ -446,20 +469,21 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
         }
     } else if (pa0) {
         for (int idx = tid; idx < nvox; idx += NT) {
-            const int l = idx / M, k = idx - l * M;
+            const int l = line_of(idx), k = idx - l * M;
             const long long vi = v0 + (long long)l * ny + (odd ? k : 2 * k);
             if (!odd) {
                 cp8(&aux0[idx], pa0 + vi);
                 if (pa1) cp8(&aux1[idx], pa1 + vi);
             } else {
-                cp4(&aux0[idx], pa0 + vi);
-                if (pa1) cp4(&aux1[idx], pa1 + vi);
+                cp4(pairs ? (float*)aux0 + idx : (float*)&aux0[idx], pa0 + vi);
+                if (pa1) cp4(pairs ? (float*)aux1 + idx : (float*)&aux1[idx], pa1 + vi);
             }
         }
     }
     cp_commit();
     // tables (plain loads; they stay in L2)
-    for (int i = tid; i < (P == 0 ? M : plan_tw_size(P)); i += NT) tw[i] = A.tw[i];
+    if (!G)
+        for (int i = tid; i < (P == 0 ? M : plan_tw_size(P)); i += NT) tw[i] = A.tw[i];
     if (!odd)
         for (int i = tid; i <= M; i += NT) twrc[i] = d.tw_rc[i];
     double acc0 = 0.0, acc1 = 0.0;
@@ -473,30 +497,46 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
         if (!odd) {
             const int half = M / 2 + 1;
             const int np = Lc * half;
+            const pkgen::FastDiv divH(half);
             for (int p = tid; p < np; p += NT) {
-                const int l = p / half, k = p - l * half;
-                const float2 xk = buf[pad(l * M + k)];
-                const float2 xm = k == 0 ? nyq[l] : buf[pad(l * M + (M - k))];
+                const int l = P == 0 ? divH(p) : p / half, k = p - l * half;
+                const float2 xk = buf[slot(l * M + k)];
+                const float2 xm = k == 0 ? nyq[l] : buf[slot(l * M + (M - k))];
                 {
                     const float2 a = xk, b = conjf2(xm);
                     float2 w = twrc[k];
                     w.y = -w.y;
                     const float2 s2 = cadd(a, b), t2 = cmul(csub(a, b), w);
-                    buf[pad(l * M + k)] = make_float2(s2.x - t2.y, s2.y + t2.x);
+                    buf[slot(l * M + k)] = make_float2(s2.x - t2.y, s2.y + t2.x);
                 }
                 if (k != 0 && 2 * k != M) {
                     const float2 a = xm, b = conjf2(xk);
                     float2 w = twrc[M - k];
                     w.y = -w.y;
                     const float2 s2 = cadd(a, b), t2 = cmul(csub(a, b), w);
-                    buf[pad(l * M + (M - k))] = make_float2(s2.x - t2.y, s2.y + t2.x);
+                    buf[slot(l * M + (M - k))] = make_float2(s2.x - t2.y, s2.y + t2.x);
                 }
+            }
+        } else if (pairs) {
+            // Z[k] = X0[k] + i X1[k], the bins past the half from the conjugates
+            const int Lp = (Lc + 1) / 2;
+            for (int p = tid; p < Lp * M; p += NT) {
+                const int l = line_of(p), k = p - l * M;
+                const int kk = k < Py ? k : ny - k;
+                float2 a = gb1[2 * l * Py + kk];
+                float2 b = 2 * l + 1 < Lc ? gb1[(2 * l + 1) * Py + kk] : make_float2(0.f, 0.f);
+                if (k >= Py) {
+                    a.y = -a.y;
+                    b.y = -b.y;
+                }
+                buf[slot(p)] = make_float2(a.x - b.y, a.y + b.x);
             }
         } else {
             const int nf = Lc * (ny - Py);
+            const pkgen::FastDiv divF(ny - Py > 0 ? ny - Py : 1);
             for (int p = tid; p < nf; p += NT) {
-                const int l = p / (ny - Py), k = Py + (p - l * (ny - Py));
-                buf[pad(l * M + k)] = conjf2(buf[pad(l * M + (ny - k))]);
+                const int l = divF(p), k = Py + (p - l * (ny - Py));
+                buf[slot(l * M + k)] = conjf2(buf[slot(l * M + (ny - k))]);
             }
         }
         __syncthreads();
@@ -651,29 +691,52 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
         }
     }
     if (!fused) {
-    if (spec_in) fft_y<P, true, TP>(buf, A, tw, L, tid);
+    pkgen::GenEdge ge{};
+    ge.sc = 1.f;
+    if (spec_in) {
+        if constexpr (GEN > 0) {
+            ge.inv = 1;
+            buf = pkgen::gen_transform<false, GEN == 2>(G, buf, gb0, gb1, pairs ? (Lc + 1) / 2 : Lc, 0, ge, tid, NT, [] {}, [] {});
+            ge.inv = 0;
+        } else {
+            fft_y<P, true, TP>(buf, A, tw, L, tid);
+        }
+    }
     cp_wait<0>();
     __syncthreads();
 
     // ---- per-voxel phase (descriptor fields in registers: the loop stores to the volume's arrays)
     const VoxFields f(d);
     for (int idx = tid; idx < nvox; idx += NT) {
-        const int l = idx / M, k = idx - l * M;
+        const int l = line_of(idx), k = idx - l * M;
         const long long row = row0 + l;
         const int y = odd ? k : 2 * k;
         float2 out;
         if (mode == Y_PRE) {
-            out = pre_pair(f, raw_sync, odd, aux0[idx], row, y, zeros);
+            out = pre_pair(f, raw_sync, odd, aux(aux0, idx), row, y, zeros);
         } else {
-            const float2 cval = spec_in ? buf[pad(idx)] : make_float2(0.f, 0.f);
-            out = voxel_pair(f, mode, cval, pa0 ? aux0[idx] : make_float2(0.f, 0.f), pa1 ? aux1[idx] : make_float2(0.f, 0.f),
-                             row, y, !odd, lam, acc0, acc1);
+            float2 cval = make_float2(0.f, 0.f);
+            if (spec_in) {
+                if (pairs) cval.x = reinterpret_cast<const float*>(&buf[slot((l >> 1) * M + k)])[l & 1];
+                else cval = buf[slot(idx)];
+            }
+            out = voxel_pair(f, mode, cval, pa0 ? aux(aux0, idx) : make_float2(0.f, 0.f),
+                             pa1 ? aux(aux1, idx) : make_float2(0.f, 0.f), row, y, !odd, lam, acc0, acc1);
         }
-        if (spec_out) buf[pad(idx)] = odd ? make_float2(out.x, 0.f) : out;
+        if (spec_out) {
+            if (pairs) reinterpret_cast<float*>(&buf[slot((l >> 1) * M + k)])[l & 1] = out.x;
+            else buf[slot(idx)] = odd ? make_float2(out.x, 0.f) : out;
+        }
     }
+    if (spec_out && pairs && (Lc & 1))   // no partner for the last row
+        for (int k = tid; k < M; k += NT) buf[slot((Lc >> 1) * M + k)].y = 0.f;
     if (spec_out) {
         __syncthreads();
-        fft_y<P, false, TP>(buf, A, tw, L, tid);
+        if constexpr (GEN > 0) {
+            buf = pkgen::gen_transform<false, GEN == 2>(G, buf, gb0, gb1, pairs ? (Lc + 1) / 2 : Lc, 0, ge, tid, NT, [] {}, [] {});
+        } else {
+            fft_y<P, false, TP>(buf, A, tw, L, tid);
+        }
     }
     }
 
@@ -684,8 +747,8 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
         if (P > 0 && !odd) {
             // X[k] = (Z[k] + Z*[M-k]) / 2 + W^k (Z[k] - Z*[M-k]) / 2i for k < M; X[M] from Z[0]
             auto split = [&](int l, int k) {
-                const float2 zk = buf[pad(l * M + k)];
-                const float2 zc = conjf2(buf[pad(l * M + (k == 0 ? 0 : M - k))]);
+                const float2 zk = buf[slot(l * M + k)];
+                const float2 zc = conjf2(buf[slot(l * M + (k == 0 ? 0 : M - k))]);
                 const float2 fe = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
                 const float2 df = csub(zk, zc);
                 const float2 fo = make_float2(0.5f * df.y, -0.5f * df.x);
@@ -694,19 +757,19 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
             if (M % 2 == 0 && (reinterpret_cast<uintptr_t>(S0) & 15) == 0) {
                 // two bins per thread, one 16-byte store (even M and row pitch keep the pairs aligned)
                 for (int idx = 2 * tid; idx < Lc * M; idx += 2 * NT) {
-                    const int l = idx / M, k = idx - l * M;
+                    const int l = line_of(idx), k = idx - l * M;
                     const float2 x0 = split(l, k), x1 = split(l, k + 1);
                     if (PK_IN(d, k + 1 < Pp, 14))
                         *reinterpret_cast<float4*>(S0 + l * Pp + k) = make_float4(x0.x, x0.y, x1.x, x1.y);
                 }
             } else {
                 for (int idx = tid; idx < Lc * M; idx += NT) {
-                    const int l = idx / M, k = idx - l * M;
+                    const int l = line_of(idx), k = idx - l * M;
                     S0[l * Pp + k] = split(l, k);
                 }
             }
             for (int l = tid; l < Lc; l += NT) {
-                const float2 zk = buf[pad(l * M)];
+                const float2 zk = buf[slot(l * M)];
                 const float2 zc = conjf2(zk);
                 const float2 fe = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
                 const float2 df = csub(zk, zc);
@@ -715,17 +778,22 @@ __global__ void __launch_bounds__(PK_THREADS, 3) k_y(const VolDesc* __restrict__
             }
         } else {
             for (int idx = tid; idx < nout; idx += NT) {
-                const int l = idx / Py, k = idx - l * Py;
+                const int l = divPy(idx), k = idx - l * Py;
                 float2 X;
                 if (!odd) {
-                    const float2 zk = buf[pad(l * M + (k == M ? 0 : k))];
-                    const float2 zc = conjf2(buf[pad(l * M + (k == 0 ? 0 : M - k))]);
+                    const float2 zk = buf[slot(l * M + (k == M ? 0 : k))];
+                    const float2 zc = conjf2(buf[slot(l * M + (k == 0 ? 0 : M - k))]);
                     const float2 fe = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
                     const float2 df = csub(zk, zc);
                     const float2 fo = make_float2(0.5f * df.y, -0.5f * df.x);  // (zk - zc) / (2i)
                     X = cadd(fe, cmul(twrc[k], fo));
+                } else if (pairs) {
+                    const float2 zk = buf[slot((l >> 1) * M + k)];
+                    const float2 zc = conjf2(buf[slot((l >> 1) * M + (k == 0 ? 0 : M - k))]);
+                    X = (l & 1) ? make_float2(0.5f * (zk.y - zc.y), 0.5f * (zc.x - zk.x))
+                                : make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
                 } else {
-                    X = buf[pad(l * M + k)];
+                    X = buf[slot(l * M + k)];
                 }
                 S0[l * Pp + k] = X;
             }
@@ -959,7 +1027,8 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
 constexpr int kYModes = Y_C2R + 1;
 
 // Entries [0, kNumPlans) hold the 4096-point-tile kernels, [kNumPlans + p] the small-tile kernels
-// of plan p (small_tile_plan(p)); a program step's plan id carries that offset.
+// of plan p (small_tile_plan(p)); a program step's plan id carries that offset.  The y entries of the plans
+// without small tiles, kNumPlans and kNumPlans + 1, hold the mixed-radix engine's kernels (GEN 1 and 2).
 struct KernelTable {
     void (*y[2 * kNumPlans][kYModes])(const VolDesc*, const int*, int, int);
     void (*xz[2 * kNumPlans])(const VolDesc*, const int*, int, int, int);
@@ -979,6 +1048,21 @@ struct RegisterY {
 };
 template <int P>
 struct RegisterY<P, kYModes> {
+    static void fill(KernelTable&) {}
+};
+
+static_assert(!small_tile_plan(0) && !small_tile_plan(1), "the mixed-radix y kernels take these entries");
+template <int GEN, int MD>
+struct RegisterYGen {
+    static void fill(KernelTable& t) {
+        auto fn = k_y<0, MD, PK_TILE_POINTS, GEN>;
+        t.y[kNumPlans + GEN - 1][MD] = fn;
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        RegisterYGen<GEN, MD + 1>::fill(t);
+    }
+};
+template <int GEN>
+struct RegisterYGen<GEN, kYModes> {
     static void fill(KernelTable&) {}
 };
 

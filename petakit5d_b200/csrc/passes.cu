@@ -26,6 +26,7 @@
 #include "pass_kernels.cuh"
 #include "pass_tma.cuh"
 #include "pass_conv3.cuh"
+#include "pass_gen.cuh"
 #include "pass_yreg.cuh"
 #include "pk_internal.h"
 #include "plans.h"
@@ -41,12 +42,15 @@ void pk_fill_kernels_f(pkpass::KernelTable& t);
 void pk_fill_kernels_g(pkpass::KernelTable& t);
 void pk_fill_kernels_h(pkpass::KernelTable& t);
 void pk_fill_kernels_i(pkpass::KernelTable& t);
+void pk_fill_kernels_g1(pkpass::KernelTable& t);
+void pk_fill_kernels_g2(pkpass::KernelTable& t);
 void pk_fill_tma_0(pkpass::TmaTable& t);
 void pk_fill_tma_1(pkpass::TmaTable& t);
 void pk_fill_tma_2(pkpass::TmaTable& t);
 void pk_fill_tma_3(pkpass::TmaTable& t);
 void pk_fill_conv3(std::vector<pkpass::Conv3Entry>& v);
 void pk_fill_yreg(pkpass::YregTable& t);
+void pk_fill_gen(pkpass::GenKernel& k);
 
 static int sm_count() {
     static int n = 0;
@@ -73,9 +77,16 @@ void pk_fill_all_kernels(pkpass::KernelTable& t) {
     pk_fill_kernels_g(t);
     pk_fill_kernels_h(t);
     pk_fill_kernels_i(t);
+    pk_fill_kernels_g1(t);
+    pk_fill_kernels_g2(t);
 }
 
 static size_t step_smem(int kind, int mode, const VolDesc& v) {
+    if (kind == PK_STEP_Y && v.ay.gen) {
+        const int lines = v.odd ? (v.Ly + 1) / 2 : v.Ly, len = v.odd ? std::max(v.ay.genL, v.M + 1) : v.ay.genL;
+        return sizeof(float2) * ((v.odd ? 0 : v.M + 1) + 2 * (size_t)pkpass::gen_y_slots(lines, len) + v.Ly +
+                                 (size_t)pkpass::y_aux_arrays(mode) * (v.odd ? pkpass::gen_y_slots(v.Ly, v.M) / 2 : v.Ly * v.M));
+    }
     if (kind == PK_STEP_Y)
         return sizeof(float2) * (tw_slots(v.M) + (v.odd ? 0 : v.M + 1) + padded_size(v.Ly * v.M) + v.Ly +
                                  (size_t)pkpass::y_aux_arrays(mode) * v.Ly * v.M);
@@ -152,6 +163,14 @@ const pkpass::YregTable* yreg_kernels() {
     return on ? &t : nullptr;
 }
 
+// The x / z kernels of lengths without a plan (pass_gen.cuh); null where they could not be set up.
+const pkpass::GenKernel& gen_kernel() {
+    static pkpass::GenKernel k{};
+    static std::once_flag once;
+    std::call_once(once, [] { pk_fill_gen(k); });
+    return k;
+}
+
 // A y step's descriptor the register-packing kernel can take: 512-voxel rows on the 4096-point
 // tiles, per-voxel inputs 16-byte aligned (bulk copies), the rolled kernel's fused-path conditions
 // (no padded / float64 raw input, no damping, scaling, mask or crop in the final pass).
@@ -192,12 +211,11 @@ EncodeTiledFn encode_tiled() {
 }
 
 // Tensor map of a half spectrum (S or an OTF) laid out [z][x][k] with row pitch Pp, as
-// {2 Py floats, nx, nz}, with the column-tile box of an x (axis 1) or z (axis 2) pass of plan p.
-bool encode_spec_map(CUtensorMap* m, const void* base, const VolDesc& d, int axis, int p, int T) {
+// {2 Py floats, nx, nz}, with the column-tile box of an x (axis 1) or z (axis 2) pass.
+// `rows`: elements of the transformed axis per box.
+bool encode_spec_box(CUtensorMap* m, const void* base, const VolDesc& d, int axis, int rows, int T) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc || !base || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
-    const int n = kPlans[p].n;
-    const int rows = pkpass::tma_box_rows(n);
     const cuuint64_t dims[3] = {(cuuint64_t)2 * d.Py, (cuuint64_t)d.nx, (cuuint64_t)d.nz};
     const cuuint64_t strides[2] = {(cuuint64_t)d.Pp * 8, (cuuint64_t)d.Pp * 8 * (cuuint64_t)d.nx};
     const cuuint32_t box[3] = {(cuuint32_t)(2 * T), (cuuint32_t)(axis == 1 ? rows : 1), (cuuint32_t)(axis == 2 ? rows : 1)};
@@ -212,6 +230,10 @@ bool encode_spec_map(CUtensorMap* m, const void* base, const VolDesc& d, int axi
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, promo,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool encode_spec_map(CUtensorMap* m, const void* base, const VolDesc& d, int axis, int p, int T) {
+    return encode_spec_box(m, base, d, axis, pkpass::tma_box_rows(kPlans[p].n), T);
 }
 
 // Index of a step's TMA kernel in the table, or -1 when the step keeps the register-IO kernels.
@@ -576,6 +598,39 @@ static void fuse_conv3(pk_ctx* ctx, PkProgram& prog) {
     prog.steps.swap(out);
 }
 
+// An x / z step of lengths without a compile-time plan: the generic TMA kernel when every volume has a
+// run-time plan with a tile that fits shared memory, else the in-place engine of k_xz.
+static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
+    s.gen = 0;
+    bool ok = gen_kernel().fn[0] && gen_kernel().fn[1];
+    int land = 0, work = 0, big = 0;
+    for (int i = 0; i < s.nvol && ok; i++) {
+        const VolDesc& d = prog.descs[s.desc_off + i];
+        const AxisDev& A = axis == 1 ? d.ax : d.az;
+        ok = A.gen && A.genT > 0 && encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
+        if (!ok) break;
+        land = std::max(land, A.gen_land);
+        work = std::max(work, A.gen_work);
+        big |= A.gen_big;
+    }
+    const size_t smem = pkpass::gen_smem(land, work);
+    if (!ok || smem > (size_t)226 * 1024) return;
+    int* pf = prog.prefix.data() + s.prefix_off;
+    for (int i = 0; i < s.nvol; i++) {
+        const VolDesc& d = prog.descs[s.desc_off + i];
+        const AxisDev& A = axis == 1 ? d.ax : d.az;
+        pf[i + 1] = pf[i] + (axis == 1 ? d.nz : d.nx) * ((d.Py + A.genT - 1) / A.genT);
+    }
+    s.grid = pf[s.nvol];
+    s.gen = 1 + big;
+    s.tma_smem = smem;
+    s.gen_land = land;
+    s.gen_work = work;
+    // resident CTAs: two or three by registers, fewer where their shared memory (and its 1 KB a CTA) does not fit
+    const int per_sm = std::max(1, std::min(big ? 2 : 3, (int)((size_t)228 * 1024 / (smem + 1024))));
+    s.tma_grid = std::min(s.grid, per_sm * sm_count());
+}
+
 void assign_tma(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
     fuse_conv3(ctx, prog);
     prog.maps.assign(prog.descs.size(), XZMaps());
@@ -603,9 +658,13 @@ void assign_tma(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
             }
             continue;
         }
+        const int axis = s.kind == PK_STEP_X ? 1 : 2;
+        if ((s.kind == PK_STEP_X || s.kind == PK_STEP_Z) && s.plan == 0 && s.grid > 0) {
+            assign_gen(prog, s, axis);
+            continue;
+        }
         const int idx = tma_index(s);
         if (idx < 0 || s.grid == 0) continue;
-        const int axis = s.kind == PK_STEP_X ? 1 : 2;
         const pkpass::TmaTable* t = tma_kernels();
         int* pf = prog.prefix.data() + s.prefix_off;
         const int var = choose_variant(ctx, prog, s, idx, st);
@@ -808,6 +867,208 @@ pk_status pk_get_axis_table(pk_ctx* ctx, int n, const float2** out) {
     return PK_OK;
 }
 
+// ---- run-time plans of lengths without a compile-time plan (gen_engine.cuh)
+namespace {
+
+// instructions of one butterfly of the engine's radices (counted from its source: adds, multiplies, fused)
+struct GenRadix { int r, cost; };
+constexpr GenRadix kGenRadices[] = {{16, 150}, {15, 190}, {13, 190}, {12, 112}, {11, 140}, {10, 100}, {9, 90},
+                                    {8, 56},   {7, 60},   {6, 40},   {5, 34},   {4, 16},   {3, 14},   {2, 4},
+                                    {17, 310}, {19, 380}, {23, 550}, {29, 860}, {31, 980}};
+
+// Columns of an x / z tile (n points a line, L in the stages): the widest power of two (16: whole 128-byte
+// lines; 32 on short lines, for the work of a tile) whose three buffers let three CTAs share an SM, at least
+// 4 (one 32-byte sector of the spectrum) where that fits one CTA, else 2; 0 where nothing fits.  Timed on the
+// 270-long z pass of a 512 x 1140 x 270 volume: 16 columns at two CTAs an SM 1.07 ms, 8 at three 0.98 ms,
+// 4 at three 1.53 ms.
+int gen_tile(int n, int L, GenAxis* g) {
+    for (int T = L <= 64 ? 32 : 16; T >= 2; T /= 2) {
+        const int gran = T >= 16 ? 1 : 16 / T;   // box rows keep each box on a 128-byte boundary
+        g->L = L;
+        g->T = T;
+        for (g->nbox = (n + 255) / 256;; g->nbox++) {
+            g->rows = ((n + g->nbox - 1) / g->nbox + gran - 1) / gran * gran;
+            if (g->rows <= 256) break;
+        }
+        const size_t smem = pkpass::gen_smem(pkpass::gen_land(*g), pkpass::gen_work(*g));
+        if (smem <= (T > 4 ? (size_t)75 * 1024 : (size_t)226 * 1024)) {
+            for (g->lt = 0; (1 << g->lt) < T;) g->lt++;
+            return T;
+        }
+    }
+    g->T = g->rows = g->nbox = 0;
+    return 0;
+}
+
+// Instructions per point of a radix stage over `pts` points (by the counts above, plus the loads, stores,
+// twiddles and index arithmetic), with the threads that its last round leaves idle.
+double gen_stage_cost(const GenRadix& g, int pts, bool first) {
+    const int nth = pkpass::kGenThreads, B = std::max(1, pts / g.r);
+    const double idle = (double)((B + nth - 1) / nth * nth) / B;
+    return idle * (14.0 + (12.0 + g.cost) / g.r + (first ? 0.0 : 6.0 * (g.r - 1) / g.r));
+}
+
+// Cheapest radix sequence of n on tiles of `pts` points; infinite where a prime factor has no radix.
+double gen_factor(int n, int pts, int depth, std::vector<int>& best) {
+    best.clear();
+    if (n == 1) return 0.0;
+    double c = 1e30;
+    if (depth == PK_GEN_MAXST) return c;
+    for (const GenRadix& g : kGenRadices) {
+        if (n % g.r) continue;
+        std::vector<int> rest;
+        const double v = gen_stage_cost(g, pts, false) + gen_factor(n / g.r, pts, depth + 1, rest);
+        if (v < c) {
+            c = v;
+            best = rest;
+            best.push_back(g.r);
+        }
+    }
+    return c;
+}
+
+// The stages of a length-n transform, in order: an odd radix first (its stores of consecutive
+// butterflies then start on different banks), the others from the largest down.
+double gen_search(int n, int pts, std::vector<int>& rad) {
+    double best = 1e30;
+    for (const GenRadix& g : kGenRadices) {
+        if (g.r % 2 == 0 || n % g.r) continue;
+        std::vector<int> rest;
+        const double c = gen_stage_cost(g, pts, true) + gen_factor(n / g.r, pts, 1, rest);
+        if (c < best) {
+            best = c;
+            std::sort(rest.begin(), rest.end(), [](int a, int b) { return a > b; });
+            rad.assign(1, g.r);
+            rad.insert(rad.end(), rest.begin(), rest.end());
+        }
+    }
+    return best;
+}
+
+// Discrete Fourier transform in double, by the smallest prime factor at each level.
+void host_dft(const double2* x, int n, int stride, double2* out) {
+    if (n == 1) {
+        out[0] = x[0];
+        return;
+    }
+    int p = 2;
+    while (n % p) p++;
+    const int m = n / p;
+    std::vector<double2> sub(n);
+    for (int r = 0; r < p; r++) host_dft(x + (size_t)r * stride, m, stride * p, sub.data() + (size_t)r * m);
+    for (int k = 0; k < n; k++) {
+        double re = 0, im = 0;
+        for (int r = 0; r < p; r++) {
+            const double a = -2.0 * M_PI * (double)((long long)r * k % n) / n, c = std::cos(a), s = std::sin(a);
+            const double2 v = sub[(size_t)r * m + k % m];
+            re += v.x * c - v.y * s;
+            im += v.x * s + v.y * c;
+        }
+        out[k] = make_double2(re, im);
+    }
+}
+
+}  // namespace
+
+// Plan (stages, tile shape) of length n; false where no tile fits shared memory.  `tables` receives
+// the stage twiddles, then for a chirp transform the chirp and the filter's transform.
+static bool gen_plan(int n, GenAxis* g, std::vector<float2>& tables) {
+    *g = GenAxis();
+    g->n = n;
+    std::vector<int> rad;
+    if (n < 2) return false;
+    auto points = [&](int L) { return L * std::max(1, gen_tile(n, L, g)); };
+    int len = n;
+    if (gen_search(n, points(n), rad) > 1e29) {
+        // the cheapest smooth length of 2 n - 1 .. 4 n
+        double best = 1e30;
+        for (int L = 2 * n - 1; L < 4 * n; L++) {
+            int r = L;
+            for (int p : {2, 3, 5, 7}) while (r % p == 0) r /= p;
+            if (r != 1 || 14.0 * L > best) continue;
+            std::vector<int> q;
+            const double c = gen_search(L, points(L), q) * L;
+            if (c < best) {
+                best = c;
+                rad = q;
+                len = L;
+            }
+        }
+        if (best > 1e29) return false;
+        g->blue = 1;
+    }
+    gen_tile(n, len, g);
+    g->L = len;
+    for (int r : rad) g->big |= r > 16;
+    const int L = g->L;
+    auto magic = [](int d) { return d > 1 ? 0xFFFFFFFFu / (unsigned)d + 1u : 0u; };
+    g->nst = (int)rad.size();
+    int ns = 1;
+    tables.clear();
+    for (int s = 0; s < g->nst; s++) {
+        const int R = rad[s];
+        g->rad[s] = R;
+        g->ns[s] = ns;
+        g->m[s] = L / R;
+        g->mg_ns[s] = magic(ns);
+        g->mg_m[s] = magic(L / R);
+        g->off[s] = (int)tables.size();
+        if (ns > 1)
+            for (int k = 0; k < ns; k++)
+                for (int r = 1; r <= pkgen::tw_row(R); r++)
+                    tables.push_back(root_of((int)((long long)r * k * (L / (ns * R)) % L), L));
+        ns *= R;
+    }
+    if (g->blue) {
+        auto chirp = [&](long long e) {   // exp(-i pi e^2 / n)
+            const double a = -M_PI * (double)(e * e % (2LL * n)) / n;
+            return make_double2(std::cos(a), std::sin(a));
+        };
+        for (int e = 0; e < n; e++) {
+            const double2 w = chirp(e);
+            tables.push_back(make_float2((float)w.x, (float)w.y));
+        }
+        std::vector<double2> b(L, make_double2(0, 0)), bk(L);
+        for (int e = 0; e < n; e++) {
+            const double2 w = chirp(e);
+            b[e] = make_double2(w.x, -w.y);
+            if (e) b[L - e] = b[e];
+        }
+        host_dft(b.data(), L, 1, bk.data());
+        for (int k = 0; k < L; k++) tables.push_back(make_float2((float)(bk[k].x / L), (float)(bk[k].y / L)));
+    }
+    return true;
+}
+
+static pk_status pk_get_gen(pk_ctx* ctx, int n, GenAxis* host, const GenAxis** dev) {
+    auto it = ctx->gen.find(n);
+    if (it == ctx->gen.end()) {
+        GenAxis g;
+        std::vector<float2> tables;
+        GenAxis* d = nullptr;
+        if (gen_plan(n, &g, tables)) {
+            const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
+            PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
+            const float2* t = (const float2*)((const char*)d + head);
+            size_t stage_tw = tables.size() - (g.blue ? (size_t)g.n + g.L : 0);
+            g.tw = t;
+            g.chirp = g.blue ? t + stage_tw : nullptr;
+            g.bk = g.blue ? t + stage_tw + g.n : nullptr;
+            cudaError_t e = cudaMemcpy(d, &g, sizeof(g), cudaMemcpyHostToDevice);
+            if (e == cudaSuccess && !tables.empty())
+                e = cudaMemcpy((void*)t, tables.data(), sizeof(float2) * tables.size(), cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) {
+                cudaFree(d);
+                PK_CUDA(e);
+            }
+        }
+        it = ctx->gen.emplace(n, std::make_pair(g, d)).first;
+    }
+    *host = it->second.first;
+    *dev = it->second.second;
+    return PK_OK;
+}
+
 pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a) {
     AxisPlan p;
     if (!pk_make_axis_plan(n, &p)) return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
@@ -818,6 +1079,21 @@ pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a) {
     a->twN = twN;
     a->twStride = twN / n;
     a->plan = pk_find_plan(n);
+    if (a->plan == 0) {
+        GenAxis g;
+        const pk_status st = pk_get_gen(ctx, n, &g, &a->gen);
+        if (st != PK_OK) return st;
+        if (a->gen) {
+            a->genL = g.L;
+            a->genT = g.T;
+            a->gen_rows = g.rows;
+            a->gen_big = g.big;
+            if (g.T) {
+                a->gen_land = pkpass::gen_land(g);
+                a->gen_work = pkpass::gen_work(g);
+            }
+        }
+    }
     return pk_get_axis_table(ctx, n, &a->tw);
 }
 
@@ -841,7 +1117,16 @@ pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
     if ((st = pk_fill_axis(ctx, nx, nx, &d->ax)) != PK_OK) return st;
     if ((st = pk_fill_axis(ctx, nz, nz, &d->az)) != PK_OK) return st;
     if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
-    d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
+    if (d->ay.gen) {   // odd rows run in pairs
+        d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->ay.genL);
+    } else {
+        d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
+    }
+    // a line whose engine buffers do not fit shared memory keeps the in-place engine
+    if (d->ay.gen && step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) {
+        d->ay.gen = nullptr;
+        d->Ly = std::max(1, P / d->M);
+    }
     if ((long long)d->Ly > d->nrows && d->ay.plan == 0) d->Ly = (int)d->nrows;
     d->Tx = d->ax.plan ? plan_cols_xz(nx) : std::max(1, std::min(P / nx, d->Py));
     d->Tz = d->az.plan ? plan_cols_xz(nz) : std::max(1, std::min(P / nz, d->Py));
@@ -876,6 +1161,7 @@ size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; 
 // back to back without host synchronisation and can be captured into a CUDA graph.
 // Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels.
 static int step_plan(int kind, const VolDesc& v) {
+    if (kind == PK_STEP_Y && v.ay.gen) return kNumPlans + v.ay.gen_big;   // the mixed-radix engine's y kernels
     const int p = kind == PK_STEP_Y ? v.ay.plan : kind == PK_STEP_X ? v.ax.plan : kind == PK_STEP_Z ? v.az.plan : 0;
     return (v.tiles_small && kind != PK_STEP_LAMBDA) ? kNumPlans + p : p;
 }
@@ -1017,7 +1303,7 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
             if (detail) {   // diagnostics: the transform length and the kernel family in the kind
                 const int pl = s.plan % kNumPlans;
                 rec.kind += "@" + std::to_string(kPlans[pl].n) +
-                            (s.tma >= 0 ? ":tma" : s.yreg ? ":yreg" : s.kind == PK_STEP_Y ? ":rolled" : ":rio") +
+                            (s.tma >= 0 ? ":tma" : s.gen ? ":gen" : s.yreg ? ":yreg" : s.kind == PK_STEP_Y ? ":rolled" : ":rio") +
                             (s.plan >= kNumPlans ? "-1k" : "");
             }
             rec.bytes = pk_step_bytes(s, prog.descs.data() + s.desc_off);
@@ -1033,6 +1319,10 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
             tma_kernels()->k[s.plan][s.tma][s.tma_var]<<<s.tma_grid, tma_kernels()->threads[s.plan][s.tma][s.tma_var],
                                                          s.tma_smem, st>>>(
                 dd, prog.d_maps + s.desc_off, dp, s.nvol, ctx ? ctx->d_err : nullptr);
+        } else if (s.gen) {
+            gen_kernel().fn[s.gen - 1]<<<s.tma_grid, pkpass::kGenThreads, s.tma_smem, st>>>(
+                dd, prog.d_maps + s.desc_off, dp, s.nvol, s.kind == PK_STEP_X ? 1 : 2, s.mode, s.gen_land, s.gen_work,
+                ctx ? ctx->d_err : nullptr);
         } else if (s.yreg) {
             yreg_kernels()->k[s.mode]<<<s.grid, kThreads, s.yreg_smem, st>>>(dd, dp, s.nvol, ctx ? ctx->d_err : nullptr);
         } else if (s.kind == PK_STEP_Y) {
@@ -1077,6 +1367,9 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
         void* args2[] = {(void*)&dd, (void*)&nvol};
         void* argst[] = {(void*)&dd, (void*)&dm, (void*)&dp, (void*)&nvol, (void*)&de};
         void* argsy[] = {(void*)&dd, (void*)&dp, (void*)&nvol, (void*)&de};
+        int land = s.gen_land, work = s.gen_work;
+        void* argsg[] = {(void*)&dd, (void*)&dm, (void*)&dp, (void*)&nvol, (void*)&axis, (void*)&mode, (void*)&land,
+                         (void*)&work, (void*)&de};
         cudaKernelNodeParams p = {};
         p.blockDim = dim3(kThreads);
         p.gridDim = dim3(s.grid);
@@ -1095,6 +1388,12 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
             p.blockDim = dim3(tma_kernels()->threads[s.plan][s.tma][s.tma_var]);
             p.sharedMemBytes = (unsigned)s.tma_smem;
             p.kernelParams = argst;
+        } else if (s.gen) {
+            p.func = (void*)gen_kernel().fn[s.gen - 1];
+            p.gridDim = dim3(s.tma_grid);
+            p.blockDim = dim3(pkpass::kGenThreads);
+            p.sharedMemBytes = (unsigned)s.tma_smem;
+            p.kernelParams = argsg;
         } else if (s.yreg) {
             p.func = (void*)yreg_kernels()->k[s.mode];
             p.sharedMemBytes = (unsigned)s.yreg_smem;
@@ -1206,8 +1505,8 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
         key.push_back((long long)prog.prefix.size());
         for (const PkStep& s : prog.steps) {
             const long long v[] = {s.kind, s.mode, s.plan, s.nvol, s.grid, (long long)s.smem, s.desc_off, s.prefix_off,
-                                   s.tma, s.tma_var, s.tma_grid, s.yreg, s.conv3};
-            key.insert(key.end(), v, v + 13);
+                                   s.tma, s.tma_var, s.tma_grid, s.yreg, s.conv3, s.gen, s.gen_land, s.gen_work};
+            key.insert(key.end(), v, v + 16);
         }
         auto it = ctx->graphs.find(key);
         if (it == ctx->graphs.end() && ctx->graph_seen.size() >= 4096) ctx->graph_seen.clear();  // bounded

@@ -39,6 +39,21 @@ struct PkRange {
 #endif
 
 // ------------------------------------------------------------------ device-visible structs
+// Run-time plan of a transform length without a compile-time plan (gen_engine.cuh): its stages over
+// L points (L = n, or the length of the chirp convolution when n has a prime factor above 31).
+#define PK_GEN_MAXST 8
+struct GenAxis {
+    int n, L, blue, nst, big;   // blue: chirp transform; big: has a radix above 16
+    int rad[PK_GEN_MAXST], ns[PK_GEN_MAXST], m[PK_GEN_MAXST];    // radix, stride, butterflies per line
+    unsigned mg_ns[PK_GEN_MAXST], mg_m[PK_GEN_MAXST];            // multiply-high reciprocals of ns and m
+    int off[PK_GEN_MAXST];                                       // stage's twiddles W^{rk} at tw[off + k tw_row(R) + r - 1]
+    const float2* tw;
+    const float2* chirp;   // exp(-i pi e^2 / n), e < n
+    const float2* bk;      // transform of the conjugate chirp over L points, / L
+    int T, lt;             // x / z pass: columns per tile (2^lt)
+    int rows, nbox;        // x / z pass: the tile arrives as nbox boxes of `rows` elements of the line
+};
+
 struct AxisDev {
     int n;            // complex transform length along the axis
     int nst;          // number of radix stages (runtime engine)
@@ -47,6 +62,9 @@ struct AxisDev {
     int twN;          // table length (= n)
     int twStride;     // 1
     int plan;         // compile-time plan id (0 = runtime engine)
+    const GenAxis* gen;   // plan 0: the length's run-time plan (device), or null: the in-place engine
+    int genL, genT, gen_rows;   // its L, T and rows, and an x / z tile's buffers (pass_gen.cuh)
+    int gen_land, gen_work, gen_big;
 };
 
 // Pass modes of the y kernel.
@@ -162,6 +180,7 @@ struct pk_ctx {
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::map<int, TwTable> tw;                                   // twN -> table
+    std::map<int, std::pair<GenAxis, GenAxis*>> gen;             // run-time plans by length: host copy, device copy
     // OTF cache: key = (psf content hash, ny, nx, nz)
     std::map<std::tuple<uint64_t, int, int, int>, OtfEntry> otf;
     std::vector<std::pair<void*, size_t>> scratch;               // reusable device buffers by slot
@@ -251,6 +270,9 @@ struct PkStep {
     // set at upload: this y step runs the register-packing kernel (512-voxel rows), with its smem
     int yreg = 0;
     size_t yreg_smem = 0;
+    // set at upload: this x / z step of a length without a plan runs the generic TMA kernel (pass_gen.cuh)
+    // (1: radices up to 16, 2: all) on buffers of these sizes
+    int gen = 0, gen_land = 0, gen_work = 0;
 };
 struct PkProgram {
     std::vector<VolDesc> descs;
