@@ -254,7 +254,7 @@ int tma_index(const PkStep& s) {
 // The first time a single-volume step of a (pass, plan, size class) is seen, every candidate runs
 // once to warm up and twice timed on scratch buffers of that step's geometry (zeroed spectrum and
 // OTF; no live data is touched); the fastest is kept for the context and appended to an on-disk
-// cache (PK_TUNE_FILE, else ~/.cache/pkdecon/tune-v5.txt), keyed by the device name, so later
+// cache (PK_TUNE_FILE, else ~/.cache/pkdecon/tune-v6.txt), keyed by the device name, so later
 // processes skip the timing.  PK_TUNE=0 turns the timing off (the fallback choice everywhere).
 
 std::mutex g_tf_mu;
@@ -266,10 +266,18 @@ std::string tune_path() {
     if (e && *e) return e;
     const char* h = getenv("HOME");
     if (!h || !*h) return "";
-    return std::string(h) + "/.cache/pkdecon/tune-v5.txt";
+    return std::string(h) + "/.cache/pkdecon/tune-v6.txt";
 }
 
+// Name and SM count of a device, read once: cudaGetDeviceProperties takes milliseconds and waits on the
+// device's queued work (it cost 10 ms and the overlap of queued calls on every call whose z step had no
+// timing on record: 1024x1024x512 OMW x2, queued, 189 ms a call of which 31 ms were kernels).
 std::string device_tag(int dev) {
+    static std::mutex mu;
+    static std::map<int, std::string> tags;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = tags.find(dev);
+    if (it != tags.end()) return it->second;
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) {
         cudaGetLastError();
@@ -278,7 +286,7 @@ std::string device_tag(int dev) {
     std::string n = prop.name;
     for (char& c : n)
         if (c == ' ' || c == '|') c = '_';
-    return n + "_sm" + std::to_string(prop.multiProcessorCount);
+    return tags[dev] = n + "_sm" + std::to_string(prop.multiProcessorCount);
 }
 
 void tf_load() {
@@ -422,9 +430,11 @@ int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& ge
     return best;
 }
 
-// Size class of an x / z step: how many waves of variant 0's resident CTAs its tiles make (0: under
-// one wave, 1: one to three, 2: three to twelve, 3: more -- a batch's or a serving round's steps).
-// Variants are chosen per (pass, plan, size class).
+// Size class of an x / z step: how many waves of variant 0's resident CTAs its tiles make (under 1, 2, 3, 5,
+// 8, 12, 24, or more -- a batch's or a serving round's steps).  Variants are chosen per (pass, plan, size
+// class).  The classes are narrow because the order of the candidates changes within a few waves: with one
+// class from 3 to 12, the 512-long x pass of 512x512x128 (9.5 waves) took the register-IO kernel (0.067 ms)
+// that a volume of 3 waves had chosen, where the 16-column TMA kernel takes 0.060 ms.
 int size_class(const PkProgram& prog, const PkStep& s, int idx) {
     const pkpass::TmaTable* t = tma_kernels();
     const int T = t->cols[s.plan][idx][0];
@@ -434,7 +444,9 @@ int size_class(const PkProgram& prog, const PkStep& s, int idx) {
         tiles += (long long)(s.kind == PK_STEP_X ? d.nz : d.nx) * ((d.Py + T - 1) / T);
     }
     const long long wave = (long long)std::max(1, t->per_sm[s.plan][idx][0]) * sm_count();
-    return tiles < wave ? 0 : tiles < 3 * wave ? 1 : tiles < 12 * wave ? 2 : 3;
+    int c = 0;
+    for (int w : {1, 2, 3, 5, 8, 12, 24}) c += tiles >= w * wave;
+    return c;
 }
 
 // The variant an x / z step runs: the context's earlier choice, the on-disk cache's, or a timing.
@@ -516,11 +528,27 @@ int choose_variant(pk_ctx* ctx, const PkProgram& prog, const PkStep& s, int idx,
             used += need;
         }
     }
-    const VolDesc& dt = d0;
+    // a volume above the scratch limit is timed on its first planes (x pass) or rows (z pass): the same lines
+    // and tiles, fewer of them
+    {
+        VolDesc& g = geo[0];
+        const size_t unit = (size_t)(s.mode == XZ_CONV ? 2 : 1) * 8 * g.Pp * (s.kind == PK_STEP_X ? g.nx : g.nz);
+        int& outer = s.kind == PK_STEP_X ? g.nz : g.nx;
+        const int fit = (int)std::min<size_t>(outer, (((size_t)3 << 29) - 1024) / unit);
+        if (fit >= 1 && fit < outer) {
+            if (s.kind == PK_STEP_X) g.blocksX = g.blocksX / outer * fit;
+            else g.blocksZ = g.blocksZ / outer * fit;
+            outer = fit;
+        }
+    }
+    const VolDesc& dt = geo[0];
     std::vector<float> ms;
     PkRange range("pk autotune");
     int best = time_candidates(ctx, s, geo, idx, cands, st, ms);
-    if (best == -2) return fallback;
+    if (best == -2) {   // nothing could be timed: the next call does not try again
+        ctx->tune[key] = fallback;
+        return fallback;
+    }
     ctx->tune[key] = best;
     record(best, "timed", &ms, dt);
     {
