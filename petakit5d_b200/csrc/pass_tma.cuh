@@ -10,9 +10,20 @@
 // TMA box lays them out.  XZ_CONV also brings the OTF tile by TMA (issued at the tile's start, used
 // between the forward and the inverse transform).  All tensor maps cover this GPU's own buffers;
 // no load uses cluster multicast.
+//
+// XZ_CONV runs the inverse as the forward stages transposed, last stage first, so that the elements the
+// forward transform left in registers (multiplied by the OTF there) feed the inverse directly whatever
+// the radices; with a pass over shared memory for the multiply, the convolution of plans whose first and last
+// radix differ was slower than the register-IO kernel.  Measured, before -> after (the launches of 16
+// chunks of 224-416 voxels, and single volumes): z 288 0.493 -> 0.408 ms, z 224 0.368 -> 0.307 ms, z 128 of
+// 512x512x128 0.089 -> 0.074 ms (5460 GB/s).  Lines above 512 come here too, on tiles as wide as shared
+// memory allows (the register-IO tile of 4096 points is 4 columns wide at 1024): x 1024 of 1024x1024x512
+// 1.13 -> 0.90 ms (4780 GB/s), z 512 there 2.85 -> 1.50 ms on 16 columns (4300 GB/s; 8 columns 1.96 ms), x 544
+// of 576x544x544 0.506 -> 0.308 ms, z 544 1.08 -> 0.60 ms.
 #pragma once
 #include <cstdlib>
 
+#include "gen_engine.cuh"
 #include "pass_kernels.cuh"
 #include "tma.cuh"
 
@@ -26,9 +37,12 @@ constexpr int tma_box_rows(int n) {
     return 1;
 }
 
-// plans with a TMA kernel: compile-time plans of >= 2 stages whose column tiles are >= 8 wide
-// (lengths 32..512); longer lines keep the register-IO kernels of pass_kernels.cuh
-constexpr bool tma_plan(int p) { return p > 0 && kPlans[p].nst >= 2 && kPlans[p].n >= 32 && kPlans[p].n <= 512; }
+// plans with a TMA kernel: compile-time plans of >= 2 stages, lengths 32..2048 (a tile of 4 columns of a
+// longer line leaves no room for a second buffer beside the OTF's)
+constexpr bool tma_plan(int p) { return p > 0 && kPlans[p].nst >= 2 && kPlans[p].n >= 32 && kPlans[p].n <= 2048; }
+// columns of the first variant: the 4096-point tile's, and on longer lines as wide as shared memory allows
+// (64-byte rows to 1280, 32-byte ones above)
+constexpr int tma_cols0(int p) { return kPlans[p].n <= 512 ? plan_cols_xz(kPlans[p].n) : kPlans[p].n <= 1280 ? 8 : 4; }
 
 // shared-memory layout of k_xzt<P, ..., TC, NBUF>: NBUF tile buffers | OTF tile (XZ_CONV) | twiddles |
 // barriers, 1024 bytes of slack so the base can be aligned.  TC = columns per tile (0: the plan's
@@ -36,7 +50,7 @@ constexpr bool tma_plan(int p) { return p > 0 && kPlans[p].nst >= 2 && kPlans[p]
 template <int P, int TC = 0, int NBUF = 2>
 struct XztLayout {
     static constexpr int N = kPlans[P].n;
-    static constexpr int T = TC > 0 ? TC : plan_cols_xz(N);
+    static constexpr int T = TC > 0 ? TC : tma_cols0(P);
     static constexpr int PTS = T * N;
     static constexpr int ROWS = tma_box_rows(N);
     static constexpr int NBOX = N / ROWS;
@@ -49,7 +63,7 @@ struct XztLayout {
 // CTAs per SM a variant is compiled for (register budget): 3 for 4096-point tiles, 2 for the
 // two-buffer convolution (three tile-sized buffers) or one 8192-point buffer, 1 for two 8192-point buffers
 constexpr int xzt_min_blocks(int P, int TC, int NBUF, bool conv) {
-    return (TC > 0 ? TC : plan_cols_xz(kPlans[P].n)) * kPlans[P].n > 4096 ? (NBUF >= 2 ? 1 : 2)
+    return (TC > 0 ? TC : tma_cols0(P)) * kPlans[P].n > 4096 ? (NBUF >= 2 ? 1 : 2)
                                                                            : ((conv && NBUF >= 2) ? 2 : 3);
 }
 
@@ -72,6 +86,24 @@ __device__ __forceinline__ bool compute_bar_and(bool ok) {
 
 __device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(pktma::smem_u32(bar)) : "memory");
+}
+
+// Butterfly of any radix, in place; the odd ones above 5 with their roots as immediates (gen_engine.cuh),
+// the inverse as the forward one on swapped re/im.
+template <int R, bool INV>
+__device__ __forceinline__ void dbfly(float2* v) {
+    if constexpr (!direct_radix(R)) {
+        bfly<R, INV>(v);
+    } else {
+        float2 o[R];
+        if constexpr (INV) {
+#pragma unroll
+            for (int r = 0; r < R; r++) v[r] = pkgen::swp(v[r]);
+        }
+        pkgen::butterfly<R>(v, [&](int q, float2 x) { o[q] = INV ? pkgen::swp(x) : x; });
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = o[r];
+    }
 }
 
 // ---- dense column-tile stages (element (l, e) at e*L + l, L = T columns)
@@ -107,8 +139,7 @@ __device__ __forceinline__ void dstage(float2* __restrict__ buf, const float2* _
                     v[i][r] = cmul(v[i][r], w);
                 }
             }
-            if constexpr (!direct_radix(R)) bfly<R, INV>(v[i]);
-            else bf_direct<R, INV>(v[i], tw + OFF + (NS > 1 ? (R - 1) * NS : 0), 1);
+            dbfly<R, INV>(v[i]);
             const int a0 = ((j - k) * R + k) * L + l;
 #pragma unroll
             for (int r = 0; r < R; r++) buf[a0 + r * NS * L] = v[i][r];
@@ -149,33 +180,88 @@ __device__ __forceinline__ void dstage_s2r(const float2* __restrict__ buf, const
                     v[i][r] = cmul(v[i][r], w);
                 }
             }
-            if constexpr (!direct_radix(R)) bfly<R, INV>(v[i]);
-            else bf_direct<R, INV>(v[i], tw + OFF + (NS > 1 ? (R - 1) * NS : 0), 1);
+            dbfly<R, INV>(v[i]);
         }
     }
 }
 
-// first stage from registers: v[i][r] is element j + r (N / R) of column l; butterfly, store
-template <int R, int N, int L, bool INV, int NTH>
-__device__ __forceinline__ void dstage_r2s(float2* __restrict__ buf, int tid,
-                                           float2 (&v)[(L * (N / R) + NTH - 1) / NTH][R]) {
-    static_assert(!direct_radix(R), "first stage needs a register butterfly");
-    constexpr int M = N / R;
-    constexpr int B = L * M;
-    constexpr int NT = NTH;
-    constexpr int MAXB = (B + NT - 1) / NT;
+// The transform's stages transposed, for the inverse after the OTF multiply: a DFT is its own transpose, so
+// the stages run backwards (butterfly, then the stage's twiddles; read where the stage stores, write
+// where it loads).  The first of them starts from the elements that the forward transform's last stage
+// left in registers, whatever the radices: no pass over shared memory between the transforms.
+// Last stage's transpose from registers: the outputs go where the thread's inputs were.
+template <int R, int NS, int N, int L, bool INV, int OFF, int NTH>
+__device__ __forceinline__ void dstage_t_r2s(float2* __restrict__ buf, const float2* __restrict__ tw, int tid,
+                                             float2 (&v)[(L * (N / R) + NTH - 1) / NTH][R]) {
+    static_assert(NS * R == N, "the last stage of the transform");
+    constexpr int B = L * NS;
+    constexpr int MAXB = (B + NTH - 1) / NTH;
 #pragma unroll
     for (int i = 0; i < MAXB; i++) {
-        const int b = tid + i * NT;
-        if (B % NT == 0 || b < B) {
+        const int b = tid + i * NTH;
+        if (B % NTH == 0 || b < B) {
             const int l = b % L, j = b / L;
-            bfly<R, INV>(v[i]);
-            const int a0 = j * R * L + l;
+            dbfly<R, INV>(v[i]);
+            if constexpr (NS > 1) {
 #pragma unroll
-            for (int r = 0; r < R; r++) buf[a0 + r * L] = v[i][r];
+                for (int r = 1; r < R; r++) {
+                    float2 w = tw[OFF + (r - 1) * NS + j];
+                    if (INV) w.y = -w.y;
+                    v[i][r] = cmul(v[i][r], w);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) buf[(j + r * NS) * L + l] = v[i][r];
         }
     }
     compute_bar<NTH>();
+}
+
+template <int R, int NS, int N, int L, bool INV, int OFF, int NTH>
+__device__ __forceinline__ void dstage_t(float2* __restrict__ buf, const float2* __restrict__ tw, int tid) {
+    constexpr int M = N / R;
+    constexpr int B = L * M;
+    constexpr int MAXB = (B + NTH - 1) / NTH;
+    float2 v[MAXB][R];
+#pragma unroll
+    for (int i = 0; i < MAXB; i++) {
+        const int b = tid + i * NTH;
+        const int bb = (B % NTH == 0 || b < B) ? b : 0;   // as in dstage: an unconditional load
+        const int l = bb % L, j = bb / L, k = j % NS;
+        const int a0 = ((j - k) * R + k) * L + l;
+#pragma unroll
+        for (int r = 0; r < R; r++) v[i][r] = buf[a0 + r * NS * L];
+    }
+    compute_bar<NTH>();
+#pragma unroll
+    for (int i = 0; i < MAXB; i++) {
+        const int b = tid + i * NTH;
+        if (B % NTH == 0 || b < B) {
+            const int l = b % L, j = b / L, k = j % NS;
+            dbfly<R, INV>(v[i]);
+            if constexpr (NS > 1) {
+#pragma unroll
+                for (int r = 1; r < R; r++) {
+                    float2 w = tw[OFF + (r - 1) * NS + k];
+                    if (INV) w.y = -w.y;
+                    v[i][r] = cmul(v[i][r], w);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) buf[(j + r * M) * L + l] = v[i][r];
+        }
+    }
+    compute_bar<NTH>();
+}
+
+// stages S, S - 1, .., 0 of plan P transposed
+template <int P, int S, int L, bool INV, int NTH>
+__device__ __forceinline__ void run_dense_t(float2* buf, const float2* tw, int tid) {
+    if constexpr (S >= 0) {
+        constexpr int R = kPlans[P].rad[S];
+        dstage_t<R, plan_ns_before(P, S), kPlans[P].n, L, INV, stage_tw_off(P, S), NTH>(buf, tw, tid);
+        run_dense_t<P, S - 1, L, INV, NTH>(buf, tw, tid);
+    }
 }
 
 template <int P, int S, int S1, int NS, int L, bool INV, int NTH>
@@ -328,49 +414,35 @@ __global__ void __launch_bounds__(NTH + 32, xzt_min_blocks(P, TC, NBUF, MODE == 
             run_dense<P, 0, NST, 1, T, MODE == XZ_INV, NTH>(cur, tw, tid);
         } else {
             const bool cj = descs[vol].conj != 0;
-            if constexpr (pkpass::same_end_radix(P)) {
-                constexpr int R = kPlans[P].rad[0], MS = N / R, MAXB = (T * MS + NT - 1) / NT;
-                float2 v[MAXB][R];
-                run_dense<P, 0, NST - 1, 1, T, false, NTH>(cur, tw, tid);
-                dstage_s2r<R, plan_ns_before(P, NST - 1), N, T, false, stage_tw_off(P, NST - 1), NTH>(cur, tw, tid, v);
-                ok = pktma::mbar_wait(otf_full, (uint32_t)(it & 1));
-                if (!compute_bar_and<NTH>(ok)) {
-                    if (tid == 0) pktma::report_wait_failure(err, 1);
-                    return;
-                }
+            // the last forward stage leaves each thread R elements j + r MS of a column in registers: OTF
+            // multiply there, then the inverse's stages from the last backwards
+            constexpr int R = kPlans[P].rad[NST - 1], MS = N / R, MAXB = (T * MS + NT - 1) / NT;
+            constexpr int OFF = stage_tw_off(P, NST - 1);
+            float2 v[MAXB][R];
+            run_dense<P, 0, NST - 1, 1, T, false, NTH>(cur, tw, tid);
+            dstage_s2r<R, MS, N, T, false, OFF, NTH>(cur, tw, tid, v);
+            ok = pktma::mbar_wait(otf_full, (uint32_t)(it & 1));
+            if (!compute_bar_and<NTH>(ok)) {
+                if (tid == 0) pktma::report_wait_failure(err, 1);
+                return;
+            }
 #pragma unroll
-                for (int i = 0; i < MAXB; i++) {
-                    const int b = tid + i * NT;
-                    if (MAXB * NT == T * MS || b < T * MS) {
-                        const int l = b % T, j = b / T;
+            for (int i = 0; i < MAXB; i++) {
+                const int b = tid + i * NT;
+                if (MAXB * NT == T * MS || b < T * MS) {
+                    const int l = b % T, j = b / T;
 #pragma unroll
-                        for (int r = 0; r < R; r++) {
-                            float2 h = hb[(j + r * MS) * T + l];
-                            if (cj) h.y = -h.y;
-                            v[i][r] = cmul(v[i][r], h);
-                        }
+                    for (int r = 0; r < R; r++) {
+                        float2 h = hb[(j + r * MS) * T + l];
+                        if (cj) h.y = -h.y;
+                        v[i][r] = cmul(v[i][r], h);
                     }
                 }
-                compute_bar<NTH>();   // every OTF read done: the producer may refill it
-                if (tid == 0) mbar_arrive_cta(otf_empty);
-                dstage_r2s<R, N, T, true, NTH>(cur, tid, v);
-                run_dense<P, 1, NST, R, T, true, NTH>(cur, tw, tid);
-            } else {
-                run_dense<P, 0, NST, 1, T, false, NTH>(cur, tw, tid);
-                ok = pktma::mbar_wait(otf_full, (uint32_t)(it & 1));
-                if (!compute_bar_and<NTH>(ok)) {
-                    if (tid == 0) pktma::report_wait_failure(err, 1);
-                    return;
-                }
-                for (int i = tid; i < PTS; i += NT) {
-                    float2 h = hb[i];
-                    if (cj) h.y = -h.y;
-                    cur[i] = cmul(cur[i], h);
-                }
-                compute_bar<NTH>();
-                if (tid == 0) mbar_arrive_cta(otf_empty);
-                run_dense<P, 0, NST, 1, T, true, NTH>(cur, tw, tid);
             }
+            compute_bar<NTH>();   // every OTF read done: the producer may refill it
+            if (tid == 0) mbar_arrive_cta(otf_empty);
+            dstage_t_r2s<R, MS, N, T, true, OFF, NTH>(cur, tw, tid, v);
+            run_dense_t<P, NST - 2, T, true, NTH>(cur, tw, tid);
         }
         // the tile leaves by TMA: each thread's writes are ordered before the async proxy's reads,
         // then the buffer is handed to the producer
@@ -414,42 +486,66 @@ inline void register_tma_one(TmaTable& t) {
     t.per_sm[P][IDX][VAR] = n;
 }
 
+// x forward and inverse, variant VAR
+template <int P, int VAR, int TC, int NBUF, int NTH>
+inline void register_tma_x(TmaTable& t) {
+    register_tma_one<P, TMA_X_FWD, VAR, 1, XZ_FWD, TC, NBUF, NTH>(t);
+    register_tma_one<P, TMA_X_INV, VAR, 1, XZ_INV, TC, NBUF, NTH>(t);
+}
+
 template <int P, int HI>
 struct RegisterTma {
     static void fill(TmaTable& t) {
         if constexpr (tma_plan(P)) {
-            register_tma_one<P, TMA_X_FWD, 0, 1, XZ_FWD>(t);
-            register_tma_one<P, TMA_X_INV, 0, 1, XZ_INV>(t);
-            register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV>(t);
-            if constexpr (kPlans[P].n == 512) {
+            constexpr int N = kPlans[P].n;
+            if constexpr (N <= 512) {
+                register_tma_x<P, 0, 0, 2, PK_THREADS>(t);
+                register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV>(t);
+            }
+            if constexpr (N == 512) {
                 // 8-column tiles (64-byte rows, 3 CTAs per SM) against 16-column tiles (128-byte rows,
                 // one CTA per SM, 16 compute warps) with two or three buffers
-                register_tma_one<P, TMA_X_FWD, 1, 1, XZ_FWD, 16, 2, 512>(t);
-                register_tma_one<P, TMA_X_INV, 1, 1, XZ_INV, 16, 2, 512>(t);
-                register_tma_one<P, TMA_X_FWD, 2, 1, XZ_FWD, 16, 3, 512>(t);
-                register_tma_one<P, TMA_X_INV, 2, 1, XZ_INV, 16, 3, 512>(t);
+                register_tma_x<P, 1, 16, 2, 512>(t);
+                register_tma_x<P, 2, 16, 3, 512>(t);
+                register_tma_one<P, TMA_Z_CONV, 1, 2, XZ_CONV, 16, 2, 512>(t);
             }
-            if constexpr (kPlans[P].n == 256) {
+            if constexpr (N == 256) {
                 // the convolution with 32-column tiles (256-byte rows, two buffers, 16 compute warps) and
                 // with 24-column tiles (three buffers, 12 compute warps), one CTA per SM
                 register_tma_one<P, TMA_Z_CONV, 1, 2, XZ_CONV, 32, 2, 512>(t);
                 register_tma_one<P, TMA_Z_CONV, 2, 2, XZ_CONV, 24, 3, 384>(t);
             }
-            if constexpr (kPlans[P].n > 256 && kPlans[P].n < 512) {
+            if constexpr (N > 256 && N < 512) {
                 // lines longer than 256: the 4096-point tile is 8 columns (64-byte rows) or fewer wide;
                 // 16-column tiles (128-byte rows), 16 compute warps, three or two buffers, one CTA per SM
-                register_tma_one<P, TMA_X_FWD, 1, 1, XZ_FWD, 16, 3, 512>(t);
-                register_tma_one<P, TMA_X_INV, 1, 1, XZ_INV, 16, 3, 512>(t);
-                register_tma_one<P, TMA_X_FWD, 2, 1, XZ_FWD, 16, 2, 512>(t);
-                register_tma_one<P, TMA_X_INV, 2, 1, XZ_INV, 16, 2, 512>(t);
+                register_tma_x<P, 1, 16, 3, 512>(t);
+                register_tma_x<P, 2, 16, 2, 512>(t);
                 if constexpr (XztLayout<P, 16, 3>::bytes(true) <= 227 * 1024)
                     register_tma_one<P, TMA_Z_CONV, 1, 2, XZ_CONV, 16, 3, 384>(t);
                 register_tma_one<P, TMA_Z_CONV, 2, 2, XZ_CONV, 16, 2, 512>(t);
             }
-            if constexpr (kPlans[P].n >= 128 && kPlans[P].n < 256) {
+            if constexpr (N >= 128 && N < 256) {
                 // 16- or 32-column tiles already: three buffers (x)
-                register_tma_one<P, TMA_X_FWD, 1, 1, XZ_FWD, 0, 3>(t);
-                register_tma_one<P, TMA_X_INV, 1, 1, XZ_INV, 0, 3>(t);
+                register_tma_x<P, 1, 0, 3, PK_THREADS>(t);
+            }
+            if constexpr (N > 512 && N <= 768) {
+                // 8-column tiles, two buffers, 2-3 CTAs per SM, against 16-column ones on one CTA per SM
+                // with as many buffers as fit
+                register_tma_x<P, 0, 8, 2, PK_THREADS>(t);
+                register_tma_x<P, 1, 16, 2, 512>(t);
+                register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV, 8, 2, PK_THREADS>(t);
+                register_tma_one<P, TMA_Z_CONV, 1, 2, XZ_CONV, 16, N <= 576 ? 2 : 1, 512>(t);
+            }
+            if constexpr (N <= 576 && N > 512) register_tma_x<P, 2, 16, 3, 512>(t);
+            if constexpr (N > 768 && N <= 1280) {
+                register_tma_x<P, 0, 8, 2, 512>(t);
+                if constexpr (N <= 1152) register_tma_x<P, 1, 8, 3, 512>(t);
+                register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV, 8, N <= 1152 ? 2 : 1, 512>(t);
+            }
+            if constexpr (N > 1280) {
+                register_tma_x<P, 0, 4, 2, 512>(t);
+                register_tma_x<P, 1, 4, 3, 512>(t);
+                register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV, 4, 2, 512>(t);
             }
         }
         RegisterTma<P + 1, HI>::fill(t);
