@@ -135,48 +135,119 @@ __global__ void k_to_u16(const float* __restrict__ J, long long n, uint16_t* __r
     }
 }
 
-// ---- irregular-mask edge erosion (decon_mask_edge_erosion.m:18-29)
-__global__ void k_mask_faces(uint8_t* m, int ny, int nx, int nz) {
-    const long long n = (long long)ny * nx * nz;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(i % ny);
-        const int x = (int)((i / ny) % nx);
-        const int z = (int)(i / ((long long)ny * nx));
+// ---- edge erosion of a byte mask (decon_mask_edge_erosion.m:8-29), on 32 voxels of a row per word
+//
+// The erosion by strel('disk', E - 1) is, for each column offset of the disk, an erosion of the shifted row by
+// a run of 2 h + 1 voxels (the disk's columns are symmetric runs), done on packed words by shift-and-AND
+// doubling; then the line along z is an AND of words.  Bound by the passes over the byte mask (read to pack,
+// written at the end): 0.45 ms on 512 x 1140 x 270 voxels at E = 8, where one byte load per voxel and disk
+// offset took 13.9 ms.  `zeros` (the raw mask's zero voxels, counted by the pass before) picks the
+// branch on the device: a full mask only loses E voxels at each face, and no call waits for the count.
+__device__ __forceinline__ int mask_words(int ny) { return (ny + 31) >> 5; }
+
+// irregular mask: bytes -> words, faces cleared (:18-20); voxels past the row's end count as set
+__global__ void k_mask_pack(const uint8_t* __restrict__ m, unsigned* __restrict__ bits, int ny, int nx, int nz,
+                            const unsigned* __restrict__ zeros) {
+    if (*zeros == 0) return;
+    const int lane = threadIdx.x & 31, W = mask_words(ny);
+    const long long rows = (long long)nx * nz;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+        const int x = (int)(r % nx), z = (int)(r / nx);
         // one plane is MATLAB's 2-D case (ndims 2): no z faces
-        if (y == 0 || y == ny - 1 || x == 0 || x == nx - 1 || (nz > 1 && (z == 0 || z == nz - 1))) m[i] = 0;
+        const bool face = x == 0 || x == nx - 1 || (nz > 1 && (z == 0 || z == nz - 1));
+        const uint8_t* row = m + r * ny;
+        for (int w0 = 0; w0 < W; w0 += 32) {   // lane q keeps word w0 + q
+            unsigned mine = 0;
+#pragma unroll 8
+            for (int q = 0; q < 32; q++) {
+                const int y = (w0 + q) * 32 + lane;
+                if ((w0 + q) * 32 >= ny) break;
+                const bool set = y >= ny || (!face && y > 0 && y < ny - 1 && row[y] != 0);
+                const unsigned v = __ballot_sync(0xffffffffu, set);
+                if (lane == q) mine = v;
+            }
+            if (w0 + lane < W) bits[r * W + w0 + lane] = mine;
+        }
     }
 }
 
-// erosion with a 2D (per z-slice) neighbourhood given as (dy, dx) offsets; outside counts as true
-__global__ void k_erode_xy(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int ny, int nx, int nz,
-                           const int2* __restrict__ offs, int noff) {
-    const long long n = (long long)ny * nx * nz;
+// AND over t = -h .. h of bit i + t, for the 32 bits i of word w of a row
+__device__ __forceinline__ unsigned erode_run(const unsigned* __restrict__ row, int w, int W, int h) {
+    auto at = [&](int i) { return i >= 0 && i < W ? row[i] : 0xffffffffu; };
+    if (h == 0) return row[w];
+    if (h < 32) {
+        const unsigned p = at(w - 1), c = row[w], n = at(w + 1);
+        // a: the bits from 32 w - h on; each doubling ANDs it with itself shifted by what it covers
+        const int s = 32 - h;
+        unsigned a0 = __funnelshift_rc(p, c, s), a1 = __funnelshift_rc(c, n, s), a2 = __funnelshift_rc(n, 0xffffffffu, s);
+        const int len = 2 * h + 1;
+        int cov = 1;
+        for (; 2 * cov <= len; cov *= 2) {
+            a0 &= __funnelshift_rc(a0, a1, cov);
+            a1 &= __funnelshift_rc(a1, a2, cov);
+            a2 &= __funnelshift_rc(a2, 0xffffffffu, cov);
+        }
+        return a0 & __funnelshift_rc(a0, a1, len - cov);
+    }
+    unsigned v = 0xffffffffu;
+    for (int t = -h; t <= h && v; t++) {
+        const int q = t >= 0 ? t >> 5 : -((31 - t) >> 5), s = t - 32 * q;
+        v &= __funnelshift_rc(at(w + q), at(w + q + 1), s);
+    }
+    return v;
+}
+
+// erosion by the disk within each plane (:23-25); hw[c]: half length of the disk's run at column offset c - R,
+// -1 where the disk has none; voxels outside the plane count as set
+__global__ void k_mask_disk(const unsigned* __restrict__ in, unsigned* __restrict__ out, int ny, int nx, int nz,
+                            const int* __restrict__ hw, int R, const unsigned* __restrict__ zeros) {
+    if (*zeros == 0) return;
+    const int W = mask_words(ny);
+    const long long n = (long long)W * nx * nz;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(i % ny);
-        const int x = (int)((i / ny) % nx);
-        const long long zo = (i / ((long long)ny * nx)) * (long long)ny * nx;
-        uint8_t v = in[i];
-        for (int k = 0; v && k < noff; k++) {
-            const int yy = y + offs[k].x, xx = x + offs[k].y;
-            if (yy < 0 || yy >= ny || xx < 0 || xx >= nx) continue;
-            v = in[zo + yy + (long long)ny * xx];
+        const int w = (int)(i % W);
+        const long long r = i / W;
+        const int x = (int)(r % nx);
+        unsigned v = in[i];
+        for (int c = -R; c <= R && v; c++) {
+            if (x + c < 0 || x + c >= nx || hw[c + R] < 0) continue;
+            v &= erode_run(in + (r + c) * W, w, W, hw[c + R]);
         }
         out[i] = v;
     }
 }
 
-__global__ void k_erode_z(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int ny, int nx, int nz, int h) {
-    const long long n = (long long)ny * nx * nz;
-    const long long plane = (long long)ny * nx;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int z = (int)(i / plane);
-        uint8_t v = in[i];
-        for (int o = -h; v && o <= h; o++) {
-            const int zz = z + o;
-            if (zz < 0 || zz >= nz) continue;
-            v = in[i + (long long)o * plane];
+// the line of 2 E - 1 voxels along z (:26-28; none for one plane) and words -> bytes; a full mask instead loses
+// E voxels at each face (:8-15)
+__global__ void k_mask_line(const unsigned* __restrict__ bits, uint8_t* __restrict__ m, int ny, int nx, int nz, int E,
+                            const unsigned* __restrict__ zeros) {
+    const int lane = threadIdx.x & 31, W = mask_words(ny);
+    const long long rows = (long long)nx * nz;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    const bool full = *zeros == 0;
+    for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+        const int x = (int)(r % nx), z = (int)(r / nx);
+        uint8_t* row = m + r * ny;
+        if (full) {
+            const bool face = x < E || x >= nx - E || (nz > 1 && (z < E || z >= nz - E));
+            for (int y = lane; y < ny; y += 32)
+                if (face || y < E || y >= ny - E) row[y] = 0;
+            continue;
         }
-        out[i] = v;
+        for (int w0 = 0; w0 < W; w0 += 32) {
+            unsigned v = 0;
+            if (w0 + lane < W) {
+                v = 0xffffffffu;
+                for (int q = max(0, z - E + 1); q <= min(nz - 1, z + E - 1) && v; q++)
+                    v &= bits[(r + (long long)(q - z) * nx) * W + w0 + lane];
+            }
+            for (int q = 0; q < 32 && w0 + q < W; q++) {
+                const unsigned word = __shfl_sync(0xffffffffu, v, q);
+                const int y = (w0 + q) * 32 + lane;
+                if (y < ny) row[y] = (word >> lane) & 1u;
+            }
+        }
     }
 }
 
@@ -281,7 +352,34 @@ pk_status pk_scratch(pk_ctx* ctx, int slot, size_t bytes, void** ptr) {
 }
 
 enum { SL_ARENA = 0, SL_JB = 2, SL_S = 5, SL_MASK2 = 7, SL_IN = 9, SL_OUT = 10, SL_PSF = 11, SL_SUM = 12,
-       SL_OFFS = 13, SL_ZC = 14 };
+       SL_ZC = 14 };
+
+// mask = decon_mask_edge_erosion(mask, E) on a device byte mask, on `st`; *zeros: 0 where the mask is full.
+static pk_status erode_mask(pk_ctx* ctx, uint8_t* mask, int ny, int nx, int nz, int E, const unsigned* zeros,
+                            cudaStream_t st) {
+    const int R = E - 1;
+    void*& hw = ctx->dev_tables["disk:" + std::to_string(R)];   // the disk's runs, once per radius
+    if (!hw) {
+        std::vector<int> h(2 * R + 1, -1);
+        for (const int2& o : pk_disk_offsets(R)) h[o.y + R] = std::max(h[o.y + R], o.x);
+        void* d = nullptr;
+        PK_CUDA(cudaMalloc(&d, sizeof(int) * h.size()));
+        hw = d;
+        PK_CUDA(cudaMemcpy(hw, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
+    }
+    const size_t words = (size_t)((ny + 31) / 32) * nx * nz;
+    void* b;
+    pk_status s;
+    if ((s = pk_scratch(ctx, SL_MASK2, 2 * words * sizeof(unsigned), &b)) != PK_OK) return s;
+    unsigned *b0 = (unsigned*)b, *b1 = b0 + words;
+    const int gr = grid_for((long long)nx * nz * 32);
+    k_mask_pack<<<gr, 256, 0, st>>>(mask, b0, ny, nx, nz, zeros);
+    k_mask_disk<<<grid_for((long long)words), 256, 0, st>>>(b0, b1, ny, nx, nz, (const int*)hw, R, zeros);
+    k_mask_line<<<gr, 256, 0, st>>>(b1, mask, ny, nx, nz, E, zeros);
+    ctx->launches += 3;
+    PK_CUDA(cudaGetLastError());
+    return PK_OK;
+}
 
 // Half-spectrum OTF of a PSF at the volume size, scaled by `scale` (1/N for the iterations).
 pk_status pk_make_otf(pk_ctx* ctx, const float* h_psf, const int64_t pd[3], int ny, int nx, int nz, double scale,
@@ -551,32 +649,15 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
     }
     PkProgram prog;
     pk_program_add(prog, PK_STEP_Y, Y_PRE, base);
-    std::vector<int> mask_mode(nj, need_mask ? 1 : 0);
+    const std::vector<int> mask_mode(nj, need_mask ? 1 : 0);
     if (p->edge_erosion > 0) {
-        // the erosion branch depends on whether the raw mask is full (decon_mask_edge_erosion.m:8)
+        // the masks are eroded behind the pre-pass, which writes them and counts the raw zeros
         if ((s = pk_program_upload(ctx, prog, st)) != PK_OK) return s;
         if ((s = pk_program_launch(ctx, prog, st)) != PK_OK) return s;
         prog = PkProgram();
-        std::vector<unsigned int> zeros(nj, 0);
-        PK_CUDA(cudaMemcpyAsync(zeros.data(), zc, sizeof(unsigned int) * nj, cudaMemcpyDeviceToHost, st));
-        PK_CUDA(cudaStreamSynchronize(st));
-        std::vector<int2> disk = pk_disk_offsets(p->edge_erosion - 1);
         for (size_t i = 0; i < nj; i++) {
-            if (zeros[i] == 0) { mask_mode[i] = 2; continue; }
-            mask_mode[i] = 3;
-            DeconJob& j = jobs[i];
-            const int ny = j.dims[0], nx = j.dims[1], nz = j.dims[2];
-            const size_t N = (size_t)ny * nx * nz;
-            void *m2, *offs;
-            if ((s = pk_scratch(ctx, SL_MASK2, N, &m2)) != PK_OK) return s;
-            if ((s = pk_scratch(ctx, SL_OFFS, sizeof(int2) * disk.size(), &offs)) != PK_OK) return s;
-            PK_CUDA(cudaMemcpyAsync(offs, disk.data(), sizeof(int2) * disk.size(), cudaMemcpyHostToDevice, st));
-            k_mask_faces<<<grid_for((long long)N), 256, 0, st>>>(j.mask, ny, nx, nz);
-            k_erode_xy<<<grid_for((long long)N), 256, 0, st>>>(j.mask, (uint8_t*)m2, ny, nx, nz, (const int2*)offs,
-                                                                (int)disk.size());
-            k_erode_z<<<grid_for((long long)N), 256, 0, st>>>((const uint8_t*)m2, j.mask, ny, nx, nz, p->edge_erosion - 1);
-            PK_CUDA(cudaGetLastError());
-            PK_CUDA(cudaStreamSynchronize(st));  // the offsets are a host temporary, m2 is reused
+            const DeconJob& j = jobs[i];
+            if ((s = erode_mask(ctx, j.mask, j.dims[0], j.dims[1], j.dims[2], p->edge_erosion, zc + i, st)) != PK_OK) return s;
         }
     }
     for (VolDesc& d : base) {
@@ -791,26 +872,14 @@ pk_status pk_decon_run(pk_ctx* ctx, int method, const void* d_in, pk_dtype in_ty
 namespace {
 
 template <typename T>
-__global__ void k_positive(const T* __restrict__ im, long long n, uint8_t* __restrict__ m,
-                           unsigned long long* __restrict__ zeros) {
-    unsigned long long z = 0;
+__global__ void k_positive(const T* __restrict__ im, long long n, uint8_t* __restrict__ m, unsigned* __restrict__ zeros) {
+    bool z = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const bool p = im[i] > (T)0;
         m[i] = p;
-        z += !p;
+        z |= !p;
     }
-    if (z) atomicAdd(zeros, z);
-}
-
-// full mask: E voxels cleared at each face (:8-15), z only for more than one plane
-__global__ void k_full_faces(uint8_t* m, int ny, int nx, int nz, int E) {
-    const long long n = (long long)ny * nx * nz;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(i % ny);
-        const int x = (int)((i / ny) % nx);
-        const int z = (int)(i / ((long long)ny * nx));
-        if (y < E || y >= ny - E || x < E || x >= nx - E || (nz > 1 && (z < E || z >= nz - E))) m[i] = 0;
-    }
+    if (z) *zeros = 1;   // every writer stores the same value
 }
 
 }  // namespace
@@ -830,31 +899,16 @@ extern "C" pk_status pk_mask_edge_erosion(pk_ctx* ctx, const void* im, pk_dtype 
     cudaSetDevice(ctx->device);
     cudaStream_t st = ctx->stream;
     pk_status s;
-    void *din, *dm, *dm2, *dz, *doffs;
-    const std::vector<int2> disk = pk_disk_offsets(erosion - 1);
+    void *din, *dm, *dz;
     if ((s = pk_scratch(ctx, 37, es * n, &din)) != PK_OK) return s;
     if ((s = pk_scratch(ctx, 38, n, &dm)) != PK_OK) return s;
-    if ((s = pk_scratch(ctx, 39, n, &dm2)) != PK_OK) return s;
-    if ((s = pk_scratch(ctx, 40, sizeof(unsigned long long), &dz)) != PK_OK) return s;
-    if ((s = pk_scratch(ctx, 41, sizeof(int2) * disk.size(), &doffs)) != PK_OK) return s;
+    if ((s = pk_scratch(ctx, 40, sizeof(unsigned), &dz)) != PK_OK) return s;
     PK_CUDA(cudaMemcpyAsync(din, im, es * n, cudaMemcpyHostToDevice, st));
-    PK_CUDA(cudaMemsetAsync(dz, 0, sizeof(unsigned long long), st));
-    if (type == PK_U16) k_positive<<<grid_for(n), 256, 0, st>>>((const uint16_t*)din, n, (uint8_t*)dm, (unsigned long long*)dz);
-    else k_positive<<<grid_for(n), 256, 0, st>>>((const float*)din, n, (uint8_t*)dm, (unsigned long long*)dz);
-    unsigned long long zeros = 0;
-    PK_CUDA(cudaMemcpyAsync(&zeros, dz, sizeof(zeros), cudaMemcpyDeviceToHost, st));
-    PK_CUDA(cudaStreamSynchronize(st));
-    if (zeros == 0) {
-        k_full_faces<<<grid_for(n), 256, 0, st>>>((uint8_t*)dm, ny, nx, nz, erosion);
-        ctx->launches += 2;
-    } else {                                                     // :18-29; k_erode_z is a copy for one plane
-        PK_CUDA(cudaMemcpyAsync(doffs, disk.data(), sizeof(int2) * disk.size(), cudaMemcpyHostToDevice, st));
-        k_mask_faces<<<grid_for(n), 256, 0, st>>>((uint8_t*)dm, ny, nx, nz);
-        k_erode_xy<<<grid_for(n), 256, 0, st>>>((const uint8_t*)dm, (uint8_t*)dm2, ny, nx, nz, (const int2*)doffs,
-                                                (int)disk.size());
-        k_erode_z<<<grid_for(n), 256, 0, st>>>((const uint8_t*)dm2, (uint8_t*)dm, ny, nx, nz, erosion - 1);
-        ctx->launches += 4;
-    }
+    PK_CUDA(cudaMemsetAsync(dz, 0, sizeof(unsigned), st));
+    if (type == PK_U16) k_positive<<<grid_for(n), 256, 0, st>>>((const uint16_t*)din, n, (uint8_t*)dm, (unsigned*)dz);
+    else k_positive<<<grid_for(n), 256, 0, st>>>((const float*)din, n, (uint8_t*)dm, (unsigned*)dz);
+    ctx->launches++;
+    if ((s = erode_mask(ctx, (uint8_t*)dm, ny, nx, nz, erosion, (const unsigned*)dz, st)) != PK_OK) return s;
     PK_CUDA(cudaGetLastError());
     PK_CUDA(cudaMemcpyAsync(mask, dm, n, cudaMemcpyDeviceToHost, st));
     PK_CUDA(cudaStreamSynchronize(st));

@@ -47,8 +47,8 @@ __host__ __device__ constexpr size_t yreg_smem_bytes(int mode) {
     return 128 + sizeof(float2) * ((size_t)y_naux(mode) * 4096 + (size_t)(4096 + 4096 / 16 + 1 + 1) + (256 + 32) + 258) + 16;
 }
 
-// Volume descriptor fields the kernel needs for a voxel's post-processing are those of the rolled
-// kernel's fused path: no damping, scaling, mask or crop (the host only picks this kernel then).
+// Post-processing here is scaling, offset and a byte mask; damping, crops and the border mask take the
+// rolled kernel (the host's choice).
 template <int P, int MODE>
 __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)
     k_yr(const VolDesc* __restrict__ descs, const int* __restrict__ prefix, int nvol, int* err) {
@@ -222,12 +222,23 @@ __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)
         void* const o = kPost ? d.out : nullptr;
         const bool vec_out = kPost && ((reinterpret_cast<uintptr_t>(o) & (d.save16 ? 3 : 7)) == 0);
         const bool s16 = kPost && d.save16;
+        const int smode = kPost ? d.scale_mode : 0;
+        const float scale = d.scale, offset = d.offset;
+        const uint8_t* const pm = kPost && d.mask_mode != 0 ? d.mask8 : nullptr;
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int e = j + 16 * r;
             const long long vi = row * (long long)ny + 2 * e;
-            const float2 val = v[0][r];
+            float2 val = v[0][r];
             if constexpr (kPost) {
+                if (smode != 0) {   // post_value's scaling, then offset and mask
+                    val = make_float2(__fmul_rn(val.x, scale), __fmul_rn(val.y, scale));
+                    if (smode == 2) {
+                        const unsigned m2 = pm ? *reinterpret_cast<const uint16_t*>(pm + vi) : 0x0101u;
+                        val.x = __fmul_rn(__fadd_rn(val.x, offset), (m2 & 0xffu) ? 1.f : 0.f);
+                        val.y = __fmul_rn(__fadd_rn(val.y, offset), (m2 >> 8) ? 1.f : 0.f);
+                    }
+                }
                 if (vec_out) {
                     if (s16) {
                         const unsigned lo = (unsigned)u16_of(val.x), hi = (unsigned)u16_of(val.y);
