@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kGenThreads, BIG ? 2 : 3)
         pktma::mbar_init(bar, 1);
         pktma::fence_mbar_init();
         for (int v = 0; v < nvol; v++) pktma::tmap_acquire(&maps[v].s);
+        pdl_wait();   // only this thread moves what other passes write
         load(locate(blockIdx.x));
     }
     __syncthreads();

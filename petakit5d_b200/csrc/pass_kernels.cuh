@@ -46,6 +46,14 @@ __device__ __forceinline__ void cp16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+// Programmatic dependent launch.  In a program's graph each pass starts while the one before it runs: its
+// CTAs take free slots, read the descriptors and tables (constant over the program) and stop at
+// pdl_wait() until every earlier pass is complete and visible; only then is the next pass let in, so at
+// most one pass waits beside a running one.  Every thread that reads or writes what another pass writes
+// does so behind it.  Launched without the attribute both do nothing.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -404,7 +412,14 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
         if (d.crop && !rows_meet_box(d, row0, Lc)) return;   // none of these rows has a stored voxel
     }
 
-    // ---- issue the asynchronous loads: group A = spectrum rows, group B = per-voxel inputs
+    // tables (cached in L2; nothing writes them during a program)
+    if (!G)
+        for (int i = tid; i < (P == 0 ? M : plan_tw_size(P)); i += NT) cp8(&tw[i], A.tw + i);
+    if (!odd)
+        for (int i = tid; i <= M; i += NT) cp8(&twrc[i], d.tw_rc + i);
+    pdl_wait();
+
+    // ---- issue the asynchronous loads: group A = tables and spectrum rows, group B = per-voxel inputs
     if (spec_in) {
         const int Pp = d.Pp;
         const float2* S0 = d.S + row0 * (long long)Pp;
@@ -481,11 +496,6 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
         }
     }
     cp_commit();
-    // tables (plain loads; they stay in L2)
-    if (!G)
-        for (int i = tid; i < (P == 0 ? M : plan_tw_size(P)); i += NT) tw[i] = A.tw[i];
-    if (!odd)
-        for (int i = tid; i <= M; i += NT) twrc[i] = d.tw_rc[i];
     double acc0 = 0.0, acc1 = 0.0;
     unsigned zeros = 0;
     const float lam = (mode == Y_RLPRE && d.lam_on) ? (float)d.partials[0] : 0.f;  // partials[0] = lambda
@@ -862,8 +872,12 @@ struct XZTile {
         if (conj) v.y = -v.y;
         return v;
     }
-    __device__ __forceinline__ void after_loads() const {
+    // queues the twiddles and (XZ_CONV) the OTF tile, which no pass of a program writes
+    __device__ __forceinline__ void stage_tables() const {
         const int tid = threadIdx.x;
+#pragma unroll 1
+        for (int i = tid; i < ntw; i += PK_THREADS) cp8(&tw[i], gtw + i);
+        cp_commit();
         if (gh) {
             if (T % 2 == 0 && n % 2 == 0) {   // column pairs, one 16-byte copy each: with even T, n, Pp and
                                               // column offsets, source and shared tile are 16-byte aligned
@@ -880,11 +894,10 @@ struct XZTile {
                     if (t < ncol) cp8(&h[idx], gh + e * es + t);
                 }
             }
-            cp_commit();
         }
-#pragma unroll 1
-        for (int i = tid; i < ntw; i += PK_THREADS) tw[i] = gtw[i];
+        cp_commit();
     }
+    __device__ __forceinline__ void after_loads() const { cp_wait<1>(); }   // the twiddles have landed
     __device__ __forceinline__ void before_last() const {
         cp_wait<0>();
         __syncthreads();
@@ -944,6 +957,8 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
         const XZTile g{d.S + base + k0, es, Py - k0, mode == XZ_FWD_SCALE ? d.xz_scale : 1.f, A.tw,
                        conv ? d.otf + base + k0 : nullptr, tw, hbuf, TT, kPlans[P].n, plan_tw_size(P), d.conj};
 #endif
+        g.stage_tables();
+        pdl_wait();
         if (mode == XZ_INV) fft_g<P, TT, true, true, false, true>(buf, tw, g, tid);
         else if (!conv) fft_g<P, TT, true, false, false, true>(buf, tw, g, tid);
         else if constexpr (same_end_radix(P)) {
@@ -979,6 +994,7 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
             fft_s2g<P, TT, true, true>(buf, tw, g.fenced(), tid2);
         }
     } else {
+        pdl_wait();
         for (int idx = tid; idx < P_; idx += NT) {
             const int e = idx / T, t = idx - e * T;
             if (k0 + t < Py) cp8(&buf[pad(idx)], d.S + base + e * es + k0 + t);

@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(NTH + 32, xzt_min_blocks(P, TC, NBUF, MODE == 
             pktma::tmap_acquire(&maps[v].s);
             if (CONV) pktma::tmap_acquire(&maps[v].otf);
         }
+        pdl_wait();   // the compute warps touch nothing that other passes write
         int it = 0;
         int pv[NBUF], pc[NBUF][3];   // volume and coordinates of each buffer's tile
         for (int g = blockIdx.x; g < total; g += gridDim.x, it++) {

@@ -92,6 +92,9 @@ __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)
     else if constexpr (MODE == Y_RLPRE) { src0 = d.J2; src1 = d.J3; }
     else if constexpr (MODE == Y_RLUPD) { src0 = d.Yb; src1 = d.rl_first ? nullptr : d.J4; }
     else if constexpr (MODE == Y_RLFINAL) src0 = d.Yb;
+    for (int i = tid; i < plan_tw_size(P); i += NT) tw[i] = d.ay.tw[i];
+    for (int i = tid; i <= M; i += NT) twrc[i] = d.tw_rc[i];
+    pdl_wait();
     if (tid == 0 && NAUX > 0) {
         pktma::mbar_init(bar, 1);
         pktma::fence_mbar_init();
@@ -113,8 +116,6 @@ __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = valid ? Srow[j + 16 * r] : make_float2(0.f, 0.f);
         const float2 nyq = (valid && j == 0) ? Srow[M] : make_float2(0.f, 0.f);
-        for (int i = tid; i < plan_tw_size(P); i += NT) tw[i] = d.ay.tw[i];
-        for (int i = tid; i <= M; i += NT) twrc[i] = d.tw_rc[i];
         __syncthreads();
         float2 t[R];
 #pragma unroll
@@ -137,8 +138,6 @@ __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)
         stage_r2s<R, N, LL, false, true>(buf, tid, v);                  // inverse stage 1 of 2
         stage_s2r<R, 16, N, LL, false, true, OFF1>(buf, tw, tid, v);    // stage 2: v = c at bins j + 16 r
     } else {
-        for (int i = tid; i < plan_tw_size(P); i += NT) tw[i] = d.ay.tw[i];
-        for (int i = tid; i <= M; i += NT) twrc[i] = d.tw_rc[i];
         __syncthreads();
     }
 

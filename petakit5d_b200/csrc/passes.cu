@@ -254,7 +254,7 @@ int tma_index(const PkStep& s) {
 // An x / z step can run on the register-IO kernel (k_xz, variant -1) or on a TMA variant (k_xzt:
 // 0 = the plan's 4096-point tile with two buffers; 1, 2 = the alternatives built for the plan).
 // The first time a single-volume step of a (pass, plan, size class) is seen, every candidate runs
-// once to warm up and twice timed on scratch buffers of that step's geometry (zeroed spectrum and
+// once to warm up and three times timed (the fastest counts) on scratch buffers of that step's geometry (zeroed spectrum and
 // OTF; no live data is touched); the fastest is kept for the context and appended to an on-disk
 // cache (PK_TUNE_FILE, else ~/.cache/pkdecon/tune-v6.txt), keyed by the device name, so later
 // processes skip the timing.  PK_TUNE=0 turns the timing off (the fallback choice everywhere).
@@ -402,19 +402,24 @@ int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& ge
             if (v < 0) kt.xz[s.plan]<<<grid, PK_THREADS, smem, st>>>(dd, dp, nrep, axis, s.mode);
             else t->k[s.plan][idx][v]<<<grid, t->threads[s.plan][idx][v], smem, st>>>(dd, dm, dp, nrep, ctx->d_err);
         };
-        for (int r = 0; ok && r < 1; r++) launch();
-        ok = ok && cudaEventRecord(e0, st) == cudaSuccess;
-        for (int r = 0; ok && r < 2; r++) launch();
-        const cudaError_t le = cudaGetLastError();   // a launch that failed did no work: not a candidate
-        ok = ok && cudaEventRecord(e1, st) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
-        float el = 0.f;
-        ok = ok && cudaEventElapsedTime(&el, e0, e1) == cudaSuccess;
+        launch();
+        float el = 1e30f;   // the fastest of three launches: one slow one (a clock ramp, another stream) decides nothing
+        cudaError_t le = cudaGetLastError();   // a launch that failed did no work: not a candidate
+        for (int r = 0; ok && le == cudaSuccess && r < 3; r++) {
+            ok = cudaEventRecord(e0, st) == cudaSuccess;
+            launch();
+            le = cudaGetLastError();
+            float one = 0.f;
+            ok = ok && cudaEventRecord(e1, st) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess &&
+                 cudaEventElapsedTime(&one, e0, e1) == cudaSuccess;
+            el = std::min(el, one);
+        }
         if (!ok) break;
         // a time below the pass's bytes at 10 TB/s (above any B200's HBM) means the launch did not do
         // the work either
         const double floor_ms = (double)(conv ? 3 : 2) * (double)Sb_all / 10e12 * 1e3;
-        if (le != cudaSuccess || el / 2.f < floor_ms) continue;
-        ms[ci] = el / 2.f;
+        if (le != cudaSuccess || el < floor_ms) continue;
+        ms[ci] = el;
         if (ms[ci] < best_ms) {
             best_ms = ms[ci];
             best = v;
@@ -767,6 +772,7 @@ __global__ void k_lambda(const VolDesc* __restrict__ descs, int nvol) {
     const VolDesc& d = descs[blockIdx.x];
     __shared__ double s0[256], s1[256];
     const int tid = threadIdx.x;
+    pkpass::pdl_wait();
     double a = 0.0, b = 0.0;
     for (int i = tid; i < d.blocksY; i += blockDim.x) {
         a += d.partials[2 + 2 * i];
@@ -1378,13 +1384,15 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
 // The program's launches as a graph of kernel nodes in launch order, built node by node (no stream
 // capture, so other threads' CUDA calls cannot disturb it).
 
+// pdl: passes follow each other by programmatic edges (pdl_wait in the kernels) where both sides know them;
+// a graph for device launch (flags) takes plain edges.
 static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int* d_prefix, const XZMaps* d_maps,
-                        int* d_err, cudaGraphExec_t* out, unsigned long long flags = 0, int* d_done = nullptr) {
+                        int* d_err, bool pdl, cudaGraphExec_t* out, unsigned long long flags = 0, int* d_done = nullptr) {
     const pkpass::KernelTable& kt = kernels();
     cudaGraph_t g = nullptr;
     if (cudaGraphCreate(&g, 0) != cudaSuccess) { cudaGetLastError(); return false; }
     cudaGraphNode_t prev = nullptr;
-    bool ok = true;
+    bool ok = true, prev_brief = false;
     for (const PkStep& s : prog.steps) {
         if (s.grid == 0) continue;
         const VolDesc* dd = d_desc + s.desc_off;
@@ -1442,7 +1450,20 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
             p.kernelParams = args2;
         }
         cudaGraphNode_t node = nullptr;
-        const cudaError_t ea = cudaGraphAddKernelNode(&node, g, prev ? &prev : nullptr, prev ? 1 : 0, &p);
+        // between two short passes only (128 MB of algorithmic traffic, about 20 us, each): there the next one's
+        // start hides behind this one (128x128x64 RL 1.11 -> 0.96 ms, a 2048x2048 plane 4.13 -> 3.88 ms); on
+        // long ones the early CTAs cost more than the gap (1024x1024x512 OMW 23.9 -> 26.6 ms, 512x1140x270
+        // 10.3 -> 11.4 ms)
+        const bool brief = s.kind != PK_STEP_CONV3 && pk_step_bytes(s, prog.descs.data() + s.desc_off) < 128e6;
+        const bool edge = pdl && prev && brief && prev_brief;
+        prev_brief = brief;
+        cudaError_t ea = cudaGraphAddKernelNode(&node, g, prev && !edge ? &prev : nullptr, prev && !edge ? 1 : 0, &p);
+        if (ea == cudaSuccess && edge) {
+            cudaGraphEdgeData ed = {};
+            ed.from_port = cudaGraphKernelNodePortProgrammatic;
+            ed.type = cudaGraphDependencyTypeProgrammatic;
+            ea = cudaGraphAddDependencies_v2(g, &prev, &node, &ed, 1);
+        }
         if (ea != cudaSuccess) {
             if (getenv("PK_DEBUG_GRAPHS")) fprintf(stderr, "graph node %s: %s\n", pk_step_name(s), cudaGetErrorString(ea));
             ok = false;
@@ -1471,6 +1492,12 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
     cudaGraphDestroy(g);
     if (!ok) cudaGetLastError();
     return ok;
+}
+
+// PK_NO_PDL=1: plain edges between a graph's passes (diagnostics and A/B timing)
+static bool pdl_enabled() {
+    static const bool on = !(getenv("PK_NO_PDL") && getenv("PK_NO_PDL")[0] == '1');
+    return on;
 }
 
 static bool graphs_enabled() {
@@ -1553,7 +1580,7 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
                 bool ok = cudaMalloc(&e.d, e.bytes) == cudaSuccess && cudaMallocHost(&e.h, e.bytes) == cudaSuccess &&
                           cudaEventCreateWithFlags(&e.ev, cudaEventDisableTiming) == cudaSuccess;
                 ok = ok && build_graph(prog, (const VolDesc*)e.d, (const int*)((char*)e.d + dbytes),
-                                       (const XZMaps*)((char*)e.d + moff), ctx->d_err, &e.exec);
+                                       (const XZMaps*)((char*)e.d + moff), ctx->d_err, pdl_enabled(), &e.exec);
                 if (!ok) {
                     cudaGetLastError();
                     if (e.d) cudaFree(e.d);
@@ -1605,7 +1632,7 @@ pk_status pk_program_device_graph(pk_ctx* ctx, PkProgram& prog, cudaStream_t st,
     blob_fill(prog, h);
     cudaError_t e = cudaMemcpyAsync(d, h, need, cudaMemcpyHostToDevice, st);
     bool ok = e == cudaSuccess && build_graph(prog, (const VolDesc*)d, (const int*)((char*)d + dbytes),
-                                              (const XZMaps*)((char*)d + moff), ctx->d_err, out,
+                                              (const XZMaps*)((char*)d + moff), ctx->d_err, false, out,
                                               cudaGraphInstantiateFlagDeviceLaunch, d_done);
     if (ok) {
         e = cudaGraphUpload(*out, st);
