@@ -1234,9 +1234,8 @@ void pk_program_add(PkProgram& prog, int kind, int mode, const std::vector<VolDe
     }
 }
 
-pk_status pk_program_upload(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
-    for (VolDesc& d : prog.descs) d.chk = ctx && ctx->d_err ? ctx->d_err + 1 : nullptr;
-    assign_tma(ctx, prog, st);
+// The program's blob into the next ring slot, for launches that are not a graph's.
+static pk_status program_to_slot(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
     size_t dbytes, moff, need;
     blob_layout(prog, &dbytes, &moff, &need);
     const int si = ctx->next_slot;
@@ -1265,6 +1264,15 @@ pk_status pk_program_upload(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
     prog.d_maps = (XZMaps*)((char*)sl.d + moff);
     prog.slot = si;
     return PK_OK;
+}
+
+// Fixes the kernels of the program's steps.  Its blob goes up here only when it will be launched step by step:
+// a graph keeps a blob of its own, filled when it is replayed.
+pk_status pk_program_upload(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
+    for (VolDesc& d : prog.descs) d.chk = ctx && ctx->d_err ? ctx->d_err + 1 : nullptr;
+    assign_tma(ctx, prog, st);
+    prog.slot = -1;
+    return prog.no_graph ? program_to_slot(ctx, prog, st) : PK_OK;
 }
 
 const char* pk_step_name(const PkStep& s) {
@@ -1542,7 +1550,7 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
         if (w != PK_OK) return w;
     }
     const int nk = pk_program_kernel_count(prog);
-    bool direct = !ctx || ctx->prof_on || prog.slot < 0 || prog.no_graph || !graphs_enabled() || nk < 2;
+    bool direct = !ctx || ctx->prof_on || prog.no_graph || !graphs_enabled() || nk < 2;
     if (!direct) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
@@ -1553,8 +1561,15 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
         }
     }
     pk_status rs = PK_OK;
+    auto launch_direct = [&]() {
+        if (prog.slot < 0) {
+            const pk_status us = program_to_slot(ctx, prog, st);
+            if (us != PK_OK) return us;
+        }
+        return launch_steps(ctx, prog, st);
+    };
     if (direct) {
-        rs = launch_steps(ctx, prog, st);
+        rs = launch_direct();
     } else {
         std::vector<long long> key;
         key.reserve(2 + 8 * prog.steps.size());
@@ -1569,7 +1584,7 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
         if (it == ctx->graphs.end() && ctx->graph_seen.size() >= 4096) ctx->graph_seen.clear();  // bounded
         int* seen = it == ctx->graphs.end() ? &ctx->graph_seen[key] : nullptr;
         if (seen && (*seen < 0 || (*seen)++ == 0)) {
-            rs = launch_steps(ctx, prog, st);   // first sighting (or no graph possible): launch directly
+            rs = launch_direct();   // first sighting (or no graph possible)
         } else {
             if (it == ctx->graphs.end()) {
                 if (ctx->graphs.size() >= 64) pk_release_graphs(ctx);   // bounded cache: start over
@@ -1578,7 +1593,8 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
                 pk_ctx::GraphEntry e;
                 e.bytes = total;
                 bool ok = cudaMalloc(&e.d, e.bytes) == cudaSuccess && cudaMallocHost(&e.h, e.bytes) == cudaSuccess &&
-                          cudaEventCreateWithFlags(&e.ev, cudaEventDisableTiming) == cudaSuccess;
+                          cudaEventCreateWithFlags(&e.ev, cudaEventDisableTiming) == cudaSuccess &&
+                          cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) == cudaSuccess;
                 ok = ok && build_graph(prog, (const VolDesc*)e.d, (const int*)((char*)e.d + dbytes),
                                        (const XZMaps*)((char*)e.d + moff), ctx->d_err, pdl_enabled(), &e.exec);
                 if (!ok) {
@@ -1586,23 +1602,29 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
                     if (e.d) cudaFree(e.d);
                     if (e.h) cudaFreeHost(e.h);
                     if (e.ev) cudaEventDestroy(e.ev);
+                    if (e.done) cudaEventDestroy(e.done);
                     *seen = -1;   // never try this program again
-                    rs = launch_steps(ctx, prog, st);
+                    rs = launch_direct();
                 } else {
                     it = ctx->graphs.emplace(key, e).first;
                 }
             }
             if (it != ctx->graphs.end()) {
                 pk_ctx::GraphEntry& e = it->second;
-                if (e.used) PK_CUDA(cudaEventSynchronize(e.ev));   // the previous refresh has been read
+                // the host copy may be refilled once the previous refresh has read it (not only when that replay is
+                // done: a queued call's descriptors are ready when the GPU gets there); the device copy is
+                // refreshed behind the previous replay, whatever stream that ran on
+                if (e.used) PK_CUDA(cudaEventSynchronize(e.ev));
                 blob_fill(prog, e.h);
+                if (e.used) PK_CUDA(cudaStreamWaitEvent(st, e.done, 0));
                 {
                     const pk_status bs = blob_upload(ctx, e.d, e.h, e.bytes, st);
                     if (bs != PK_OK) return bs;
                 }
-                PK_CUDA(cudaGraphLaunch(e.exec, st));
                 PK_CUDA(cudaEventRecord(e.ev, st));
                 e.used = true;
+                PK_CUDA(cudaGraphLaunch(e.exec, st));
+                PK_CUDA(cudaEventRecord(e.done, st));
             }
         }
     }
@@ -1670,11 +1692,12 @@ pk_status pk_program_launch_range(pk_ctx* ctx, PkProgram& prog, cudaStream_t st,
 void pk_release_graphs(pk_ctx* ctx) {
     for (auto& kv : ctx->graphs) {
         pk_ctx::GraphEntry& e = kv.second;
-        if (e.ev) cudaEventSynchronize(e.ev);
+        if (e.used) cudaEventSynchronize(e.done);
         if (e.exec) cudaGraphExecDestroy(e.exec);
         if (e.d) cudaFree(e.d);
         if (e.h) cudaFreeHost(e.h);
         if (e.ev) cudaEventDestroy(e.ev);
+        if (e.done) cudaEventDestroy(e.done);
     }
     ctx->graphs.clear();
     ctx->graph_seen.clear();

@@ -205,7 +205,8 @@ struct pk_ctx {
         void* d = nullptr;
         void* h = nullptr;
         size_t bytes = 0;
-        cudaEvent_t ev = nullptr;
+        cudaEvent_t ev = nullptr;     // the last refresh has read the host copy
+        cudaEvent_t done = nullptr;   // the last replay is done
         bool used = false;
     };
     std::map<std::vector<long long>, GraphEntry> graphs;
