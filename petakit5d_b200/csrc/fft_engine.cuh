@@ -236,9 +236,123 @@ __device__ void stage_generic(float2* __restrict__ buf, const float2* __restrict
     __syncthreads();
 }
 
+// ---- the same sums for the lengths of stage_direct: the products' roots come from a table laid out for them
+//
+// Two outputs to a packed instruction (mul / fma / add.f32x2 round each half as the scalar ones do).
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2 un2(unsigned long long a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+
+// Floats of one row of a stage's root matrix: the cosines of its R outputs, then their sines, each rounded up
+// to whole 16-byte groups.
+__host__ __device__ constexpr int direct_half(int R) { return (R + 3) & ~3; }
+
+// Prime-factor stage R of lines of which CL at a time (CL divides g.L) are summed by one thread for four
+// outputs: out[j, s] = sum_q in[j + q n/R] W_{Ns R}^{q (k + Ns s)}, k = j mod Ns, in the order and with the
+// roundings of stage_generic (x * w as fma(x.x, w.x, -(x.y w.y)), fma(x.x, w.y, x.y w.x); for the inverse
+// fma(x.x, w.x, x.y w.y), fma(x.y, w.x, -(x.x w.y)), from conjugated inputs and sums).  At such lengths the
+// sums' rounding (6e-6 of the result after 10 RL iterations at 467) is as large as what a faster algorithm
+// changes (Bluestein's chirp took 0.17 ms for the x pass below, with results up to 5e-3 of their RMS away at single
+// voxels, where this rounding itself is as far from the truth), so results stay what they were.
+// mat[k][q]: the four outputs' roots are one 16-byte load each of cosines and sines, the same for every column,
+// from L1 / L2; x: the tile with each part twice, (re, re, im, im), so an input's products need no moves.
+// Bound by the FMA pipe (58% active; a packed instruction takes it for two cycles): 467-long x pass of
+// 301 x 467 x 97 2.18 -> 1.16 ms, 97-long z convolution 1.11 -> 0.68 ms, y ratio of 301-voxel rows 1.36 -> 0.92 ms.
+// Eight columns a thread left too few warps (1.32 ms).
+template <bool INV, int CL>
+__device__ __noinline__ void stage_direct(float2* __restrict__ buf, float4* __restrict__ x, const float* __restrict__ mat,
+                                          const TileGeom& g, int R, int Ns, int tid, int nthr) {
+    const int m = g.n / R, L = g.L;
+    for (int i = tid; i < L * g.n; i += nthr) {
+        int l, e;
+        if (g.lineFast) { e = i / L; l = i - e * L; }
+        else { l = i / g.n; e = i - l * g.n; }
+        const float2 v = buf[pad(l * g.ls + e * g.es)];
+        const float im = INV ? -v.y : v.y;
+        x[e * L + l] = make_float4(v.x, v.x, im, im);
+    }
+    __syncthreads();
+    const unsigned long long neg = 0x8000000080000000ull;
+    const int half = direct_half(R), ng = half / 4, nc = L / CL;
+    const int items = m * nc * ng;
+    for (int it = tid; it < items; it += nthr) {
+        const int rest = it / ng, s0 = 4 * (it - rest * ng), j = rest / nc, c0 = CL * (rest - j * nc);
+        const int k = j % Ns;
+        const float* __restrict__ w = mat + (size_t)k * R * (2 * half) + s0;
+        const float4* __restrict__ xp = x + j * L + c0;
+        unsigned long long ar[2][CL], ai[2][CL];
+#pragma unroll
+        for (int u = 0; u < CL; u++) ar[0][u] = ar[1][u] = ai[0][u] = ai[1][u] = 0ull;
+        // the roots of the next two inputs are in flight while one input's products are formed
+        constexpr int AHEAD = 2;
+        ulonglong2 c[AHEAD], s[AHEAD];
+#pragma unroll
+        for (int t = 0; t < AHEAD; t++) {   // R >= 7
+            c[t] = __ldg(reinterpret_cast<const ulonglong2*>(w + t * 2 * half));
+            s[t] = __ldg(reinterpret_cast<const ulonglong2*>(w + t * 2 * half + half));
+        }
+        w += AHEAD * 2 * half;
+        for (int q0 = 0; q0 < R; q0 += AHEAD) {
+#pragma unroll
+            for (int t = 0; t < AHEAD; t++) {
+                if (q0 + t < R) {
+                    const ulonglong2 cq = c[t], sq = s[t];
+                    if (q0 + t + AHEAD < R) {
+                        c[t] = __ldg(reinterpret_cast<const ulonglong2*>(w));
+                        s[t] = __ldg(reinterpret_cast<const ulonglong2*>(w + half));
+                        w += 2 * half;
+                    }
+#pragma unroll
+                    for (int u = 0; u < CL; u++) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xp + u);
+                        const unsigned long long nv = v.y ^ neg;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const unsigned long long cc = h ? cq.y : cq.x, ss = h ? sq.y : sq.x;
+                            ar[h][u] = add2(ar[h][u], fma2(v.x, cc, mul2(nv, ss)));
+                            ai[h][u] = add2(ai[h][u], INV ? fma2(v.y, cc, mul2(v.x, ss)) : fma2(v.x, ss, mul2(v.y, cc)));
+                        }
+                    }
+                    xp += m * L;
+                }
+            }
+        }
+        const int o0 = (j - k) * R + k;
+#pragma unroll
+        for (int u = 0; u < CL; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float2 re = un2(ar[h][u]), im = un2(ai[h][u]);
+                const int so = s0 + 2 * h, a = (c0 + u) * g.ls + (o0 + Ns * so) * g.es;
+                if (so < R) buf[pad(a)] = make_float2(re.x, INV ? -im.x : im.x);
+                if (so + 1 < R) buf[pad(a + Ns * g.es)] = make_float2(re.y, INV ? -im.y : im.y);
+            }
+    }
+    __syncthreads();
+}
+
 // Full transform of the tile's L lines (unnormalised; INV = +i sign).
-template <bool INV>
-__device__ void fft_lines(float2* buf, const AxisDev& A, const float2* tw, const TileGeom& g, int tid, int nthr) {
+// x (DIRECT): room for g.L n float4 beside the tile.
+template <bool INV, bool DIRECT = false>
+__device__ void fft_lines(float2* buf, const AxisDev& A, const float2* tw, const TileGeom& g, int tid, int nthr,
+                          float4* x = nullptr) {
     int Ns = 1;
     for (int s = 0; s < A.nst; s++) {
         const int R = A.rad[s];
@@ -249,7 +363,13 @@ __device__ void fft_lines(float2* buf, const AxisDev& A, const float2* tw, const
             case 5: stage<5, INV>(buf, tw, A.twStride, g, Ns, tid, nthr); break;
             case 8: stage<8, INV>(buf, tw, A.twStride, g, Ns, tid, nthr); break;
             case 16: stage<16, INV>(buf, tw, A.twStride, g, Ns, tid, nthr); break;
-            default: stage_generic<INV>(buf, tw, A.twStride, g, R, Ns, tid, nthr); break;
+            default:
+                if constexpr (DIRECT) {
+                    stage_direct<INV, 4>(buf, x, A.gen->mat + A.gen->off[s], g, R, Ns, tid, nthr);
+                } else {
+                    stage_generic<INV>(buf, tw, A.twStride, g, R, Ns, tid, nthr);
+                }
+                break;
         }
         Ns *= R;
     }

@@ -5,18 +5,12 @@
 //  * Lengths whose prime factors are at most 31 run as Stockham stages of the radices below; primes
 //    above 5 use the symmetric form of the DFT with the roots as immediates (a quarter of the
 //    multiply-adds of the plain sum, no table reads), composites are nested in registers.
-//  * Other lengths run as Bluestein's chirp transform (L. Bluestein, 1970): n points become a circular
-//    convolution of a length L >= 2 n - 1 with small factors.  The chirp multiplies, the zero padding
-//    and the pointwise product ride on the loads and stores of the first and last stages.
+//  * Lengths with a larger prime factor keep the in-place engine's sums (stage_direct of fft_engine.cuh).
 //
 // Stages go from one shared-memory buffer to another, so a stage takes one barrier and its loop is not
 // limited by what a thread can hold in registers.  The inverse transform is the forward one on
 // swapped re/im, swapped back: the swaps ride on the first load and the last store, and only
-// forward butterflies are instantiated.
-//
-// A direct sum over a large prime factor p costs p complex multiply-adds per point: the y pass of 301-voxel
-// rows took 1.36 ms (ratio) on the in-place engine and takes 0.59 ms here, with two real rows of odd length
-// in one complex transform.  pass_gen.cuh has the figures of the x / z passes.
+// forward butterflies are instantiated.  pass_gen.cuh has the figures of the x / z passes.
 #pragma once
 #include <type_traits>
 #include <utility>
@@ -71,8 +65,36 @@ __device__ __forceinline__ void bf_small(float2* v) {
     else bf16<false>(v);
 }
 
-// Forward DFT of R registers; emit(q, X[q]) takes the outputs (a prime radix hands each pair on as it
-// is formed, so it never holds R outputs beside its R inputs).
+// Forward DFT of odd length R in its symmetric form: with a_m = v_m + v_{R-m}, b_m = v_m - v_{R-m}, X_q and
+// X_{R-q} = t1 +- (t2.y, -t2.x) for t1 = v_0 + sum_m a_m cos, t2 = sum_m b_m sin.  emit(q, X[q]) takes each pair
+// as it is formed, so R outputs are never held beside the inputs.
+template <int R, class E>
+__device__ __forceinline__ void bf_odd(float2* v, E&& emit) {
+    constexpr int H = (R - 1) / 2;
+    float2 a[H], b[H];
+    float2 y0 = v[0];
+    static_for<H>([&](auto i) {
+        a[i.value] = cadd(v[i.value + 1], v[R - 1 - i.value]);
+        b[i.value] = csub(v[i.value + 1], v[R - 1 - i.value]);
+        y0 = cadd(y0, a[i.value]);
+    });
+    emit(0, y0);
+    static_for<H>([&](auto qi) {
+        constexpr int q = qi.value + 1;
+        float2 t1 = v[0], t2 = make_float2(0.f, 0.f);
+        static_for<H>([&](auto i) {
+            constexpr int e = (q * (i.value + 1)) % R;
+            t1.x += a[i.value].x * kCos<e, R>;
+            t1.y += a[i.value].y * kCos<e, R>;
+            t2.x += b[i.value].x * kSin<e, R>;
+            t2.y += b[i.value].y * kSin<e, R>;
+        });
+        emit(q, make_float2(t1.x + t2.y, t1.y - t2.x));
+        emit(R - q, make_float2(t1.x - t2.y, t1.y + t2.x));
+    });
+}
+
+// Forward DFT of R registers; emit(q, X[q]) takes the outputs.
 template <int R, class E>
 __device__ __forceinline__ void butterfly(float2* v, E&& emit) {
     if constexpr (simple_radix(R)) {
@@ -99,29 +121,7 @@ __device__ __forceinline__ void butterfly(float2* v, E&& emit) {
             static_for<B>([&](auto q) { emit(p.value + A * q.value, u[q.value]); });
         });
     } else {
-        // odd prime: with a_m = v_m + v_{R-m}, b_m = v_m - v_{R-m}: X_q, X_{R-q} = t1 +- (t2.y, -t2.x)
-        constexpr int H = (R - 1) / 2;
-        float2 a[H], b[H];
-        float2 y0 = v[0];
-        static_for<H>([&](auto i) {
-            a[i.value] = cadd(v[i.value + 1], v[R - 1 - i.value]);
-            b[i.value] = csub(v[i.value + 1], v[R - 1 - i.value]);
-            y0 = cadd(y0, a[i.value]);
-        });
-        emit(0, y0);
-        static_for<H>([&](auto qi) {
-            constexpr int q = qi.value + 1;
-            float2 t1 = v[0], t2 = make_float2(0.f, 0.f);
-            static_for<H>([&](auto i) {
-                constexpr int e = (q * (i.value + 1)) % R;
-                t1.x += a[i.value].x * kCos<e, R>;
-                t1.y += a[i.value].y * kCos<e, R>;
-                t2.x += b[i.value].x * kSin<e, R>;
-                t2.y += b[i.value].y * kSin<e, R>;
-            });
-            emit(q, make_float2(t1.x + t2.y, t1.y - t2.x));
-            emit(R - q, make_float2(t1.x - t2.y, t1.y + t2.x));
-        });
+        bf_odd<R>(v, emit);
     }
 }
 
@@ -139,12 +139,10 @@ struct GenEdge {
     float sc;                // factor of the results
 };
 
-// Loads of a first stage: as stored; swapped (inverse); * OTF, swapped; [swapped,] * chirp, zero past
-// n; * filter, swapped (the chirp transform's second round); * OTF, swapped, * chirp; any of them,
-// chosen at run time (transforms of one stage).  Stores of a last stage: as computed; [swapped,] scaled;
-// swapped, * chirp, [swapped,] scaled, up to n; any.
-enum GenIn { GI_PLAIN, GI_SWAP, GI_OTF, GI_CHIRP, GI_BK, GI_OTFCHIRP, GI_ANY };
-enum GenOut { GO_PLAIN, GO_SCALE, GO_CHIRP, GO_ANY };
+// Loads of a first stage: as stored; swapped (inverse); * OTF, swapped; any of them, chosen at run time
+// (transforms of one stage).  Stores of a last stage: as computed; [swapped,] scaled; either.
+enum GenIn { GI_PLAIN, GI_SWAP, GI_OTF, GI_ANY };
+enum GenOut { GO_PLAIN, GO_SCALE, GO_ANY };
 
 // Word of element (l, e): column tiles (LF) hold a row of T columns per element, dense as TMA lays it
 // out; row tiles hold lines one after the other.  Neither needs spare slots: the first radix is odd, so
@@ -152,20 +150,16 @@ enum GenOut { GO_PLAIN, GO_SCALE, GO_CHIRP, GO_ANY };
 template <bool LF>
 __device__ __forceinline__ int word(int l, int e, int ls) { return LF ? e * ls + l : l * ls + e; }
 
-// One Stockham stage of radix R over `lines` lines.  nin / nout: line strides of the buffers of a row
-// tile; elements at or past lin read as zero, those past lout are not stored (the chirp's padding).
+// One Stockham stage of radix R over `lines` lines.
 template <int R, bool LF, int IN, int OUT>
 __device__ __forceinline__ void gstage(const float2* __restrict__ in, float2* __restrict__ out, const GenAxis& A, int s,
                                        int lines, int lt, const GenEdge& g, int kin, int kout, int tid, int nthr) {
-    const int m = A.m[s], Ns = A.ns[s], n = A.n, L = A.L;
+    const int m = A.m[s], Ns = A.ns[s];
     const unsigned mg_ns = A.mg_ns[s], mg_m = A.mg_m[s];
     const float2* __restrict__ tw = A.tw + A.off[s];
-    const float2* __restrict__ chirp = A.chirp;
     const int B = lines * m;
     const int in_kind = IN == GI_ANY ? kin : IN, out_kind = OUT == GO_ANY ? kout : OUT;
-    const bool i_otf = in_kind == GI_OTF || in_kind == GI_OTFCHIRP, i_chirp = in_kind == GI_CHIRP || in_kind == GI_OTFCHIRP;
-    const bool i_swap = in_kind != GI_PLAIN && (in_kind != GI_CHIRP || g.inv);
-    const int lsi = LF ? lines : (i_chirp ? n : L), lso = LF ? lines : (out_kind == GO_CHIRP ? n : L);
+    const int ls = LF ? lines : A.n;
     for (int b = tid; b < B; b += nthr) {
         int l, j;
         if constexpr (LF) {
@@ -177,37 +171,23 @@ __device__ __forceinline__ void gstage(const float2* __restrict__ in, float2* __
         }
         const int k = Ns > 1 ? j - fdiv(j, mg_ns) * Ns : 0;
         float2 v[R];
-        if (i_otf) {
+        if (in_kind == GI_OTF) {
             // every OTF element is requested before the first is used; columns past the spectrum's
             // (never stored) take the last valid one
             const float2* __restrict__ hp = g.otf + min(l, g.ncol - 1);
 #pragma unroll
-            for (int r = 0; r < R; r++) v[r] = j + r * m < n ? __ldg(hp + (j + r * m) * g.es) : make_float2(0.f, 0.f);
+            for (int r = 0; r < R; r++) v[r] = __ldg(hp + (j + r * m) * g.es);
             const float sg = g.conj ? -1.f : 1.f;
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const int e = j + r * m;
-                const float2 x = !i_chirp || e < n ? in[word<LF>(l, e, lsi)] : make_float2(0.f, 0.f);
-                v[r] = swp(cmul(x, make_float2(v[r].x, sg * v[r].y)));
-            }
+            for (int r = 0; r < R; r++)
+                v[r] = swp(cmul(in[word<LF>(l, j + r * m, ls)], make_float2(v[r].x, sg * v[r].y)));
         } else {
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const int e = j + r * m;
-                v[r] = !i_chirp || e < n ? in[word<LF>(l, e, lsi)] : make_float2(0.f, 0.f);
-            }
-            if (in_kind == GI_BK) {
-#pragma unroll
-                for (int r = 0; r < R; r++) v[r] = cmul(v[r], __ldg(A.bk + j + r * m));
-            }
-            if (i_swap) {
+            for (int r = 0; r < R; r++) v[r] = in[word<LF>(l, j + r * m, ls)];
+            if (in_kind == GI_SWAP) {
 #pragma unroll
                 for (int r = 0; r < R; r++) v[r] = swp(v[r]);
             }
-        }
-        if (i_chirp) {
-#pragma unroll
-            for (int r = 0; r < R; r++) v[r] = cmul(v[r], __ldg(chirp + min(j + r * m, n - 1)));
         }
         if (Ns > 1) {
             // the butterfly's R - 1 twiddles lie side by side: one address, 16-byte loads
@@ -222,24 +202,17 @@ __device__ __forceinline__ void gstage(const float2* __restrict__ in, float2* __
         const int o0 = (j - k) * R + k;
         butterfly<R>(v, [&](int q, float2 x) {
             const int e = o0 + q * Ns;
-            if (out_kind == GO_CHIRP) {
-                if (e < n) {
-                    x = cmul(swp(x), __ldg(chirp + e));
-                    if (g.inv) x = swp(x);
-                    out[word<LF>(l, e, lso)] = make_float2(x.x * g.sc, x.y * g.sc);
-                }
-            } else if (out_kind == GO_SCALE) {
+            if (out_kind == GO_SCALE) {
                 if (g.inv) x = swp(x);
-                out[word<LF>(l, e, lso)] = make_float2(x.x * g.sc, x.y * g.sc);
-            } else {
-                out[word<LF>(l, e, lso)] = x;
+                x = make_float2(x.x * g.sc, x.y * g.sc);
             }
+            out[word<LF>(l, e, ls)] = x;
         });
     }
 }
 
-// Stages by radix.  First stages take an odd radix, and those of a chirp transform one of its smooth
-// length's; BIG adds the radices above 16 (kernels without them run with fewer registers).
+// Stages by radix.  First stages take an odd radix; BIG adds the radices above 16 (kernels without them run
+// with fewer registers).
 #define PK_GS_CASE(R, I, O) \
     case R: gstage<R, LF, I, O>(in, out, *A, s, lines, lt, *g, kin, kout, tid, nthr); break;
 #define PK_GS_EVEN(I, O) \
@@ -257,7 +230,7 @@ __device__ __forceinline__ void gstage(const float2* __restrict__ in, float2* __
     const float2 *in, float2 *out, const GenAxis *A, int s, int lines, int lt, const GenEdge *g, int kin, int kout, int tid, \
         int nthr
 
-template <bool LF, bool BIG, int IN>   // first of several stages, not a chirp's
+template <bool LF, bool BIG, int IN>   // first of several stages
 __device__ __noinline__ void gs_first(PK_GS_ARGS) {
     const int rad = A->rad[s];
     switch (rad) {
@@ -265,26 +238,12 @@ __device__ __noinline__ void gs_first(PK_GS_ARGS) {
         default: PK_GS_BIG(IN, GO_PLAIN) break;
     }
 }
-template <bool LF, int IN>             // first stage of a chirp round
-__device__ __noinline__ void gs_chirp(PK_GS_ARGS) {
-    switch (A->rad[s]) {
-        PK_GS_SMOOTH(IN, GO_PLAIN)
-        default: break;
-    }
-}
 template <bool LF, bool BIG, int OUT>  // middle (OUT = GO_PLAIN) or last of several stages
 __device__ __noinline__ void gs_rest(PK_GS_ARGS) {
     const int rad = A->rad[s];
     switch (rad) {
-        PK_GS_EVEN(GI_PLAIN, OUT) PK_GS_SMOOTH(GI_PLAIN, OUT)
-        default:
-            if constexpr (OUT != GO_CHIRP) {
-                switch (rad) {
-                    PK_GS_MID(GI_PLAIN, OUT)
-                    default: PK_GS_BIG(GI_PLAIN, OUT) break;
-                }
-            }
-            break;
+        PK_GS_EVEN(GI_PLAIN, OUT) PK_GS_SMOOTH(GI_PLAIN, OUT) PK_GS_MID(GI_PLAIN, OUT)
+        default: PK_GS_BIG(GI_PLAIN, OUT) break;
     }
 }
 template <bool LF, bool BIG>           // the only stage of a transform
@@ -307,39 +266,29 @@ __device__ __forceinline__ float2* gen_transform(const GenAxis* A, const float2*
     const int nst = A->nst;
     const float2* in = src;
     float2* out = src == b0 ? b1 : b0;
-    const int blue = A->blue, rounds = blue ? 2 : 1;
-    const bool otf = LF && edge.otf;
-    for (int q = 0; q < rounds; q++) {
-        const bool end = q == rounds - 1;
-        const int kin = q == 1 ? GI_BK : blue ? (otf ? GI_OTFCHIRP : GI_CHIRP) : otf ? GI_OTF : edge.inv ? GI_SWAP : GI_PLAIN;
-        const int kout = !end ? GO_PLAIN : blue ? GO_CHIRP : (edge.inv || edge.sc != 1.f) ? GO_SCALE : GO_PLAIN;
-        for (int s = 0; s < nst; s++) {
+    const int kin = LF && edge.otf ? GI_OTF : edge.inv ? GI_SWAP : GI_PLAIN;
+    const int kout = edge.inv || edge.sc != 1.f ? GO_SCALE : GO_PLAIN;
+    for (int s = 0; s < nst; s++) {
 #define PK_GS_CALL(F) F(in, out, A, s, lines, lt, &edge, kin, kout, tid, nthr)
-            if (nst == 1) {
-                PK_GS_CALL((gs_only<LF, BIG>));
-            } else if (s == 0) {
-                if (kin == GI_PLAIN) PK_GS_CALL((gs_first<LF, BIG, GI_PLAIN>));
-                else if (kin == GI_SWAP) PK_GS_CALL((gs_first<LF, BIG, GI_SWAP>));
-                else if (kin == GI_CHIRP) PK_GS_CALL((gs_chirp<LF, GI_CHIRP>));
-                else if (kin == GI_BK) PK_GS_CALL((gs_chirp<LF, GI_BK>));
-                if constexpr (LF) {
-                    if (kin == GI_OTF) PK_GS_CALL((gs_first<LF, BIG, GI_OTF>));
-                    else if (kin == GI_OTFCHIRP) PK_GS_CALL((gs_chirp<LF, GI_OTFCHIRP>));
-                }
-            } else if (s < nst - 1 || kout == GO_PLAIN) {
-                PK_GS_CALL((gs_rest<LF, BIG, GO_PLAIN>));
-            } else if (kout == GO_SCALE) {
-                PK_GS_CALL((gs_rest<LF, BIG, GO_SCALE>));
-            } else {
-                PK_GS_CALL((gs_rest<LF, BIG, GO_CHIRP>));
+        if (nst == 1) {
+            PK_GS_CALL((gs_only<LF, BIG>));
+        } else if (s == 0) {
+            if (kin == GI_PLAIN) PK_GS_CALL((gs_first<LF, BIG, GI_PLAIN>));
+            else if (kin == GI_SWAP) PK_GS_CALL((gs_first<LF, BIG, GI_SWAP>));
+            if constexpr (LF) {
+                if (kin == GI_OTF) PK_GS_CALL((gs_first<LF, BIG, GI_OTF>));
             }
-#undef PK_GS_CALL
-            if (s == 0 && q == 0) before_sync();
-            __syncthreads();
-            if (s == 0 && q == 0) after_first();
-            in = out;
-            out = out == b0 ? b1 : b0;
+        } else if (s < nst - 1 || kout == GO_PLAIN) {
+            PK_GS_CALL((gs_rest<LF, BIG, GO_PLAIN>));
+        } else {
+            PK_GS_CALL((gs_rest<LF, BIG, GO_SCALE>));
         }
+#undef PK_GS_CALL
+        if (s == 0) before_sync();
+        __syncthreads();
+        if (s == 0) after_first();
+        in = out;
+        out = out == b0 ? b1 : b0;
     }
     return const_cast<float2*>(in);
 }

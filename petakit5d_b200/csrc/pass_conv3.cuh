@@ -27,29 +27,6 @@
 
 namespace pkpass {
 
-// first stage from registers: v[i][r] is element j + r (N / R) of column l; butterfly, store
-template <int R, int N, int L, bool INV, int NTH>
-__device__ __forceinline__ void dstage_r2s(float2* __restrict__ buf, int tid,
-                                           float2 (&v)[(L * (N / R) + NTH - 1) / NTH][R]) {
-    static_assert(!direct_radix(R), "first stage needs a register butterfly");
-    constexpr int M = N / R;
-    constexpr int B = L * M;
-    constexpr int NT = NTH;
-    constexpr int MAXB = (B + NT - 1) / NT;
-#pragma unroll
-    for (int i = 0; i < MAXB; i++) {
-        const int b = tid + i * NT;
-        if (B % NT == 0 || b < B) {
-            const int l = b % L, j = b / L;
-            bfly<R, INV>(v[i]);
-            const int a0 = j * R * L + l;
-#pragma unroll
-            for (int r = 0; r < R; r++) buf[a0 + r * L] = v[i][r];
-        }
-    }
-    compute_bar<NTH>();
-}
-
 enum { C3_X = 0, C3_Z = 1, C3_I = 2 };
 
 // Sequence index -> item: type, column tile c, line o (z for X / I items, x for Z items).  The

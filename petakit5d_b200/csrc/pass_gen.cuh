@@ -7,11 +7,9 @@
 // store that the next tile's first stage overlaps.  Elements past the line's end in the last box and
 // past Py in the last tile are zero-filled on load and clipped on store.
 //
-// Bound by instruction issue (0.54-0.58 of the issue slots at 24 warps an SM), not by memory: the stages
-// over a chirp length twice n, twice a transform, cost about 37 instructions a point each.  Measured
-// against the in-place engine of k_xz (direct sums over prime factors, tiles of 4096 / n columns):
-//   301 x 467 x 97:   x (467, chirp) 2.18 -> 0.165 ms, z convolution (97, chirp) 1.11 -> 0.295 ms
-//   512 x 1140 x 270: x (1140 = 19 * 15 * 4) 2.40 -> 0.48 ms, z convolution (270) 3.80 -> 0.96 ms
+// Mixed radices: bound by instruction issue (0.54-0.58 of the issue slots at 24 warps an SM), not by memory.
+// Measured against the in-place engine of k_xz (sums over prime factors, tiles of 4096 / n columns), on
+// 512 x 1140 x 270: x (1140 = 19 * 15 * 4) 2.40 -> 0.48 ms, z convolution (270) 3.80 -> 0.96 ms.
 // The OTF is read straight from memory by the inverse's first stage (all its loads are issued before the
 // first is used); a run-time choice of what each load and store does, element by element, took 3.42 ms there.
 #pragma once
@@ -26,10 +24,10 @@ constexpr int kGenThreads = 256;
 // Elements of a tile's landing buffer and of each of its two stage buffers (whole boxes: the result
 // leaves from a stage buffer box by box), in multiples of 128 bytes; a launch takes the largest of its volumes.
 inline int gen_land(const GenAxis& A) { return (A.T * A.rows * A.nbox + 15) & ~15; }
-inline int gen_work(const GenAxis& A) { return (A.T * (A.L > A.rows * A.nbox ? A.L : A.rows * A.nbox) + 15) & ~15; }
+inline int gen_work(const GenAxis& A) { return (A.T * A.rows * A.nbox + 15) & ~15; }
 inline size_t gen_smem(int land, int work) { return 256 + sizeof(float2) * ((size_t)land + 2 * (size_t)work); }
 
-struct GenKernel {   // [0]: radices up to 16, [1]: all
+struct GenKernel {   // [0]: radices up to 16, [1]: up to 31
     void (*fn[2])(const VolDesc*, const XZMaps*, const int*, int, int, int, int, int, int*);
 };
 

@@ -361,10 +361,11 @@ __host__ __device__ inline int y_aux_arrays(int mode) {
 // (even, so that what follows stays on a 16-byte boundary).
 __host__ __device__ inline int gen_y_slots(int lines, int len) { return (lines * len + 1) & ~1; }
 
-// GEN (P = 0): 1 and 2 run lengths without a plan on the mixed-radix / chirp engine (gen_engine.cuh; 2: with
-// its radices above 16), 0 on the in-place run-time engine.
+// GEN (P = 0): 1 and 2 run lengths without a plan on the mixed-radix engine (gen_engine.cuh; 2: with
+// its radices above 16), 3 those with a prime factor above 31 on the in-place engine with stage_direct, 0 others
+// on the plain in-place engine.
 template <int P, int MODE, int TP = PK_TILE_POINTS, int GEN = 0>
-__global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
+__global__ void __launch_bounds__(PK_THREADS, GEN >= 2 ? 2 : 3) k_y(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
                                                      int nvol, int) {
     constexpr int mode = MODE;   // one kernel per mode: only that mode's code is in the kernel
     extern __shared__ float2 smem[];
@@ -378,15 +379,16 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
     const int L = P == 0 ? d.Ly : plan_lines_y(kPlans[P].n, TP);
     const bool odd = d.odd;
     const int Py = d.Py, ny = d.ny;
-    // lengths without a plan run the mixed-radix / chirp engine on two buffers of its L points a line
-    const GenAxis* const G = P == 0 ? A.gen : nullptr;
+    // lengths without a plan run the mixed-radix engine on two buffers of M points a line
+    constexpr bool MIXED = GEN == 1 || GEN == 2;
+    const GenAxis* const G = MIXED ? A.gen : nullptr;
     // odd ny: the odd rows of a pair travel as the imaginary part of the even ones (two real transforms in one)
-    const bool pairs = GEN && odd;
+    const bool pairs = MIXED && odd;
     const int lines = pairs ? (L + 1) / 2 : L;   // complex lines of a full tile
-    const int bufn = GEN ? gen_y_slots(lines, odd ? max(G->L, M + 1) : G->L) : padded_size(L * M);
+    const int bufn = MIXED ? gen_y_slots(lines, odd ? M + 1 : M) : padded_size(L * M);
     const pkgen::FastDiv divM(M), divPy(Py);
     auto line_of = [&](int idx) { return P == 0 ? divM(idx) : idx / M; };
-    auto slot = [](int a) { return GEN ? a : pad(a); };   // the tile's word of element a
+    auto slot = [](int a) { return MIXED ? a : pad(a); };   // the tile's word of element a
     // shared memory: tw[tw_slots(M)] (not with G) | twrc[M+1] (even ny) | buf[padded L*M] | second buf (G) | nyq[L]
     // | aux0[L*M] | aux1[L*M]
     float2* tw = smem;
@@ -398,6 +400,8 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
     float2* aux0 = nyq + L;
     const int auxn = pairs ? gen_y_slots(L, M) / 2 : L * M;   // pairs of odd rows: one float a voxel
     float2* aux1 = aux0 + auxn;
+    // GEN 3: the sums' doubled inputs, on the next 16-byte boundary
+    float4* const xbuf = (float4*)(((uintptr_t)(aux0 + y_aux_arrays(mode) * auxn) + 15) & ~(uintptr_t)15);
     auto aux = [&](const float2* p, int idx) {
         return pairs ? make_float2(reinterpret_cast<const float*>(p)[idx], 0.f) : p[idx];
     };
@@ -704,10 +708,12 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
     pkgen::GenEdge ge{};
     ge.sc = 1.f;
     if (spec_in) {
-        if constexpr (GEN > 0) {
+        if constexpr (MIXED) {
             ge.inv = 1;
             buf = pkgen::gen_transform<false, GEN == 2>(G, buf, gb0, gb1, pairs ? (Lc + 1) / 2 : Lc, 0, ge, tid, NT, [] {}, [] {});
             ge.inv = 0;
+        } else if constexpr (GEN == 3) {
+            fft_lines<true, true>(buf, A, tw, TileGeom{L, A.n, A.n, 1, false}, tid, NT, xbuf);
         } else {
             fft_y<P, true, TP>(buf, A, tw, L, tid);
         }
@@ -742,8 +748,10 @@ __global__ void __launch_bounds__(PK_THREADS, GEN == 2 ? 2 : 3) k_y(const VolDes
         for (int k = tid; k < M; k += NT) buf[slot((Lc >> 1) * M + k)].y = 0.f;
     if (spec_out) {
         __syncthreads();
-        if constexpr (GEN > 0) {
+        if constexpr (MIXED) {
             buf = pkgen::gen_transform<false, GEN == 2>(G, buf, gb0, gb1, pairs ? (Lc + 1) / 2 : Lc, 0, ge, tid, NT, [] {}, [] {});
+        } else if constexpr (GEN == 3) {
+            fft_lines<false, true>(buf, A, tw, TileGeom{L, A.n, A.n, 1, false}, tid, NT, xbuf);
         } else {
             fft_y<P, false, TP>(buf, A, tw, L, tid);
         }
@@ -919,8 +927,10 @@ constexpr int xz_min_blocks(int p) {
     return p > 0 && kPlans[p].n == 512 ? 4 : 3;
 }
 
-template <int P, int TP = PK_TILE_POINTS>
-__global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
+// DIRECT (P = 0): lengths with a prime factor above 31 (stage_direct); the OTF is read where it is used.
+constexpr int kDirectSmem = 220 * 1024;   // beside the static sums of Y_RLUPD
+template <int P, int TP = PK_TILE_POINTS, bool DIRECT = false>
+__global__ void __launch_bounds__(PK_THREADS, DIRECT ? 2 : xz_min_blocks(P)) k_xz(const VolDesc* __restrict__ descs, const int* __restrict__ prefix,
                                                       int nvol, int axis, int mode) {
     extern __shared__ float2 smem[];
     constexpr int NT = PK_THREADS;
@@ -930,7 +940,7 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
     const int tid = threadIdx.x;
     const AxisDev& A = axis == 1 ? d.ax : d.az;
     const int n = P == 0 ? A.n : kPlans[P].n;
-    const int T = P == 0 ? (axis == 1 ? d.Tx : d.Tz) : plan_cols_xz(kPlans[P].n, TP);
+    const int T = DIRECT ? A.gen_direct : P == 0 ? (axis == 1 ? d.Tx : d.Tz) : plan_cols_xz(kPlans[P].n, TP);
     const int Py = d.Py;
     const int ctiles = (Py + T - 1) / T;
     const int outer = lb / ctiles;
@@ -1001,7 +1011,7 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
             else buf[pad(idx)] = make_float2(0.f, 0.f);
         }
         cp_commit();
-        if (conv) {
+        if (conv && !DIRECT) {
             for (int idx = tid; idx < P_; idx += NT) {
                 const int e = idx / T, t = idx - e * T;
                 if (k0 + t < Py) cp8(&hbuf[idx], d.otf + base + e * es + k0 + t);
@@ -1011,8 +1021,15 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
         for (int i = tid; i < (P == 0 ? n : plan_tw_size(P)); i += NT) tw[i] = A.tw[i];
         cp_wait<1>();
         __syncthreads();
-        if (mode == XZ_INV) fft_xz<P, true, TP>(buf, A, tw, T, tid);
-        else fft_xz<P, false, TP>(buf, A, tw, T, tid);
+        auto fft = [&](auto inv) {
+            constexpr bool INV = decltype(inv)::value;
+            if constexpr (DIRECT)
+                fft_lines<INV, true>(buf, A, tw, TileGeom{T, A.n, 1, T, true}, tid, NT,
+                                     (float4*)(((uintptr_t)hbuf + 15) & ~(uintptr_t)15));   // odd n: 8 bytes off
+            else fft_xz<P, INV, TP>(buf, A, tw, T, tid);
+        };
+        if (mode == XZ_INV) fft(std::true_type{});
+        else fft(std::false_type{});
         if (conv) {
             cp_wait<0>();
             __syncthreads();
@@ -1020,13 +1037,13 @@ __global__ void __launch_bounds__(PK_THREADS, xz_min_blocks(P)) k_xz(const VolDe
             for (int idx = tid; idx < P_; idx += NT) {
                 const int t = idx % T;
                 if (k0 + t < Py) {
-                    float2 hv = hbuf[idx];
+                    float2 hv = DIRECT ? __ldg(d.otf + base + (long long)(idx / T) * es + k0 + t) : hbuf[idx];
                     if (cj) hv.y = -hv.y;
                     buf[pad(idx)] = cmul(buf[pad(idx)], hv);
                 }
             }
             __syncthreads();
-            fft_xz<P, true, TP>(buf, A, tw, T, tid);
+            fft(std::true_type{});
         }
         const float sc = mode == XZ_FWD_SCALE ? d.xz_scale : 1.f;
         for (int idx = tid; idx < P_; idx += NT) {
@@ -1044,7 +1061,8 @@ constexpr int kYModes = Y_C2R + 1;
 
 // Entries [0, kNumPlans) hold the 4096-point-tile kernels, [kNumPlans + p] the small-tile kernels
 // of plan p (small_tile_plan(p)); a program step's plan id carries that offset.  The y entries of the plans
-// without small tiles, kNumPlans and kNumPlans + 1, hold the mixed-radix engine's kernels (GEN 1 and 2).
+// without small tiles, kNumPlans .. kNumPlans + 2, hold the kernels of lengths without a plan (GEN 1 .. 3), the
+// x / z entry kNumPlans the one of those with a prime factor above 31.
 struct KernelTable {
     void (*y[2 * kNumPlans][kYModes])(const VolDesc*, const int*, int, int);
     void (*xz[2 * kNumPlans])(const VolDesc*, const int*, int, int, int);
@@ -1067,13 +1085,13 @@ struct RegisterY<P, kYModes> {
     static void fill(KernelTable&) {}
 };
 
-static_assert(!small_tile_plan(0) && !small_tile_plan(1), "the mixed-radix y kernels take these entries");
+static_assert(!small_tile_plan(0) && !small_tile_plan(1) && !small_tile_plan(2), "lengths without a plan take these entries");
 template <int GEN, int MD>
 struct RegisterYGen {
     static void fill(KernelTable& t) {
         auto fn = k_y<0, MD, PK_TILE_POINTS, GEN>;
         t.y[kNumPlans + GEN - 1][MD] = fn;
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, GEN == 3 ? kDirectSmem : 200 * 1024);
         RegisterYGen<GEN, MD + 1>::fill(t);
     }
 };

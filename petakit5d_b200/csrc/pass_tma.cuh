@@ -11,9 +11,8 @@
 // between the forward and the inverse transform).  All tensor maps cover this GPU's own buffers;
 // no load uses cluster multicast.
 //
-// XZ_CONV runs the inverse as the forward stages transposed, last stage first, so that the elements the
-// forward transform left in registers (multiplied by the OTF there) feed the inverse directly whatever
-// the radices; with a pass over shared memory for the multiply, the convolution of plans whose first and last
+// XZ_CONV multiplies by the OTF on the elements that the forward transform's last stage leaves in registers;
+// with a pass over shared memory for the multiply, the convolution of plans whose first and last
 // radix differ was slower than the register-IO kernel.  Measured, before -> after (the launches of 16
 // chunks of 224-416 voxels, and single volumes): z 288 0.493 -> 0.408 ms, z 224 0.368 -> 0.307 ms, z 128 of
 // 512x512x128 0.089 -> 0.074 ms (5460 GB/s).  Lines above 512 come here too, on tiles as wide as shared
@@ -100,7 +99,7 @@ __device__ __forceinline__ void dbfly(float2* v) {
 #pragma unroll
             for (int r = 0; r < R; r++) v[r] = pkgen::swp(v[r]);
         }
-        pkgen::butterfly<R>(v, [&](int q, float2 x) { o[q] = INV ? pkgen::swp(x) : x; });
+        pkgen::bf_odd<R>(v, [&](int q, float2 x) { o[q] = INV ? pkgen::swp(x) : x; });
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = o[r];
     }
@@ -185,83 +184,27 @@ __device__ __forceinline__ void dstage_s2r(const float2* __restrict__ buf, const
     }
 }
 
-// The transform's stages transposed, for the inverse after the OTF multiply: a DFT is its own transpose, so
-// the stages run backwards (butterfly, then the stage's twiddles; read where the stage stores, write
-// where it loads).  The first of them starts from the elements that the forward transform's last stage
-// left in registers, whatever the radices: no pass over shared memory between the transforms.
-// Last stage's transpose from registers: the outputs go where the thread's inputs were.
-template <int R, int NS, int N, int L, bool INV, int OFF, int NTH>
-__device__ __forceinline__ void dstage_t_r2s(float2* __restrict__ buf, const float2* __restrict__ tw, int tid,
-                                             float2 (&v)[(L * (N / R) + NTH - 1) / NTH][R]) {
-    static_assert(NS * R == N, "the last stage of the transform");
-    constexpr int B = L * NS;
-    constexpr int MAXB = (B + NTH - 1) / NTH;
-#pragma unroll
-    for (int i = 0; i < MAXB; i++) {
-        const int b = tid + i * NTH;
-        if (B % NTH == 0 || b < B) {
-            const int l = b % L, j = b / L;
-            dbfly<R, INV>(v[i]);
-            if constexpr (NS > 1) {
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    float2 w = tw[OFF + (r - 1) * NS + j];
-                    if (INV) w.y = -w.y;
-                    v[i][r] = cmul(v[i][r], w);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < R; r++) buf[(j + r * NS) * L + l] = v[i][r];
-        }
-    }
-    compute_bar<NTH>();
-}
-
-template <int R, int NS, int N, int L, bool INV, int OFF, int NTH>
-__device__ __forceinline__ void dstage_t(float2* __restrict__ buf, const float2* __restrict__ tw, int tid) {
+// first stage from registers: v[i][r] is element j + r (N / R) of column l; butterfly, store
+template <int R, int N, int L, bool INV, int NTH>
+__device__ __forceinline__ void dstage_r2s(float2* __restrict__ buf, int tid,
+                                           float2 (&v)[(L * (N / R) + NTH - 1) / NTH][R]) {
+    static_assert(!direct_radix(R), "first stage needs a register butterfly");
     constexpr int M = N / R;
     constexpr int B = L * M;
-    constexpr int MAXB = (B + NTH - 1) / NTH;
-    float2 v[MAXB][R];
+    constexpr int NT = NTH;
+    constexpr int MAXB = (B + NT - 1) / NT;
 #pragma unroll
     for (int i = 0; i < MAXB; i++) {
-        const int b = tid + i * NTH;
-        const int bb = (B % NTH == 0 || b < B) ? b : 0;   // as in dstage: an unconditional load
-        const int l = bb % L, j = bb / L, k = j % NS;
-        const int a0 = ((j - k) * R + k) * L + l;
+        const int b = tid + i * NT;
+        if (B % NT == 0 || b < B) {
+            const int l = b % L, j = b / L;
+            bfly<R, INV>(v[i]);
+            const int a0 = j * R * L + l;
 #pragma unroll
-        for (int r = 0; r < R; r++) v[i][r] = buf[a0 + r * NS * L];
-    }
-    compute_bar<NTH>();
-#pragma unroll
-    for (int i = 0; i < MAXB; i++) {
-        const int b = tid + i * NTH;
-        if (B % NTH == 0 || b < B) {
-            const int l = b % L, j = b / L, k = j % NS;
-            dbfly<R, INV>(v[i]);
-            if constexpr (NS > 1) {
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    float2 w = tw[OFF + (r - 1) * NS + k];
-                    if (INV) w.y = -w.y;
-                    v[i][r] = cmul(v[i][r], w);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < R; r++) buf[(j + r * M) * L + l] = v[i][r];
+            for (int r = 0; r < R; r++) buf[a0 + r * L] = v[i][r];
         }
     }
     compute_bar<NTH>();
-}
-
-// stages S, S - 1, .., 0 of plan P transposed
-template <int P, int S, int L, bool INV, int NTH>
-__device__ __forceinline__ void run_dense_t(float2* buf, const float2* tw, int tid) {
-    if constexpr (S >= 0) {
-        constexpr int R = kPlans[P].rad[S];
-        dstage_t<R, plan_ns_before(P, S), kPlans[P].n, L, INV, stage_tw_off(P, S), NTH>(buf, tw, tid);
-        run_dense_t<P, S - 1, L, INV, NTH>(buf, tw, tid);
-    }
 }
 
 template <int P, int S, int S1, int NS, int L, bool INV, int NTH>
@@ -416,7 +359,8 @@ __global__ void __launch_bounds__(NTH + 32, xzt_min_blocks(P, TC, NBUF, MODE == 
         } else {
             const bool cj = descs[vol].conj != 0;
             // the last forward stage leaves each thread R elements j + r MS of a column in registers: OTF
-            // multiply there, then the inverse's stages from the last backwards
+            // multiply there; the inverse's first stage takes them from there when it has the same radix, else
+            // through the tile (each thread stores where it read, so no barrier comes before)
             constexpr int R = kPlans[P].rad[NST - 1], MS = N / R, MAXB = (T * MS + NT - 1) / NT;
             constexpr int OFF = stage_tw_off(P, NST - 1);
             float2 v[MAXB][R];
@@ -442,8 +386,22 @@ __global__ void __launch_bounds__(NTH + 32, xzt_min_blocks(P, TC, NBUF, MODE == 
             }
             compute_bar<NTH>();   // every OTF read done: the producer may refill it
             if (tid == 0) mbar_arrive_cta(otf_empty);
-            dstage_t_r2s<R, MS, N, T, true, OFF, NTH>(cur, tw, tid, v);
-            run_dense_t<P, NST - 2, T, true, NTH>(cur, tw, tid);
+            if constexpr (pkpass::same_end_radix(P)) {
+                dstage_r2s<R, N, T, true, NTH>(cur, tid, v);
+                run_dense<P, 1, NST, R, T, true, NTH>(cur, tw, tid);
+            } else {
+#pragma unroll
+                for (int i = 0; i < MAXB; i++) {
+                    const int b = tid + i * NT;
+                    if (MAXB * NT == T * MS || b < T * MS) {
+                        const int l = b % T, j = b / T;
+#pragma unroll
+                        for (int r = 0; r < R; r++) cur[(j + r * MS) * T + l] = v[i][r];
+                    }
+                }
+                compute_bar<NTH>();
+                run_dense<P, 0, NST, 1, T, true, NTH>(cur, tw, tid);
+            }
         }
         // the tile leaves by TMA: each thread's writes are ordered before the async proxy's reads,
         // then the buffer is handed to the producer

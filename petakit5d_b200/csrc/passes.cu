@@ -44,6 +44,7 @@ void pk_fill_kernels_h(pkpass::KernelTable& t);
 void pk_fill_kernels_i(pkpass::KernelTable& t);
 void pk_fill_kernels_g1(pkpass::KernelTable& t);
 void pk_fill_kernels_g2(pkpass::KernelTable& t);
+void pk_fill_kernels_g3(pkpass::KernelTable& t);
 void pk_fill_tma_0(pkpass::TmaTable& t);
 void pk_fill_tma_1(pkpass::TmaTable& t);
 void pk_fill_tma_2(pkpass::TmaTable& t);
@@ -79,11 +80,23 @@ void pk_fill_all_kernels(pkpass::KernelTable& t) {
     pk_fill_kernels_i(t);
     pk_fill_kernels_g1(t);
     pk_fill_kernels_g2(t);
+    pk_fill_kernels_g3(t);
+}
+
+// Dynamic shared memory of an x / z tile of `lines` columns of a length with a prime factor above 31: roots, tile,
+// doubled inputs of the sums.
+static size_t direct_xz_smem(int n, int lines) {
+    return sizeof(float2) * (tw_slots(n) + padded_size2(lines * n)) + 16 + sizeof(float4) * (size_t)lines * n;
 }
 
 static size_t step_smem(int kind, int mode, const VolDesc& v) {
+    if (kind == PK_STEP_Y && v.ay.gen_direct)
+        return sizeof(float2) * (tw_slots(v.M) + (v.odd ? 0 : v.M + 1) + padded_size(v.Ly * v.M) + v.Ly +
+                                 (size_t)pkpass::y_aux_arrays(mode) * v.Ly * v.M) + 16 + sizeof(float4) * (size_t)v.Ly * v.M;
+    if (kind == PK_STEP_X && v.ax.gen_direct) return direct_xz_smem(v.ax.n, v.ax.gen_direct);
+    if (kind == PK_STEP_Z && v.az.gen_direct) return direct_xz_smem(v.az.n, v.az.gen_direct);
     if (kind == PK_STEP_Y && v.ay.gen) {
-        const int lines = v.odd ? (v.Ly + 1) / 2 : v.Ly, len = v.odd ? std::max(v.ay.genL, v.M + 1) : v.ay.genL;
+        const int lines = v.odd ? (v.Ly + 1) / 2 : v.Ly, len = v.odd ? v.M + 1 : v.M;
         return sizeof(float2) * ((v.odd ? 0 : v.M + 1) + 2 * (size_t)pkpass::gen_y_slots(lines, len) + v.Ly +
                                  (size_t)pkpass::y_aux_arrays(mode) * (v.odd ? pkpass::gen_y_slots(v.Ly, v.M) / 2 : v.Ly * v.M));
     }
@@ -912,15 +925,13 @@ constexpr GenRadix kGenRadices[] = {{16, 150}, {15, 190}, {13, 190}, {12, 112}, 
                                     {8, 56},   {7, 60},   {6, 40},   {5, 34},   {4, 16},   {3, 14},   {2, 4},
                                     {17, 310}, {19, 380}, {23, 550}, {29, 860}, {31, 980}};
 
-// Columns of an x / z tile (n points a line, L in the stages): the widest power of two (16: whole 128-byte
-// lines; 32 on short lines, for the work of a tile) whose three buffers let three CTAs share an SM, at least
-// 4 (one 32-byte sector of the spectrum) where that fits one CTA, else 2; 0 where nothing fits.  Timed on the
-// 270-long z pass of a 512 x 1140 x 270 volume: 16 columns at two CTAs an SM 1.07 ms, 8 at three 0.98 ms,
-// 4 at three 1.53 ms.
-int gen_tile(int n, int L, GenAxis* g) {
-    for (int T = L <= 64 ? 32 : 16; T >= 2; T /= 2) {
+// Columns of an x / z tile of n-point lines: the widest power of two (16: whole 128-byte lines; 32 on short
+// lines, for the work of a tile) whose three buffers let three CTAs share an SM, at least 4 (one 32-byte
+// sector of the spectrum) where that fits one CTA, else 2; 0 where nothing fits.  Timed on the 270-long z pass
+// of a 512 x 1140 x 270 volume: 16 columns at two CTAs an SM 1.07 ms, 8 at three 0.98 ms, 4 at three 1.53 ms.
+int gen_tile(int n, GenAxis* g) {
+    for (int T = n <= 64 ? 32 : 16; T >= 2; T /= 2) {
         const int gran = T >= 16 ? 1 : 16 / T;   // box rows keep each box on a 128-byte boundary
-        g->L = L;
         g->T = T;
         for (g->nbox = (n + 255) / 256;; g->nbox++) {
             g->rows = ((n + g->nbox - 1) / g->nbox + gran - 1) / gran * gran;
@@ -981,99 +992,73 @@ double gen_search(int n, int pts, std::vector<int>& rad) {
     return best;
 }
 
-// Discrete Fourier transform in double, by the smallest prime factor at each level.
-void host_dft(const double2* x, int n, int stride, double2* out) {
-    if (n == 1) {
-        out[0] = x[0];
-        return;
-    }
-    int p = 2;
-    while (n % p) p++;
-    const int m = n / p;
-    std::vector<double2> sub(n);
-    for (int r = 0; r < p; r++) host_dft(x + (size_t)r * stride, m, stride * p, sub.data() + (size_t)r * m);
-    for (int k = 0; k < n; k++) {
-        double re = 0, im = 0;
-        for (int r = 0; r < p; r++) {
-            const double a = -2.0 * M_PI * (double)((long long)r * k % n) / n, c = std::cos(a), s = std::sin(a);
-            const double2 v = sub[(size_t)r * m + k % m];
-            re += v.x * c - v.y * s;
-            im += v.x * s + v.y * c;
-        }
-        out[k] = make_double2(re, im);
-    }
-}
-
 }  // namespace
 
-// Plan (stages, tile shape) of length n; false where no tile fits shared memory.  `tables` receives
-// the stage twiddles, then for a chirp transform the chirp and the filter's transform.
+// Largest length whose prime-factor stages get root matrices (33 MB at 2039); above it the plain engine.
+constexpr int kDirectMax = 2048;
+
+// Plan (stages, tile shape) of length n and its tables: the stages' twiddles, or with a prime factor above 31
+// the root matrices of the prime-factor stages.
 static bool gen_plan(int n, GenAxis* g, std::vector<float2>& tables) {
     *g = GenAxis();
     g->n = n;
     std::vector<int> rad;
     if (n < 2) return false;
-    auto points = [&](int L) { return L * std::max(1, gen_tile(n, L, g)); };
-    int len = n;
-    if (gen_search(n, points(n), rad) > 1e29) {
-        // the cheapest smooth length of 2 n - 1 .. 4 n
-        double best = 1e30;
-        for (int L = 2 * n - 1; L < 4 * n; L++) {
-            int r = L;
-            for (int p : {2, 3, 5, 7}) while (r % p == 0) r /= p;
-            if (r != 1 || 14.0 * L > best) continue;
-            std::vector<int> q;
-            const double c = gen_search(L, points(L), q) * L;
-            if (c < best) {
-                best = c;
-                rad = q;
-                len = L;
-            }
-        }
-        if (best > 1e29) return false;
-        g->blue = 1;
+    tables.clear();
+    if (gen_search(n, n * std::max(1, gen_tile(n, g)), rad) > 1e29) {
+        AxisPlan p;
+        if (n > kDirectMax || !pk_make_axis_plan(n, &p)) return false;
+        rad.assign(p.rad, p.rad + p.nst);
+        g->direct = 1;
+        g->T = g->rows = g->nbox = 0;
     }
-    gen_tile(n, len, g);
-    g->L = len;
     for (int r : rad) g->big |= r > 16;
-    const int L = g->L;
+    std::vector<float2> root(g->direct ? n : 0);
+    if (g->direct) pk_root_table(n, root.data());
     auto magic = [](int d) { return d > 1 ? 0xFFFFFFFFu / (unsigned)d + 1u : 0u; };
     g->nst = (int)rad.size();
     int ns = 1;
-    tables.clear();
     for (int s = 0; s < g->nst; s++) {
-        const int R = rad[s];
+        const int R = rad[s], tstep = n / (ns * R);
         g->rad[s] = R;
         g->ns[s] = ns;
-        g->m[s] = L / R;
+        g->m[s] = n / R;
         g->mg_ns[s] = magic(ns);
-        g->mg_m[s] = magic(L / R);
-        g->off[s] = (int)tables.size();
-        if (ns > 1)
+        g->mg_m[s] = magic(n / R);
+        if (!g->direct) {
+            g->off[s] = (int)tables.size();
+            if (ns > 1)
+                for (int k = 0; k < ns; k++)
+                    for (int r = 1; r <= pkgen::tw_row(R); r++)
+                        tables.push_back(root_of((int)((long long)r * k * tstep % n), n));
+        } else if (R > 5 && R != 8 && R != 16) {
+            const int half = direct_half(R);   // floats; a row is 2 half floats, half float2
+            g->off[s] = (int)tables.size() * 2;
+            tables.resize(tables.size() + (size_t)ns * R * half, make_float2(0.f, 0.f));
+            float* m = (float*)tables.data() + g->off[s];
             for (int k = 0; k < ns; k++)
-                for (int r = 1; r <= pkgen::tw_row(R); r++)
-                    tables.push_back(root_of((int)((long long)r * k * (L / (ns * R)) % L), L));
+                for (int q = 0; q < R; q++, m += 2 * half)
+                    for (int t = 0; t < R; t++) {
+                        const float2 w = root[(size_t)((long long)q * (k + (long long)ns * t) * tstep % n)];
+                        m[t] = w.x;
+                        m[half + t] = w.y;
+                    }
+        }
         ns *= R;
     }
-    if (g->blue) {
-        auto chirp = [&](long long e) {   // exp(-i pi e^2 / n)
-            const double a = -M_PI * (double)(e * e % (2LL * n)) / n;
-            return make_double2(std::cos(a), std::sin(a));
-        };
-        for (int e = 0; e < n; e++) {
-            const double2 w = chirp(e);
-            tables.push_back(make_float2((float)w.x, (float)w.y));
-        }
-        std::vector<double2> b(L, make_double2(0, 0)), bk(L);
-        for (int e = 0; e < n; e++) {
-            const double2 w = chirp(e);
-            b[e] = make_double2(w.x, -w.y);
-            if (e) b[L - e] = b[e];
-        }
-        host_dft(b.data(), L, 1, bk.data());
-        for (int k = 0; k < L; k++) tables.push_back(make_float2((float)(bk[k].x / L), (float)(bk[k].y / L)));
-    }
     return true;
+}
+
+// Lines (32 to 4) per tile of a length with a prime factor above 31, as many as their shared memory smem(lines)
+// allows; the register radices of the in-place engine take 4096 points at most.  0: none.
+template <class F>
+static int direct_lines(const GenAxis& g, F&& smem) {
+    bool small = false;
+    for (int s = 0; s < g.nst; s++) small |= g.rad[s] <= 5 || g.rad[s] == 8 || g.rad[s] == 16;
+    for (size_t lim : {(size_t)112 * 1024, (size_t)pkpass::kDirectSmem})   // two CTAs an SM, else one
+        for (int c : {32, 16, 8, 4})
+            if ((!small || c * g.n <= PK_TILE_POINTS) && smem(c) <= lim) return c;
+    return 0;
 }
 
 static pk_status pk_get_gen(pk_ctx* ctx, int n, GenAxis* host, const GenAxis** dev) {
@@ -1086,10 +1071,8 @@ static pk_status pk_get_gen(pk_ctx* ctx, int n, GenAxis* host, const GenAxis** d
             const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
             PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
             const float2* t = (const float2*)((const char*)d + head);
-            size_t stage_tw = tables.size() - (g.blue ? (size_t)g.n + g.L : 0);
             g.tw = t;
-            g.chirp = g.blue ? t + stage_tw : nullptr;
-            g.bk = g.blue ? t + stage_tw + g.n : nullptr;
+            g.mat = (const float*)t;
             cudaError_t e = cudaMemcpy(d, &g, sizeof(g), cudaMemcpyHostToDevice);
             if (e == cudaSuccess && !tables.empty())
                 e = cudaMemcpy((void*)t, tables.data(), sizeof(float2) * tables.size(), cudaMemcpyHostToDevice);
@@ -1120,10 +1103,11 @@ pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a) {
         const pk_status st = pk_get_gen(ctx, n, &g, &a->gen);
         if (st != PK_OK) return st;
         if (a->gen) {
-            a->genL = g.L;
             a->genT = g.T;
             a->gen_rows = g.rows;
             a->gen_big = g.big;
+            if (g.direct)
+                a->gen_direct = direct_lines(g, [&](int c) { return direct_xz_smem(n, c); });
             if (g.T) {
                 a->gen_land = pkpass::gen_land(g);
                 a->gen_work = pkpass::gen_work(g);
@@ -1153,19 +1137,32 @@ pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
     if ((st = pk_fill_axis(ctx, nx, nx, &d->ax)) != PK_OK) return st;
     if ((st = pk_fill_axis(ctx, nz, nz, &d->az)) != PK_OK) return st;
     if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
-    if (d->ay.gen) {   // odd rows run in pairs
-        d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->ay.genL);
+    if (d->ay.gen_direct) {
+        GenAxis g;
+        const GenAxis* dev;
+        if ((st = pk_get_gen(ctx, d->M, &g, &dev)) != PK_OK) return st;
+        d->ay.gen_direct = direct_lines(g, [&](int c) {
+            VolDesc t = *d;
+            t.Ly = t.ay.gen_direct = c;
+            return step_smem(PK_STEP_Y, Y_RLUPD, t);
+        });
+        if (!d->ay.gen_direct) d->ay.gen = nullptr;   // the plain in-place engine
+    }
+    if (d->ay.gen_direct) {
+        d->Ly = d->ay.gen_direct;
+    } else if (d->ay.gen) {   // odd rows run in pairs
+        d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->M);
     } else {
         d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
     }
     // a line whose engine buffers do not fit shared memory keeps the in-place engine
-    if (d->ay.gen && step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) {
+    if (d->ay.gen && !d->ay.gen_direct && step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) {
         d->ay.gen = nullptr;
         d->Ly = std::max(1, P / d->M);
     }
-    if ((long long)d->Ly > d->nrows && d->ay.plan == 0) d->Ly = (int)d->nrows;
-    d->Tx = d->ax.plan ? plan_cols_xz(nx) : std::max(1, std::min(P / nx, d->Py));
-    d->Tz = d->az.plan ? plan_cols_xz(nz) : std::max(1, std::min(P / nz, d->Py));
+    if ((long long)d->Ly > d->nrows && d->ay.plan == 0 && !d->ay.gen_direct) d->Ly = (int)d->nrows;
+    d->Tx = d->ax.gen_direct ? d->ax.gen_direct : d->ax.plan ? plan_cols_xz(nx) : std::max(1, std::min(P / nx, d->Py));
+    d->Tz = d->az.gen_direct ? d->az.gen_direct : d->az.plan ? plan_cols_xz(nz) : std::max(1, std::min(P / nz, d->Py));
     auto set_blocks = [&]() {
         const int ct_x = (d->Py + d->Tx - 1) / d->Tx, ct_z = (d->Py + d->Tz - 1) / d->Tz;
         d->blocksY = (int)((d->nrows + d->Ly - 1) / d->Ly);
@@ -1197,7 +1194,9 @@ size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; 
 // back to back without host synchronisation and can be captured into a CUDA graph.
 // Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels.
 static int step_plan(int kind, const VolDesc& v) {
-    if (kind == PK_STEP_Y && v.ay.gen) return kNumPlans + v.ay.gen_big;   // the mixed-radix engine's y kernels
+    // lengths without a plan: the mixed-radix engine's y kernels, the kernels of a prime factor above 31
+    if (kind == PK_STEP_Y && v.ay.gen) return kNumPlans + (v.ay.gen_direct ? 2 : v.ay.gen_big);
+    if ((kind == PK_STEP_X && v.ax.gen_direct) || (kind == PK_STEP_Z && v.az.gen_direct)) return kNumPlans;
     const int p = kind == PK_STEP_Y ? v.ay.plan : kind == PK_STEP_X ? v.ax.plan : kind == PK_STEP_Z ? v.az.plan : 0;
     return (v.tiles_small && kind != PK_STEP_LAMBDA) ? kNumPlans + p : p;
 }

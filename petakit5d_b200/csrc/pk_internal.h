@@ -39,17 +39,16 @@ struct PkRange {
 #endif
 
 // ------------------------------------------------------------------ device-visible structs
-// Run-time plan of a transform length without a compile-time plan (gen_engine.cuh): its stages over
-// L points (L = n, or the length of the chirp convolution when n has a prime factor above 31).
-#define PK_GEN_MAXST 8
+// Run-time plan of a transform length without a compile-time plan (gen_engine.cuh).
+#define PK_GEN_MAXST 16
 struct GenAxis {
-    int n, L, blue, nst, big;   // blue: chirp transform; big: has a radix above 16
+    int n, nst;
+    int big, direct;       // a radix above 16; a prime factor above 31 (stage_direct)
     int rad[PK_GEN_MAXST], ns[PK_GEN_MAXST], m[PK_GEN_MAXST];    // radix, stride, butterflies per line
     unsigned mg_ns[PK_GEN_MAXST], mg_m[PK_GEN_MAXST];            // multiply-high reciprocals of ns and m
-    int off[PK_GEN_MAXST];                                       // stage's twiddles W^{rk} at tw[off + k tw_row(R) + r - 1]
+    int off[PK_GEN_MAXST]; // stage's twiddles W^{rk} at tw[off + k tw_row(R) + r - 1]; direct: its roots at mat[off]
+    const float* mat;      // direct: root matrices of the prime-factor stages
     const float2* tw;
-    const float2* chirp;   // exp(-i pi e^2 / n), e < n
-    const float2* bk;      // transform of the conjugate chirp over L points, / L
     int T, lt;             // x / z pass: columns per tile (2^lt)
     int rows, nbox;        // x / z pass: the tile arrives as nbox boxes of `rows` elements of the line
 };
@@ -63,8 +62,9 @@ struct AxisDev {
     int twStride;     // 1
     int plan;         // compile-time plan id (0 = runtime engine)
     const GenAxis* gen;   // plan 0: the length's run-time plan (device), or null: the in-place engine
-    int genL, genT, gen_rows;   // its L, T and rows, and an x / z tile's buffers (pass_gen.cuh)
+    int genT, gen_rows;         // its T and rows, and an x / z tile's buffers (pass_gen.cuh)
     int gen_land, gen_work, gen_big;
+    int gen_direct;             // prime factor above 31: lines per tile (16, 8 or 4; 0: not direct)
 };
 
 // Pass modes of the y kernel.

@@ -1,5 +1,5 @@
-"""Transform lengths without a compile-time plan (gen_engine.cuh, pass_gen.cuh): every radix of the
-mixed-radix engine, chirp lengths, and the lengths that fall back to the in-place engine."""
+"""Transform lengths without a compile-time plan (gen_engine.cuh, pass_gen.cuh): every radix of the mixed-radix
+engine, lengths with a larger prime factor (stage_direct), and those that keep the plain in-place engine."""
 import math
 
 import numpy as np
@@ -13,15 +13,16 @@ from petakit5d_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
-# x / z lengths: primes of the radix set, composites of one and several stages, chirp lengths with
-# 16- to 2-column tiles, one and several TMA boxes a line, and 4093 (no tile: the in-place engine)
+# x / z lengths: primes of the radix set, composites of one and several stages, larger primes alone and beside
+# register radices on tiles of 32 to 4 columns, one and several TMA boxes a line, and lengths above 2048 with
+# a large prime (the plain in-place engine)
 LENGTHS = [3, 6, 7, 11, 13, 15, 17, 19, 22, 23, 27, 29, 31, 33, 37, 62, 97, 122, 130, 251, 257, 270, 299, 467, 520, 521,
            613, 930, 1140, 1151, 1558, 1721, 2047, 2310, 3001, 4093]
 
 
 def _tol(dims):
     # a transform's rounding grows with its stages: 2^-24 for each of about 4 operations on a value
-    # per stage, log2(4 n) stages at most (a chirp length runs two transforms of up to 4 n points)
+    # per stage, log2(4 n) stages at most, twice (plain sums over a prime factor round p times each)
     return 2.0 ** -24 * 4 * sum(math.log2(4 * n) + (math.log2(4 * n) if n > 1 else 0) for n in dims)
 
 
