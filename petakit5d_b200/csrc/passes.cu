@@ -997,20 +997,28 @@ double gen_search(int n, int pts, std::vector<int>& rad) {
 // Largest length whose prime-factor stages get root matrices (33 MB at 2039); above it the plain engine.
 constexpr int kDirectMax = 2048;
 
-// Plan (stages, tile shape) of length n and its tables: the stages' twiddles, or with a prime factor above 31
-// the root matrices of the prime-factor stages.
-static bool gen_plan(int n, GenAxis* g, std::vector<float2>& tables) {
+// A length of the mixed-radix engine: no prime factor above 31.
+static bool gen_smooth(int n) {
+    for (int p : {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31})
+        while (n % p == 0) n /= p;
+    return n == 1;
+}
+
+// Plan (stages, tile shape) of length n and its tables: the stages' twiddles, or for `direct` the in-place
+// engine's stages and the root matrices of the prime-factor ones.
+static bool gen_plan(int n, bool direct, GenAxis* g, std::vector<float2>& tables) {
     *g = GenAxis();
     g->n = n;
     std::vector<int> rad;
     if (n < 2) return false;
     tables.clear();
-    if (gen_search(n, n * std::max(1, gen_tile(n, g)), rad) > 1e29) {
+    if (direct) {
         AxisPlan p;
         if (n > kDirectMax || !pk_make_axis_plan(n, &p)) return false;
         rad.assign(p.rad, p.rad + p.nst);
         g->direct = 1;
-        g->T = g->rows = g->nbox = 0;
+    } else if (!gen_smooth(n) || gen_search(n, n * std::max(1, gen_tile(n, g)), rad) > 1e29) {
+        return false;
     }
     for (int r : rad) g->big |= r > 16;
     std::vector<float2> root(g->direct ? n : 0);
@@ -1049,25 +1057,27 @@ static bool gen_plan(int n, GenAxis* g, std::vector<float2>& tables) {
     return true;
 }
 
-// Lines (32 to 4) per tile of a length with a prime factor above 31, as many as their shared memory smem(lines)
-// allows; the register radices of the in-place engine take 4096 points at most.  0: none.
+// Lines (32 to 4) per tile of a direct length, as many as their shared memory smem(lines)
+// allows; the register radices of the in-place engine take 4096 points at most.  0: none, the plain engine (4
+// lines of 999 = 27 * 37 were 5% slower than it).
 template <class F>
 static int direct_lines(const GenAxis& g, F&& smem) {
     bool small = false;
     for (int s = 0; s < g.nst; s++) small |= g.rad[s] <= 5 || g.rad[s] == 8 || g.rad[s] == 16;
     for (size_t lim : {(size_t)112 * 1024, (size_t)pkpass::kDirectSmem})   // two CTAs an SM, else one
         for (int c : {32, 16, 8, 4})
-            if ((!small || c * g.n <= PK_TILE_POINTS) && smem(c) <= lim) return c;
+            if ((!small || (c >= 8 && c * g.n <= PK_TILE_POINTS)) && smem(c) <= lim) return c;
     return 0;
 }
 
-static pk_status pk_get_gen(pk_ctx* ctx, int n, GenAxis* host, const GenAxis** dev) {
-    auto it = ctx->gen.find(n);
+static pk_status pk_get_gen(pk_ctx* ctx, int n, bool direct, GenAxis* host, const GenAxis** dev) {
+    const int key = direct ? -n : n;
+    auto it = ctx->gen.find(key);
     if (it == ctx->gen.end()) {
         GenAxis g;
         std::vector<float2> tables;
         GenAxis* d = nullptr;
-        if (gen_plan(n, &g, tables)) {
+        if (gen_plan(n, direct, &g, tables)) {
             const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
             PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
             const float2* t = (const float2*)((const char*)d + head);
@@ -1081,14 +1091,14 @@ static pk_status pk_get_gen(pk_ctx* ctx, int n, GenAxis* host, const GenAxis** d
                 PK_CUDA(e);
             }
         }
-        it = ctx->gen.emplace(n, std::make_pair(g, d)).first;
+        it = ctx->gen.emplace(key, std::make_pair(g, d)).first;
     }
     *host = it->second.first;
     *dev = it->second.second;
     return PK_OK;
 }
 
-pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a) {
+pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a, bool direct) {
     AxisPlan p;
     if (!pk_make_axis_plan(n, &p)) return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
     memset(a, 0, sizeof(*a));
@@ -1098,9 +1108,9 @@ pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a) {
     a->twN = twN;
     a->twStride = twN / n;
     a->plan = pk_find_plan(n);
-    if (a->plan == 0) {
+    if (a->plan == 0 && !(direct && gen_smooth(n))) {   // small factors sum as fast on the plain in-place engine
         GenAxis g;
-        const pk_status st = pk_get_gen(ctx, n, &g, &a->gen);
+        const pk_status st = pk_get_gen(ctx, n, direct, &g, &a->gen);
         if (st != PK_OK) return st;
         if (a->gen) {
             a->genT = g.T;
@@ -1133,14 +1143,20 @@ pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
         return pk_fail(PK_ERR_UNSUPPORTED, "a transform axis is longer than " + std::to_string(P) +
                                                " (" + std::to_string(2 * P) + " along y)");
     pk_status st;
-    if ((st = pk_fill_axis(ctx, d->M, d->M, &d->ay)) != PK_OK) return st;
-    if ((st = pk_fill_axis(ctx, nx, nx, &d->ax)) != PK_OK) return st;
-    if ((st = pk_fill_axis(ctx, nz, nz, &d->az)) != PK_OK) return st;
+    // a volume with a prime factor above 31 on any axis keeps the in-place engine's sums on all that have no plan:
+    // the sums' roundings shift every voxel alike and partly cancel between the axes, so one axis made more
+    // exact can leave the result less so (117 x 999 x 336 OMW x2: 0.9e-6 of its norm off, 1.4e-6 with 117 and
+    // 336 on the mixed-radix engine and 999 as it was)
+    bool direct = false;
+    for (int n : {d->M, nx, nz}) direct = direct || (pk_find_plan(n) == 0 && !gen_smooth(n));
+    if ((st = pk_fill_axis(ctx, d->M, d->M, &d->ay, direct)) != PK_OK) return st;
+    if ((st = pk_fill_axis(ctx, nx, nx, &d->ax, direct)) != PK_OK) return st;
+    if ((st = pk_fill_axis(ctx, nz, nz, &d->az, direct)) != PK_OK) return st;
     if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
     if (d->ay.gen_direct) {
         GenAxis g;
         const GenAxis* dev;
-        if ((st = pk_get_gen(ctx, d->M, &g, &dev)) != PK_OK) return st;
+        if ((st = pk_get_gen(ctx, d->M, true, &g, &dev)) != PK_OK) return st;
         d->ay.gen_direct = direct_lines(g, [&](int c) {
             VolDesc t = *d;
             t.Ly = t.ay.gen_direct = c;

@@ -251,7 +251,7 @@ pk_status pk_fail(pk_status st, const std::string& msg);
 void pk_root_table(int n, float2* out);
 int pk_axis_table(int n, float2* out);   // writes at most n + PK_TW_EXTRA entries, returns the count
 pk_status pk_get_twiddles(pk_ctx* ctx, int twN, const float2** out);
-pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a);
+pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a, bool direct = false);
 pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d);
 size_t pk_spec_elems(const VolDesc& d);   // complex elements of the half spectrum
 
