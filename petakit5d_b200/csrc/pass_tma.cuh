@@ -411,19 +411,21 @@ __global__ void __launch_bounds__(NTH + 32, xzt_min_blocks(P, TC, NBUF, MODE == 
     }
 }
 
-// The TMA kernels by plan, pass and variant: [p][0] x forward, [p][1] x inverse, [p][2] z convolution;
+// The TMA kernels by plan, pass and variant: [p][0] x forward, [p][1] x inverse, [p][2] z convolution,
+// [p][3] x convolution (a volume of one plane);
 // variant 0 is the plan's 4096-point tile with two buffers, variants 1 and 2 (where built) are the
 // alternatives the autotuner times against it.  With each one's dynamic shared memory, resident CTAs
 // per SM (the persistent grid is that times the SMs) and tile width.
-enum { TMA_X_FWD = 0, TMA_X_INV = 1, TMA_Z_CONV = 2 };
+enum { TMA_X_FWD = 0, TMA_X_INV = 1, TMA_Z_CONV = 2, TMA_X_CONV = 3 };
+constexpr int kTmaPasses = 4;
 constexpr int kTmaVariants = 3;
 struct TmaTable {
-    void (*k[kNumPlans][3][kTmaVariants])(const VolDesc*, const XZMaps*, const int*, int, int*);
-    size_t smem[kNumPlans][3][kTmaVariants];
-    int per_sm[kNumPlans][3][kTmaVariants];
-    int cols[kNumPlans][3][kTmaVariants];    // columns per tile (the tile prefix and the TMA box follow it)
-    int nbuf[kNumPlans][3][kTmaVariants];
-    int threads[kNumPlans][3][kTmaVariants];   // compute threads + the producer warp
+    void (*k[kNumPlans][kTmaPasses][kTmaVariants])(const VolDesc*, const XZMaps*, const int*, int, int*);
+    size_t smem[kNumPlans][kTmaPasses][kTmaVariants];
+    int per_sm[kNumPlans][kTmaPasses][kTmaVariants];
+    int cols[kNumPlans][kTmaPasses][kTmaVariants];    // columns per tile (the tile prefix and the TMA box follow it)
+    int nbuf[kNumPlans][kTmaPasses][kTmaVariants];
+    int threads[kNumPlans][kTmaPasses][kTmaVariants];   // compute threads + the producer warp
 };
 
 template <int P, int IDX, int VAR, int AXIS, int MODE, int TC = 0, int NBUF = 2, int NTH = PK_THREADS>
@@ -506,6 +508,14 @@ struct RegisterTma {
                 register_tma_x<P, 1, 4, 3, 512>(t);
                 register_tma_one<P, TMA_Z_CONV, 0, 2, XZ_CONV, 4, 2, 512>(t);
             }
+        }
+        // one-plane volumes: x forward, OTF and x inverse on the tile (the z convolution's shapes)
+        if constexpr (tma_plan(P)) {
+            constexpr int N = kPlans[P].n;
+            constexpr int NB = (N > 1152 && N <= 1280) ? 1 : 2, NT = N > 768 ? 512 : PK_THREADS;
+            register_tma_one<P, TMA_X_CONV, 0, 1, XZ_CONV, 0, NB, NT>(t);
+            if constexpr (N >= 512 && N <= 768)
+                register_tma_one<P, TMA_X_CONV, 1, 1, XZ_CONV, 16, (N <= 576 ? 2 : 1), 512>(t);
         }
         RegisterTma<P + 1, HI>::fill(t);
     }

@@ -259,6 +259,7 @@ int tma_index(const PkStep& s) {
     if (s.kind == PK_STEP_X && s.mode == XZ_FWD) idx = pkpass::TMA_X_FWD;
     else if (s.kind == PK_STEP_X && s.mode == XZ_INV) idx = pkpass::TMA_X_INV;
     else if (s.kind == PK_STEP_Z && s.mode == XZ_CONV) idx = pkpass::TMA_Z_CONV;
+    else if (s.kind == PK_STEP_X && s.mode == XZ_CONV) idx = pkpass::TMA_X_CONV;
     if (idx < 0 || !t->k[s.plan][idx][0]) return -1;
     return idx;
 }

@@ -43,7 +43,7 @@ struct PkRange {
 #define PK_GEN_MAXST 16
 struct GenAxis {
     int n, nst;
-    int big, direct;       // a radix above 16; a prime factor above 31 (stage_direct)
+    int big, direct;       // a radix above 16; the in-place engine's stages (stage_direct)
     int rad[PK_GEN_MAXST], ns[PK_GEN_MAXST], m[PK_GEN_MAXST];    // radix, stride, butterflies per line
     unsigned mg_ns[PK_GEN_MAXST], mg_m[PK_GEN_MAXST];            // multiply-high reciprocals of ns and m
     int off[PK_GEN_MAXST]; // stage's twiddles W^{rk} at tw[off + k tw_row(R) + r - 1]; direct: its roots at mat[off]
@@ -180,7 +180,7 @@ struct pk_ctx {
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::map<int, TwTable> tw;                                   // twN -> table
-    std::map<int, std::pair<GenAxis, GenAxis*>> gen;             // run-time plans by length: host copy, device copy
+    std::map<int, std::pair<GenAxis, GenAxis*>> gen;             // run-time plans by length (negative: direct): host copy, device copy
     // OTF cache: key = (psf content hash, ny, nx, nz)
     std::map<std::tuple<uint64_t, int, int, int>, OtfEntry> otf;
     std::vector<std::pair<void*, size_t>> scratch;               // reusable device buffers by slot
