@@ -348,6 +348,18 @@ constexpr bool same_end_radix(int p) {
     return p > 0 && kPlans[p].nst >= 2 && kPlans[p].rad[0] == kPlans[p].rad[kPlans[p].nst - 1];
 }
 
+// y passes whose per-voxel phase runs on the registers of the inverse transform's last stage: where the forward
+// transform can start from them, and where that stage's radix is small -- the final passes (1024-voxel rows
+// of 1024x1024x512: 1.98 -> 1.61 ms) and, at radix 2, the pre-pass and the update (1.71 -> 1.60, 2.36 -> 2.30 ms).
+// With larger last radices the registers spill (ratio of 576-voxel rows 0.79 -> 0.83 ms, of 416-voxel rows
+// 0.57 -> 0.61 ms): those keep the sweep over the tile.
+constexpr bool y_fused(int p, int mode) {
+    if (p <= 0 || kPlans[p].nst < 2) return false;
+    if (same_end_radix(p)) return true;
+    const int r = kPlans[p].rad[kPlans[p].nst - 1];
+    return ((mode == Y_FINAL || mode == Y_RLFINAL) && r <= 8) || ((mode == Y_PRE || mode == Y_UPDATE) && r == 2);
+}
+
 // Number of per-voxel input arrays a y-pass mode stages in shared memory.
 __host__ __device__ inline int y_aux_arrays(int mode) {
     switch (mode) {
@@ -557,17 +569,17 @@ __global__ void __launch_bounds__(PK_THREADS, GEN >= 2 ? 2 : 3) k_y(const VolDes
     }
 
     bool fused = false;
-    if constexpr (same_end_radix(P)) {
+    if constexpr (y_fused(P, MODE)) {
         // the common cases only: damping, scaling, masks, crops and the scalar raw path keep the rolled
         // per-voxel loop below, so their code is not unrolled into this one
         constexpr bool kPostMode = mode == Y_FINAL || mode == Y_RLFINAL;
         const bool fuse_ok = !odd && !(mode == Y_PRE && raw_sync) &&
                              !(kPostMode && (d.damp > 1.f || d.scale_mode != 0 || d.need_xz));
         if (fuse_ok) {
-            // The inverse transform's last stage and the forward transform's first stage have the
-            // same radix, so each thread holds the same elements after the one and before the
-            // other: the per-voxel phase runs on registers between them.
-            constexpr int N = kPlans[P].n, NST = kPlans[P].nst, R = kPlans[P].rad[0];
+            // The per-voxel phase runs on the registers that the inverse transform's last stage leaves; the
+            // forward transform's first stage takes them from there where it has the same radix, else through
+            // the tile.
+            constexpr int N = kPlans[P].n, NST = kPlans[P].nst, R = kPlans[P].rad[NST - 1];
             constexpr int LL = plan_lines_y(N, TP), MS = N / R, MAXB = (LL * MS + NT - 1) / NT;
             float2 v[MAXB][R];
             if (spec_in) run_mid<P, 0, NST - 1, 1, LL, false, true>(buf, tw, tid);
@@ -698,8 +710,24 @@ __global__ void __launch_bounds__(PK_THREADS, GEN >= 2 ? 2 : 3) k_y(const VolDes
             if (spec_out) {
                 int tid2 = tid;  // opaque copy: the inverse's index arithmetic is not kept live for reuse
                 asm volatile("mov.b32 %0, %0;" : "+r"(tid2));
-                stage_r2s<R, N, LL, false, false>(buf, tid2, v);
-                run_mid<P, 1, NST, R, LL, false, false>(buf, tw, tid2);
+                if constexpr (same_end_radix(P)) {
+                    stage_r2s<R, N, LL, false, false>(buf, tid2, v);
+                    run_mid<P, 1, NST, R, LL, false, false>(buf, tw, tid2);
+                } else {
+                    // back to where the last stage's inputs were read (every thread has read its own by now)
+#pragma unroll
+                    for (int i = 0; i < MAXB; i++) {
+                        const int b = tid2 + i * NT;
+                        if (MAXB * NT == LL * MS || b < LL * MS) {
+                            const int l = b / MS, j = b - l * MS, a0 = l * N + j;
+                            const int p0 = pad(a0);
+#pragma unroll
+                            for (int r = 0; r < R; r++) buf[pstep<MS, false>(a0, p0, r)] = v[i][r];
+                        }
+                    }
+                    __syncthreads();
+                    run_mid<P, 0, NST, 1, LL, false, false>(buf, tw, tid2);
+                }
             }
             fused = true;
         }
