@@ -13,12 +13,11 @@
 //
 // XZ_CONV multiplies by the OTF on the elements that the forward transform's last stage leaves in registers;
 // with a pass over shared memory for the multiply, the convolution of plans whose first and last
-// radix differ was slower than the register-IO kernel.  Measured, before -> after (the launches of 16
-// chunks of 224-416 voxels, and single volumes): z 288 0.493 -> 0.408 ms, z 224 0.368 -> 0.307 ms, z 128 of
-// 512x512x128 0.089 -> 0.074 ms (5460 GB/s).  Lines above 512 come here too, on tiles as wide as shared
-// memory allows (the register-IO tile of 4096 points is 4 columns wide at 1024): x 1024 of 1024x1024x512
-// 1.13 -> 0.90 ms (4780 GB/s), z 512 there 2.85 -> 1.50 ms on 16 columns (4300 GB/s; 8 columns 1.96 ms), x 544
-// of 576x544x544 0.506 -> 0.308 ms, z 544 1.08 -> 0.60 ms.
+// radix differ was slower than the register-IO kernel.  Measured, before -> after: z 288 and 224 of 16 chunks of
+// 224-416 voxels 0.493 -> 0.472 ms and 0.368 -> 0.352 ms a launch.  Lines above 512 come here too, on tiles as wide
+// as shared memory allows (the register-IO tile of 4096 points is 4 columns wide at 1024): x 1024 of
+// 1024x1024x512 1.13 -> 0.78-0.92 ms, z 512 there 2.85 -> 1.48 ms on 16 columns (8 columns: 1.96 ms), x 544 of
+// 576x544x544 0.506 -> 0.308 ms, z 544 1.08 -> 0.69 ms.
 #pragma once
 #include <cstdlib>
 
