@@ -89,6 +89,12 @@ PK_API int32_t pk_ctx_profile_read(pk_ctx* ctx, char* buf, int32_t cap);
  * This writes the context's decisions as a JSON list and returns its length (truncated to cap-1). */
 PK_API int32_t pk_ctx_tune_read(pk_ctx* ctx, char* buf, int32_t cap);
 
+/* How the transforms of a volume of this extent run, decided from the extent alone (no device needed): a JSON list
+ * of the y, x and z axes, each with its complex length, engine ("plan": a compile-time plan; "mixed": run-time mixed
+ * radices; "sums": plain sums over prime factors above 31, register-tiled; "plain": the in-place engine), radices,
+ * lines per tile and largest shared memory of a pass.  Returns its length (truncated to cap-1), or minus a pk_status. */
+PK_API int32_t pk_plan_read(const int64_t dims[3], char* buf, int32_t cap);
+
 /* Failure-detection self-test (no counterpart in the reference).  Every wait inside the pass
  * kernels is bounded: a wait that runs out records it in the context's device-wait status word
  * and the kernel returns, and the next call on the context (or the synchronous call itself)

@@ -148,7 +148,7 @@ void pk_ctx_destroy(pk_ctx* ctx) {
         release_all(ctx);
         for (auto& kv : ctx->tw) cudaFree(kv.second.d);
         ctx->tw.clear();
-        for (auto& kv : ctx->gen) cudaFree(kv.second.second);
+        for (auto& kv : ctx->gen) cudaFree(kv.second);
         ctx->gen.clear();
         for (void* p : ctx->host_pinned) cudaFreeHost(p);
     for (auto& r : ctx->prof) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }

@@ -105,6 +105,7 @@ bool axis(int n, const float2* dtw, AxisDev* a) {
     a->twN = n;
     a->twStride = 1;
     a->plan = pk_find_plan(n);
+    a->engine = a->plan ? AE_PLAN : AE_PLAIN;
     return true;
 }
 

@@ -90,12 +90,12 @@ static size_t direct_xz_smem(int n, int lines) {
 }
 
 static size_t step_smem(int kind, int mode, const VolDesc& v) {
-    if (kind == PK_STEP_Y && v.ay.gen_direct)
+    if (kind == PK_STEP_Y && v.ay.engine == AE_SUMS)
         return sizeof(float2) * (tw_slots(v.M) + (v.odd ? 0 : v.M + 1) + padded_size(v.Ly * v.M) + v.Ly +
                                  (size_t)pkpass::y_aux_arrays(mode) * v.Ly * v.M) + 16 + sizeof(float4) * (size_t)v.Ly * v.M;
-    if (kind == PK_STEP_X && v.ax.gen_direct) return direct_xz_smem(v.ax.n, v.ax.gen_direct);
-    if (kind == PK_STEP_Z && v.az.gen_direct) return direct_xz_smem(v.az.n, v.az.gen_direct);
-    if (kind == PK_STEP_Y && v.ay.gen) {
+    if (kind == PK_STEP_X && v.ax.engine == AE_SUMS) return direct_xz_smem(v.ax.n, v.ax.gen_direct);
+    if (kind == PK_STEP_Z && v.az.engine == AE_SUMS) return direct_xz_smem(v.az.n, v.az.gen_direct);
+    if (kind == PK_STEP_Y && v.ay.engine == AE_MIXED) {
         const int lines = v.odd ? (v.Ly + 1) / 2 : v.Ly, len = v.odd ? v.M + 1 : v.M;
         return sizeof(float2) * ((v.odd ? 0 : v.M + 1) + 2 * (size_t)pkpass::gen_y_slots(lines, len) + v.Ly +
                                  (size_t)pkpass::y_aux_arrays(mode) * (v.odd ? pkpass::gen_y_slots(v.Ly, v.M) / 2 : v.Ly * v.M));
@@ -656,7 +656,7 @@ static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
     for (int i = 0; i < s.nvol && ok; i++) {
         const VolDesc& d = prog.descs[s.desc_off + i];
         const AxisDev& A = axis == 1 ? d.ax : d.az;
-        ok = A.gen && A.genT > 0 && encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
+        ok = A.engine == AE_MIXED && encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
         if (!ok) break;
         land = std::max(land, A.gen_land);
         work = std::max(work, A.gen_work);
@@ -1005,35 +1005,14 @@ static bool gen_smooth(int n) {
     return n == 1;
 }
 
-// Plan (stages, tile shape) of length n and its tables: the stages' twiddles, or for `direct` the in-place
-// engine's stages and the root matrices of the prime-factor ones.
-static bool gen_plan(int n, bool direct, GenAxis* g, std::vector<float2>& tables) {
-    *g = GenAxis();
-    g->n = n;
-    std::vector<int> rad;
-    if (n < 2) return false;
-    tables.clear();
-    if (direct) {
-        AxisPlan p;
-        if (n > kDirectMax || !pk_make_axis_plan(n, &p)) return false;
-        rad.assign(p.rad, p.rad + p.nst);
-        g->direct = 1;
-    } else if (!gen_smooth(n) || gen_search(n, n * std::max(1, gen_tile(n, g)), rad) > 1e29) {
-        return false;
-    }
-    for (int r : rad) g->big |= r > 16;
-    std::vector<float2> root(g->direct ? n : 0);
-    if (g->direct) pk_root_table(n, root.data());
-    auto magic = [](int d) { return d > 1 ? 0xFFFFFFFFu / (unsigned)d + 1u : 0u; };
-    g->nst = (int)rad.size();
-    int ns = 1;
+// Tables of a plan's stages: the mixed-radix engine's twiddles, or for `direct` the root matrices of the prime-factor
+// stages.  Fills the stages' offsets.
+static std::vector<float2> gen_tables(GenAxis* g) {
+    std::vector<float2> tables;
+    std::vector<float2> root(g->direct ? g->n : 0);
+    if (g->direct) pk_root_table(g->n, root.data());
     for (int s = 0; s < g->nst; s++) {
-        const int R = rad[s], tstep = n / (ns * R);
-        g->rad[s] = R;
-        g->ns[s] = ns;
-        g->m[s] = n / R;
-        g->mg_ns[s] = magic(ns);
-        g->mg_m[s] = magic(n / R);
+        const int n = g->n, R = g->rad[s], ns = g->ns[s], tstep = n / (ns * R);
         if (!g->direct) {
             g->off[s] = (int)tables.size();
             if (ns > 1)
@@ -1053,84 +1032,132 @@ static bool gen_plan(int n, bool direct, GenAxis* g, std::vector<float2>& tables
                         m[half + t] = w.y;
                     }
         }
-        ns *= R;
     }
-    return true;
+    return tables;
 }
 
-// Lines (32 to 4) per tile of a direct length, as many as their shared memory smem(lines)
+static void gen_stages(GenAxis* g, int n, const int* rad, int nst) {
+    auto magic = [](int d) { return d > 1 ? 0xFFFFFFFFu / (unsigned)d + 1u : 0u; };
+    g->n = n;
+    g->nst = nst;
+    int ns = 1;
+    for (int s = 0; s < nst; s++) {
+        g->rad[s] = rad[s];
+        g->big |= rad[s] > 16;
+        g->ns[s] = ns;
+        g->m[s] = n / rad[s];
+        g->mg_ns[s] = magic(ns);
+        g->mg_m[s] = magic(n / rad[s]);
+        ns *= rad[s];
+    }
+}
+
+// Mixed-radix plan (stages, tile shape) of length n; nst = 0 where it has none.  Kept for the process: it depends on
+// n alone, and the search for the radices is long.
+static const GenAxis& mixed_plan(int n) {
+    static std::mutex mu;
+    static std::map<int, GenAxis> plans;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = plans.find(n);
+    if (it == plans.end()) {
+        GenAxis g{};
+        std::vector<int> rad;
+        if (n >= 2 && gen_smooth(n) && gen_search(n, n * std::max(1, gen_tile(n, &g)), rad) < 1e29)
+            gen_stages(&g, n, rad.data(), (int)rad.size());
+        it = plans.emplace(n, g).first;
+    }
+    return it->second;
+}
+
+// Lines (32 to 4) per tile of a length with a prime factor above 31, as many as their shared memory smem(lines)
 // allows; the register radices of the in-place engine take 4096 points at most.  0: none, the plain engine (4
 // lines of 999 = 27 * 37 were 5% slower than it).
 template <class F>
-static int direct_lines(const GenAxis& g, F&& smem) {
+static int direct_lines(const AxisDev& a, F&& smem) {
     bool small = false;
-    for (int s = 0; s < g.nst; s++) small |= g.rad[s] <= 5 || g.rad[s] == 8 || g.rad[s] == 16;
+    for (int s = 0; s < a.nst; s++) small |= a.rad[s] <= 5 || a.rad[s] == 8 || a.rad[s] == 16;
     for (size_t lim : {(size_t)112 * 1024, (size_t)pkpass::kDirectSmem})   // two CTAs an SM, else one
         for (int c : {32, 16, 8, 4})
-            if ((!small || (c >= 8 && c * g.n <= PK_TILE_POINTS)) && smem(c) <= lim) return c;
+            if ((!small || (c >= 8 && c * a.n <= PK_TILE_POINTS)) && smem(c) <= lim) return c;
     return 0;
 }
 
-static pk_status pk_get_gen(pk_ctx* ctx, int n, bool direct, GenAxis* host, const GenAxis** dev) {
-    const int key = direct ? -n : n;
+// Device copy of the mixed-radix plan of length a.n, or of the plain engine's stages with their root matrices
+// (a.engine says which), made the first time it is asked for.
+static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) {
+    const int key = a.engine == AE_SUMS ? -a.n : a.n;
     auto it = ctx->gen.find(key);
     if (it == ctx->gen.end()) {
-        GenAxis g;
-        std::vector<float2> tables;
-        GenAxis* d = nullptr;
-        if (gen_plan(n, direct, &g, tables)) {
-            const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
-            PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
-            const float2* t = (const float2*)((const char*)d + head);
-            g.tw = t;
-            g.mat = (const float*)t;
-            cudaError_t e = cudaMemcpy(d, &g, sizeof(g), cudaMemcpyHostToDevice);
-            if (e == cudaSuccess && !tables.empty())
-                e = cudaMemcpy((void*)t, tables.data(), sizeof(float2) * tables.size(), cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) {
-                cudaFree(d);
-                PK_CUDA(e);
-            }
+        GenAxis g{};
+        if (a.engine == AE_SUMS) {
+            g.direct = 1;
+            gen_stages(&g, a.n, a.rad, a.nst);
+        } else {
+            g = mixed_plan(a.n);
         }
-        it = ctx->gen.emplace(key, std::make_pair(g, d)).first;
+        const std::vector<float2> tables = gen_tables(&g);
+        GenAxis* d = nullptr;
+        const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
+        PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
+        const float2* t = (const float2*)((const char*)d + head);
+        g.tw = t;
+        g.mat = (const float*)t;
+        cudaError_t e = cudaMemcpy(d, &g, sizeof(g), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && !tables.empty())
+            e = cudaMemcpy((void*)t, tables.data(), sizeof(float2) * tables.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(d);
+            PK_CUDA(e);
+        }
+        it = ctx->gen.emplace(key, d).first;
     }
-    *host = it->second.first;
-    *dev = it->second.second;
+    *dev = it->second;
     return PK_OK;
 }
 
-pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a, bool direct) {
+// Host part of an axis: its engine, stages and tile.  `sums`: the volume has a prime factor above 31; smem(a): shared
+// memory of a tile of a.gen_direct lines.
+template <class F>
+static bool choose_axis(int n, bool sums, AxisDev* a, F&& smem) {
     AxisPlan p;
-    if (!pk_make_axis_plan(n, &p)) return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
+    if (!pk_make_axis_plan(n, &p)) return false;
     memset(a, 0, sizeof(*a));
     a->n = n;
     a->nst = p.nst;
     for (int i = 0; i < p.nst; i++) a->rad[i] = p.rad[i];
-    a->twN = twN;
-    a->twStride = twN / n;
+    a->twN = n;
+    a->twStride = 1;
     a->plan = pk_find_plan(n);
-    if (a->plan == 0 && !(direct && gen_smooth(n))) {   // small factors sum as fast on the plain in-place engine
-        GenAxis g;
-        const pk_status st = pk_get_gen(ctx, n, direct, &g, &a->gen);
-        if (st != PK_OK) return st;
-        if (a->gen) {
-            a->genT = g.T;
-            a->gen_rows = g.rows;
-            a->gen_big = g.big;
-            if (g.direct)
-                a->gen_direct = direct_lines(g, [&](int c) { return direct_xz_smem(n, c); });
-            if (g.T) {
-                a->gen_land = pkpass::gen_land(g);
-                a->gen_work = pkpass::gen_work(g);
-            }
-        }
+    a->engine = a->plan ? AE_PLAN : AE_PLAIN;
+    if (a->plan) return true;
+    if (sums) {   // small factors sum as fast on the plain in-place engine
+        if (gen_smooth(n) || n > kDirectMax) return true;
+        AxisDev t = *a;
+        t.engine = AE_SUMS;
+        t.gen_direct = direct_lines(*a, [&](int c) {
+            t.gen_direct = c;
+            return smem(t);
+        });
+        if (t.gen_direct) *a = t;
+        return true;
     }
-    return pk_get_axis_table(ctx, n, &a->tw);
+    const GenAxis& g = mixed_plan(n);
+    if (!g.nst) return true;
+    a->engine = AE_MIXED;
+    a->gen_big = g.big;
+    a->genT = g.T;
+    a->gen_rows = g.rows;
+    if (g.T) {
+        a->gen_land = pkpass::gen_land(g);
+        a->gen_work = pkpass::gen_work(g);
+    }
+    return true;
 }
 
 static const int kThreads = PK_THREADS;
 
-pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
+// Engines, tiles and block counts of a volume, from its extent alone (no device memory, no context).
+static pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d) {
     memset(d, 0, sizeof(*d));
     if (ny < 1 || nx < 1 || nz < 1) return pk_fail(PK_ERR_INVALID, "volume dimensions must be positive");
     d->ny = ny; d->nx = nx; d->nz = nz;
@@ -1143,40 +1170,33 @@ pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
     if (d->M > P || nx > P || nz > P)
         return pk_fail(PK_ERR_UNSUPPORTED, "a transform axis is longer than " + std::to_string(P) +
                                                " (" + std::to_string(2 * P) + " along y)");
-    pk_status st;
     // a volume with a prime factor above 31 on any axis keeps the in-place engine's sums on all that have no plan:
     // the sums' roundings shift every voxel alike and partly cancel between the axes, so one axis made more
     // exact can leave the result less so (117 x 999 x 336 OMW x2: 0.9e-6 of its norm off, 1.4e-6 with 117 and
     // 336 on the mixed-radix engine and 999 as it was)
-    bool direct = false;
-    for (int n : {d->M, nx, nz}) direct = direct || (pk_find_plan(n) == 0 && !gen_smooth(n));
-    if ((st = pk_fill_axis(ctx, d->M, d->M, &d->ay, direct)) != PK_OK) return st;
-    if ((st = pk_fill_axis(ctx, nx, nx, &d->ax, direct)) != PK_OK) return st;
-    if ((st = pk_fill_axis(ctx, nz, nz, &d->az, direct)) != PK_OK) return st;
-    if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
-    if (d->ay.gen_direct) {
-        GenAxis g;
-        const GenAxis* dev;
-        if ((st = pk_get_gen(ctx, d->M, true, &g, &dev)) != PK_OK) return st;
-        d->ay.gen_direct = direct_lines(g, [&](int c) {
-            VolDesc t = *d;
-            t.Ly = t.ay.gen_direct = c;
-            return step_smem(PK_STEP_Y, Y_RLUPD, t);
-        });
-        if (!d->ay.gen_direct) d->ay.gen = nullptr;   // the plain in-place engine
-    }
-    if (d->ay.gen_direct) {
-        d->Ly = d->ay.gen_direct;
-    } else if (d->ay.gen) {   // odd rows run in pairs
+    bool sums = false;
+    for (int n : {d->M, nx, nz}) sums = sums || (pk_find_plan(n) == 0 && !gen_smooth(n));
+    auto xz_smem = [](const AxisDev& a) { return direct_xz_smem(a.n, a.gen_direct); };
+    auto y_smem = [&](const AxisDev& a) {
+        VolDesc t = *d;
+        t.ay = a;
+        t.Ly = a.gen_direct;
+        return step_smem(PK_STEP_Y, Y_RLUPD, t);
+    };
+    for (const auto& [n, a] : {std::make_pair(nx, &d->ax), std::make_pair(nz, &d->az)})
+        if (!choose_axis(n, sums, a, xz_smem))
+            return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
+    for (AxisDev* a : {&d->ax, &d->az})
+        if (a->engine == AE_MIXED && !a->genT) a->engine = AE_PLAIN;   // no tile fits
+    if (!choose_axis(d->M, sums, &d->ay, y_smem))
+        return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(d->M) + " needs too many radix stages");
+    if (d->ay.engine == AE_MIXED) {   // odd rows run in pairs
         d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->M);
-    } else {
-        d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
+        // a line whose engine buffers do not fit shared memory keeps the in-place engine
+        if (step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) d->ay.engine = AE_PLAIN;
     }
-    // a line whose engine buffers do not fit shared memory keeps the in-place engine
-    if (d->ay.gen && !d->ay.gen_direct && step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) {
-        d->ay.gen = nullptr;
-        d->Ly = std::max(1, P / d->M);
-    }
+    if (d->ay.engine == AE_SUMS) d->Ly = d->ay.gen_direct;
+    else if (d->ay.engine != AE_MIXED) d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
     if ((long long)d->Ly > d->nrows && d->ay.plan == 0 && !d->ay.gen_direct) d->Ly = (int)d->nrows;
     d->Tx = d->ax.gen_direct ? d->ax.gen_direct : d->ax.plan ? plan_cols_xz(nx) : std::max(1, std::min(P / nx, d->Py));
     d->Tz = d->az.gen_direct ? d->az.gen_direct : d->az.plan ? plan_cols_xz(nz) : std::max(1, std::min(P / nz, d->Py));
@@ -1203,6 +1223,17 @@ pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
     return PK_OK;
 }
 
+pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
+    pk_status st = pk_geometry(ny, nx, nz, d);
+    if (st != PK_OK) return st;
+    for (AxisDev* a : {&d->ay, &d->ax, &d->az}) {
+        if ((a->engine == AE_MIXED || a->engine == AE_SUMS) && (st = pk_get_gen(ctx, *a, &a->gen)) != PK_OK) return st;
+        if ((st = pk_get_axis_table(ctx, a->n, &a->tw)) != PK_OK) return st;
+    }
+    if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
+    return PK_OK;
+}
+
 size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; }
 
 // ------------------------------------------------------------------ programs
@@ -1212,10 +1243,12 @@ size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; 
 // Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels.
 static int step_plan(int kind, const VolDesc& v) {
     // lengths without a plan: the mixed-radix engine's y kernels, the kernels of a prime factor above 31
-    if (kind == PK_STEP_Y && v.ay.gen) return kNumPlans + (v.ay.gen_direct ? 2 : v.ay.gen_big);
-    if ((kind == PK_STEP_X && v.ax.gen_direct) || (kind == PK_STEP_Z && v.az.gen_direct)) return kNumPlans;
-    const int p = kind == PK_STEP_Y ? v.ay.plan : kind == PK_STEP_X ? v.ax.plan : kind == PK_STEP_Z ? v.az.plan : 0;
-    return (v.tiles_small && kind != PK_STEP_LAMBDA) ? kNumPlans + p : p;
+    if (kind == PK_STEP_LAMBDA) return 0;
+    const AxisDev& a = kind == PK_STEP_Y ? v.ay : kind == PK_STEP_X ? v.ax : v.az;
+    if (kind == PK_STEP_Y && a.engine == AE_MIXED) return kNumPlans + a.gen_big;
+    if (a.engine == AE_SUMS) return kNumPlans + (kind == PK_STEP_Y ? 2 : 0);
+    const int p = a.plan;
+    return v.tiles_small ? kNumPlans + p : p;
 }
 
 // One step per distinct transform plan among `vols` (a launch is instantiated for one plan).
@@ -1746,6 +1779,36 @@ extern "C" int32_t pk_ctx_tune_read(pk_ctx* ctx, char* buf, int32_t cap) {
     std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     std::string js = "[";
     for (size_t i = 0; i < ctx->tune_log.size(); i++) js += (i ? ", " : "") + ctx->tune_log[i];
+    js += "]";
+    if (buf && cap > 0) {
+        const int n = std::min((int)js.size(), cap - 1);
+        memcpy(buf, js.data(), n);
+        buf[n] = 0;
+    }
+    return (int32_t)js.size();
+}
+
+extern "C" int32_t pk_plan_read(const int64_t dims[3], char* buf, int32_t cap) {
+    if (!dims) return -(int32_t)pk_fail(PK_ERR_INVALID, "NULL dims");
+    for (int i = 0; i < 3; i++)
+        if (dims[i] < 1 || dims[i] > 2 * PK_TILE_POINTS) return -(int32_t)pk_fail(PK_ERR_UNSUPPORTED, "extent without a transform");
+    VolDesc d;
+    const pk_status s = pk_geometry((int)dims[0], (int)dims[1], (int)dims[2], &d);
+    if (s != PK_OK) return -(int32_t)s;
+    static const char* const names[] = {"plan", "plain", "mixed", "sums"};
+    std::string js = "[";
+    for (int kind : {PK_STEP_Y, PK_STEP_X, PK_STEP_Z}) {
+        const AxisDev& a = kind == PK_STEP_Y ? d.ay : kind == PK_STEP_X ? d.ax : d.az;
+        const bool tile = kind != PK_STEP_Y && a.engine == AE_MIXED;
+        const int* rad = a.engine == AE_PLAN ? kPlans[a.plan].rad : a.engine == AE_MIXED ? mixed_plan(a.n).rad : a.rad;
+        const int nst = a.engine == AE_PLAN ? kPlans[a.plan].nst : a.engine == AE_MIXED ? mixed_plan(a.n).nst : a.nst;
+        const size_t smem = tile ? pkpass::gen_smem(a.gen_land, a.gen_work) : step_smem(kind, kind == PK_STEP_Y ? (int)Y_RLUPD : (int)XZ_CONV, d);
+        js += std::string(js.size() > 1 ? ", " : "") + "{\"n\": " + std::to_string(a.n) + ", \"engine\": \"" + names[a.engine] +
+              "\", \"radices\": [";
+        for (int i = 0; i < nst; i++) js += (i ? ", " : "") + std::to_string(rad[i]);
+        js += "], \"lines\": " + std::to_string(kind == PK_STEP_Y ? d.Ly : tile ? a.genT : kind == PK_STEP_X ? d.Tx : d.Tz) +
+              ", \"smem\": " + std::to_string(smem) + "}";
+    }
     js += "]";
     if (buf && cap > 0) {
         const int n = std::min((int)js.size(), cap - 1);

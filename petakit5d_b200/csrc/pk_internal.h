@@ -53,6 +53,9 @@ struct GenAxis {
     int rows, nbox;        // x / z pass: the tile arrives as nbox boxes of `rows` elements of the line
 };
 
+// Engine of an axis: a compile-time plan, or for lengths without one the mixed radices of gen_engine.cuh, the
+// plain in-place engine, or the in-place engine with stage_direct for its large prime factors.
+enum AxisEngine : int { AE_PLAN = 0, AE_PLAIN = 1, AE_MIXED = 2, AE_SUMS = 3 };
 struct AxisDev {
     int n;            // complex transform length along the axis
     int nst;          // number of radix stages (runtime engine)
@@ -61,10 +64,11 @@ struct AxisDev {
     int twN;          // table length (= n)
     int twStride;     // 1
     int plan;         // compile-time plan id (0 = runtime engine)
-    const GenAxis* gen;   // plan 0: the length's run-time plan (device), or null: the in-place engine
+    int engine;       // AxisEngine
+    const GenAxis* gen;   // AE_MIXED, AE_SUMS: the length's run-time plan and tables (device)
     int genT, gen_rows;         // its T and rows, and an x / z tile's buffers (pass_gen.cuh)
     int gen_land, gen_work, gen_big;
-    int gen_direct;             // prime factor above 31: lines per tile (16, 8 or 4; 0: not direct)
+    int gen_direct;             // AE_SUMS: lines per tile (32, 16, 8 or 4)
 };
 
 // Pass modes of the y kernel.
@@ -180,7 +184,7 @@ struct pk_ctx {
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::map<int, TwTable> tw;                                   // twN -> table
-    std::map<int, std::pair<GenAxis, GenAxis*>> gen;             // run-time plans by length (negative: direct): host copy, device copy
+    std::map<int, GenAxis*> gen;                                 // run-time plans and tables by length (negative: AE_SUMS)
     // OTF cache: key = (psf content hash, ny, nx, nz)
     std::map<std::tuple<uint64_t, int, int, int>, OtfEntry> otf;
     std::vector<std::pair<void*, size_t>> scratch;               // reusable device buffers by slot
@@ -251,7 +255,6 @@ pk_status pk_fail(pk_status st, const std::string& msg);
 void pk_root_table(int n, float2* out);
 int pk_axis_table(int n, float2* out);   // writes at most n + PK_TW_EXTRA entries, returns the count
 pk_status pk_get_twiddles(pk_ctx* ctx, int twN, const float2** out);
-pk_status pk_fill_axis(pk_ctx* ctx, int n, int twN, AxisDev* a, bool direct = false);
 pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d);
 size_t pk_spec_elems(const VolDesc& d);   // complex elements of the half spectrum
 
