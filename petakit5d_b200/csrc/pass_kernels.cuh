@@ -554,6 +554,8 @@ __global__ void __launch_bounds__(PK_THREADS, GEN >= 2 ? 2 : 3) k_y(const VolDes
                 if (k >= Py) {
                     a.y = -a.y;
                     b.y = -b.y;
+                } else if (k == 0) {   // a row's bin 0 is its real part; an imaginary part would land in the partner
+                    a.y = b.y = 0.f;
                 }
                 buf[slot(p)] = make_float2(a.x - b.y, a.y + b.x);
             }
