@@ -806,6 +806,10 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
     all.no_graph = true;
     std::vector<int> zb(nslab + 1);
     for (int sl = 0; sl <= nslab; sl++) zb[sl] = (int)((long long)nz * sl / nslab);
+    // odd rows run in pairs (an odd row rides on the even one before it): slabs begin at an even plane, hence an
+    // even row, so that the pairs, and their roundings, are the whole volume's
+    if (j0.dims[0] & 1)
+        for (int sl = 1; sl < nslab; sl++) zb[sl] &= ~1;
     for (int sl = 0; sl < nslab; sl++)
         for (const PkStep& h : head)
             pk_program_add(all, h.kind, h.mode, {slab_view(prog.descs[h.desc_off], zb[sl], zb[sl + 1] - zb[sl],
