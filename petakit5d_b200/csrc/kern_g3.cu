@@ -4,6 +4,6 @@
 void pk_fill_kernels_g3(pkpass::KernelTable& t) {
     pkpass::RegisterYGen<3, 0>::fill(t);
     auto fn = pkpass::k_xz<0, PK_TILE_POINTS, true>;
-    t.xz[kNumPlans] = fn;
+    t.xz[pkpass::kSumsXZ] = fn;
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pkpass::kDirectSmem);
 }

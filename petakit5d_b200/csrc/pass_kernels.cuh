@@ -1090,9 +1090,11 @@ __global__ void __launch_bounds__(PK_THREADS, DIRECT ? 2 : xz_min_blocks(P)) k_x
 constexpr int kYModes = Y_C2R + 1;
 
 // Entries [0, kNumPlans) hold the 4096-point-tile kernels, [kNumPlans + p] the small-tile kernels
-// of plan p (small_tile_plan(p)); a program step's plan id carries that offset.  The y entries of the plans
-// without small tiles, kNumPlans .. kNumPlans + 2, hold the kernels of lengths without a plan (GEN 1 .. 3), the
-// x / z entry kNumPlans the one of those with a prime factor above 31.
+// of plan p (small_tile_plan(p)); a program step's plan id carries that offset.  The entries of the plans
+// without small tiles, kNumPlans .. kNumPlans + 2, hold the kernels of lengths without a plan: in y the mixed-radix
+// ones (radices up to 16, up to 31) and the plain sums', in x / z the plain sums' and the two ids of
+// the mixed-radix kernels, which have a table of their own (pass_gen.cuh; here the in-place engine, their fallback).
+constexpr int kMixedY = kNumPlans, kSumsY = kNumPlans + 2, kSumsXZ = kNumPlans, kMixedXZ = kNumPlans + 1;
 struct KernelTable {
     void (*y[2 * kNumPlans][kYModes])(const VolDesc*, const int*, int, int);
     void (*xz[2 * kNumPlans])(const VolDesc*, const int*, int, int, int);
@@ -1120,7 +1122,7 @@ template <int GEN, int MD>
 struct RegisterYGen {
     static void fill(KernelTable& t) {
         auto fn = k_y<0, MD, PK_TILE_POINTS, GEN>;
-        t.y[kNumPlans + GEN - 1][MD] = fn;
+        t.y[kMixedY + GEN - 1][MD] = fn;
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, GEN == 3 ? kDirectSmem : 200 * 1024);
         RegisterYGen<GEN, MD + 1>::fill(t);
     }

@@ -81,6 +81,7 @@ void pk_fill_all_kernels(pkpass::KernelTable& t) {
     pk_fill_kernels_g1(t);
     pk_fill_kernels_g2(t);
     pk_fill_kernels_g3(t);
+    for (int g = 0; g < 2; g++) t.xz[pkpass::kMixedXZ + g] = t.xz[0];   // where no tensor map can be made
 }
 
 // Dynamic shared memory of an x / z tile of `lines` columns of a length with a prime factor above 31: roots, tile,
@@ -647,20 +648,20 @@ static void fuse_conv3(pk_ctx* ctx, PkProgram& prog) {
     prog.steps.swap(out);
 }
 
-// An x / z step of lengths without a compile-time plan: the generic TMA kernel when every volume has a
-// run-time plan with a tile that fits shared memory, else the in-place engine of k_xz.
+// An x / z step of lengths on the mixed-radix engine: its TMA kernel when that is set up and every volume's spectrum
+// can be described to it, else the in-place engine of k_xz.
 static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
     s.gen = 0;
-    bool ok = gen_kernel().fn[0] && gen_kernel().fn[1];
-    int land = 0, work = 0, big = 0;
+    const int big = s.plan - pkpass::kMixedXZ;
+    bool ok = gen_kernel().fn[big];
+    int land = 0, work = 0;
     for (int i = 0; i < s.nvol && ok; i++) {
         const VolDesc& d = prog.descs[s.desc_off + i];
         const AxisDev& A = axis == 1 ? d.ax : d.az;
-        ok = A.engine == AE_MIXED && encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
+        ok = encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
         if (!ok) break;
         land = std::max(land, A.gen_land);
         work = std::max(work, A.gen_work);
-        big |= A.gen_big;
     }
     const size_t smem = pkpass::gen_smem(land, work);
     if (!ok || smem > (size_t)226 * 1024) return;
@@ -708,7 +709,7 @@ void assign_tma(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
             continue;
         }
         const int axis = s.kind == PK_STEP_X ? 1 : 2;
-        if ((s.kind == PK_STEP_X || s.kind == PK_STEP_Z) && s.plan == 0 && s.grid > 0) {
+        if ((s.kind == PK_STEP_X || s.kind == PK_STEP_Z) && (s.plan == pkpass::kMixedXZ || s.plan == pkpass::kMixedXZ + 1) && s.grid > 0) {
             assign_gen(prog, s, axis);
             continue;
         }
@@ -1240,13 +1241,14 @@ size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; 
 // A program is the full launch sequence of a call (or of a batch / serving round): every step's
 // descriptors and block prefix live in one device buffer uploaded once, so the launches run
 // back to back without host synchronisation and can be captured into a CUDA graph.
-// Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels.
+// Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels, or the engine of a
+// length without a plan.  Volumes share a step, hence a kernel, only where this agrees, so a volume's result does not
+// depend on the others of a batch or serving round.
 static int step_plan(int kind, const VolDesc& v) {
-    // lengths without a plan: the mixed-radix engine's y kernels, the kernels of a prime factor above 31
     if (kind == PK_STEP_LAMBDA) return 0;
     const AxisDev& a = kind == PK_STEP_Y ? v.ay : kind == PK_STEP_X ? v.ax : v.az;
-    if (kind == PK_STEP_Y && a.engine == AE_MIXED) return kNumPlans + a.gen_big;
-    if (a.engine == AE_SUMS) return kNumPlans + (kind == PK_STEP_Y ? 2 : 0);
+    if (a.engine == AE_MIXED) return (kind == PK_STEP_Y ? pkpass::kMixedY : pkpass::kMixedXZ) + a.gen_big;
+    if (a.engine == AE_SUMS) return kind == PK_STEP_Y ? pkpass::kSumsY : pkpass::kSumsXZ;
     const int p = a.plan;
     return v.tiles_small ? kNumPlans + p : p;
 }
@@ -1394,10 +1396,10 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
             rec.kind = pk_step_name(s);
             static const bool detail = getenv("PK_PROF_DETAIL") && getenv("PK_PROF_DETAIL")[0] == '1';
             if (detail) {   // diagnostics: the transform length and the kernel family in the kind
-                const int pl = s.plan % kNumPlans;
-                rec.kind += "@" + std::to_string(kPlans[pl].n) +
+                const VolDesc& d = prog.descs[s.desc_off];
+                rec.kind += "@" + std::to_string(s.kind == PK_STEP_Y ? d.ay.n : s.kind == PK_STEP_Z ? d.az.n : d.ax.n) +
                             (s.tma >= 0 ? ":tma" : s.gen ? ":gen" : s.yreg ? ":yreg" : s.kind == PK_STEP_Y ? ":rolled" : ":rio") +
-                            (s.plan >= kNumPlans ? "-1k" : "");
+                            (d.tiles_small ? "-1k" : "");
             }
             rec.bytes = pk_step_bytes(s, prog.descs.data() + s.desc_off);
             rec.a = take();
