@@ -687,21 +687,19 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
         return v;
     };
     // volumes of one plane have no z transform: one pass transforms x, multiplies and transforms back (three
-    // passes took 75 us on a 2048 x 2048 plane, the z pass of length 1 the longest of them; this one takes 30)
-    bool planes = true;
-    for (const VolDesc& d : base) planes = planes && d.nz == 1;
+    // passes took 75 us on a 2048 x 2048 plane, the z pass of length 1 the longest of them; this one takes 30),
+    // whatever volumes the call holds beside them
     auto conv = [&](int which) {
-        const auto descs = with([&](VolDesc& d, DeconJob& j, int) {
-            if (method == 1) { d.otf = which ? j.otf_b : j.otf_f; d.conj = 0; }
-            else { d.otf = j.otf_f; d.conj = which; }
-        });
-        if (planes) {
-            pk_program_add(prog, PK_STEP_X, XZ_CONV, descs);
-            return;
-        }
-        pk_program_add(prog, PK_STEP_X, XZ_FWD, base);
-        pk_program_add(prog, PK_STEP_Z, XZ_CONV, descs);
-        pk_program_add(prog, PK_STEP_X, XZ_INV, base);
+        std::vector<VolDesc> planes, vols;
+        for (const VolDesc& v : with([&](VolDesc& d, DeconJob& j, int) {
+                 if (method == 1) { d.otf = which ? j.otf_b : j.otf_f; d.conj = 0; }
+                 else { d.otf = j.otf_f; d.conj = which; }
+             }))
+            (v.nz == 1 ? planes : vols).push_back(v);
+        pk_program_add(prog, PK_STEP_X, XZ_CONV, planes);
+        pk_program_add(prog, PK_STEP_X, XZ_FWD, vols);
+        pk_program_add(prog, PK_STEP_Z, XZ_CONV, vols);
+        pk_program_add(prog, PK_STEP_X, XZ_INV, vols);
     };
     // debug runs launch each iteration's program on its own, then the caller's per-iteration work
     auto flush = [&]() -> pk_status {

@@ -203,6 +203,10 @@ void pk_server::build_steps(Request& r, const VolDesc& b, const float2* otf_f, c
         VolDesc z = base;
         if (r.method == 1) { z.otf = which ? otf_b : otf_f; z.conj = 0; }
         else { z.otf = otf_f; z.conj = which; }
+        if (b.nz == 1) {   // a plane convolves in one x pass, as in decon.cu
+            push(PK_STEP_X, XZ_CONV, z);
+            return;
+        }
         push(PK_STEP_X, XZ_FWD, base);
         push(PK_STEP_Z, XZ_CONV, z);
         push(PK_STEP_X, XZ_INV, base);

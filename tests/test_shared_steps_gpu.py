@@ -1,6 +1,6 @@
 """A volume's result does not depend on the volumes that share its launches: batches and served mixes of volumes on
-different transform engines (plain sums beside mixed radices, radices up to 16 beside larger ones) equal the
-single calls bit for bit."""
+different transform engines (plain sums beside mixed radices, radices up to 16 beside larger ones) and of planes beside
+volumes equal the single calls bit for bit."""
 import numpy as np
 import pytest
 
@@ -40,11 +40,14 @@ def _batch(method, vols, psf, numit):
     return K.batch_decon(vols, psfs, ids, numit, method, psfs_b, None, Background=100, save16bit=False)
 
 
-# z 40 and x 40 run the mixed-radix engine, beside a prime above 31 the plain sums; x 38 has a radix above 16
+# z 40 and x 40 run the mixed-radix engine, beside a prime above 31 the plain sums; x 38 has a radix above 16; a volume
+# of one plane convolves in one x pass
 MIXES = [
     [(64, 37, 40), (64, 40, 40), (64, 41, 40), (64, 42, 40)],
     [(64, 40, 40), (64, 40, 37), (74, 40, 40)],
     [(62, 38, 27), (62, 40, 27), (45, 38, 27), (45, 40, 27)],
+    [(64, 40, 1), (64, 40, 20), (64, 42, 1), (64, 40, 20)],
+    [(64, 64, 1), (64, 64, 32), (64, 37, 1), (64, 512, 1)],
 ]
 
 
