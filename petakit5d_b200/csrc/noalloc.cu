@@ -4,15 +4,16 @@
 // (a host application that owns the whole device pool, a plugin loaded into a process whose
 // allocator must not be bypassed), or code on a path where an allocation could fail or stall
 // (an instrument's acquisition loop, an allocation-free real-time section).  This entry point
-// runs the same pass kernels as pk_decon_lucy_omw_device but takes every work buffer -- the
-// background-subtracted input, the estimate, the spectrum, both OTFs, the twiddle tables and the
-// launch descriptors -- from one file-scope device array, g_noalloc_scratch, so it allocates no
+// runs the pass kernels of pk_decon_lucy_omw_device (where a compile-time plan exists, the register-IO
+// ones that its autotuner may choose) but takes every work buffer -- the
+// background-subtracted input, the estimate, the spectrum, both OTFs, the twiddle tables, the
+// launch descriptors and the tensor maps -- from one file-scope device array, g_noalloc_scratch, so it allocates no
 // device memory and calls no allocating CUDA or library routine.  The caller passes the input and
 // output volumes as device pointers (and the two PSFs as host arrays, copied into the array).
 //
 // Limits and sharing:
 //   * at most PK_NOALLOC_MAX_VOXELS voxels per volume (1,048,576, e.g. 128 x 128 x 64); larger
-//     volumes are rejected with PK_ERR_UNSUPPORTED.  The array (about 32.4 MB) is held on every
+//     volumes are rejected with PK_ERR_UNSUPPORTED.  The array (about 32.6 MB) is held on every
 //     GPU that loads the library until the process exits;
 //   * deconOffset and EdgeErosion (which need a mask volume) and NUMIT = 0 are rejected with
 //     PK_ERR_UNSUPPORTED; dampFactor, scaleFactor, save16bit and bbox are supported;
@@ -29,11 +30,13 @@
 #include <cstring>
 #include <mutex>
 
+#include "pass_gen.cuh"
 #include "pass_kernels.cuh"
 #include "pk_internal.h"
 #include "plans.h"
 
 void pk_fill_all_kernels(pkpass::KernelTable& t);
+void pk_fill_gen(pkpass::GenKernel& k);
 void set_post(VolDesc& d, const pk_decon_params* p, int mask_mode, void* d_out);
 
 #define PK_NOALLOC_MAX_VOXELS (1u << 20)
@@ -45,8 +48,18 @@ constexpr size_t kWorkBytes = 32ull * PK_NOALLOC_MAX_VOXELS + 4096;   // I, J, S
 constexpr int kTwEntries = 4096 + 8192 + 4096 + 4096;                 // y FFT, y split, x, z tables
 constexpr int kDescs = 12;
 constexpr size_t kTwBytes = sizeof(float2) * kTwEntries;
-constexpr size_t kMetaBytes = sizeof(VolDesc) * kDescs + 64 + 256;
-constexpr size_t kScratchBytes = kWorkBytes + kTwBytes + kMetaBytes;
+// lengths on the mixed-radix engine: plan and twiddles (16-byte groups) of y, x, z
+struct MixedTable {
+    GenAxis g;
+    alignas(16) float2 tw[2 * PK_TILE_POINTS];
+};
+struct Mixed {
+    MixedTable axis[3];
+    alignas(64) XZMaps map[2][3];   // x, z passes on the spectrum and both OTFs
+};
+constexpr size_t kMetaBytes = sizeof(VolDesc) * kDescs + 128 + 256;
+constexpr size_t kMixedOffset = (kWorkBytes + kTwBytes + kMetaBytes + 255) & ~(size_t)255;
+constexpr size_t kScratchBytes = kMixedOffset + sizeof(Mixed);
 
 // The scratch of every call.  Host code never takes its address directly: it passes the device
 // address looked up per device by cudaGetSymbolAddress.
@@ -59,7 +72,8 @@ void* g_addr[PK_NOALLOC_MAX_DEVICES] = {nullptr};
 struct Staging {
     float2 tw[kTwEntries];
     VolDesc desc[kDescs];
-    int prefix[8];
+    int prefix[16];
+    Mixed mixed;
 };
 Staging g_stage;
 
@@ -94,31 +108,8 @@ __global__ void k_na_psf_scatter(const float* __restrict__ psf, int py, int px, 
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-bool axis(int n, const float2* dtw, AxisDev* a) {
-    AxisPlan p;
-    if (!pk_make_axis_plan(n, &p)) return false;
-    memset(a, 0, sizeof(*a));
-    a->n = n;
-    a->nst = p.nst;
-    for (int i = 0; i < p.nst; i++) a->rad[i] = p.rad[i];
-    a->tw = dtw;
-    a->twN = n;
-    a->twStride = 1;
-    a->plan = pk_find_plan(n);
-    a->engine = a->plan ? AE_PLAN : AE_PLAIN;
-    return true;
-}
-
-size_t smem_for(int kind, int mode, const VolDesc& v) {
-    if (kind == PK_STEP_Y)
-        return sizeof(float2) * (tw_slots(v.M) + (v.odd ? 0 : v.M + 1) + pkfft::padded_size(v.Ly * v.M) + v.Ly +
-                                 (size_t)pkpass::y_aux_arrays(mode) * v.Ly * v.M);
-    const AxisDev& A = kind == PK_STEP_X ? v.ax : v.az;
-    const int T = kind == PK_STEP_X ? v.Tx : v.Tz;
-    return sizeof(float2) * (tw_slots(A.n) + pkfft::padded_size2(T * A.n) + (mode == XZ_CONV ? T * A.n : 0));
-}
-
 pkpass::KernelTable g_kt;
+pkpass::GenKernel g_gen;
 bool g_kt_dev[PK_NOALLOC_MAX_DEVICES] = {false};
 
 }  // namespace
@@ -176,6 +167,7 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     }
     if (!g_kt_dev[dev]) {
         pk_fill_all_kernels(g_kt);
+        pk_fill_gen(g_gen);
         g_kt_dev[dev] = true;
     }
     cudaStream_t st = (cudaStream_t)stream;
@@ -194,7 +186,8 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     char* twb = base + kWorkBytes;
     VolDesc* ddesc = (VolDesc*)(twb + kTwBytes);
     int* dprefix = (int*)((char*)ddesc + sizeof(VolDesc) * kDescs);
-    double* dsum = (double*)((char*)dprefix + 64);
+    double* dsum = (double*)((char*)dprefix + 128);
+    Mixed* dmix = (Mixed*)(base + kMixedOffset);
     const float2* tw_y = (const float2*)twb;
     const float2* tw_rc = tw_y + 4096;
     const float2* tw_x = tw_rc + 8192;
@@ -206,26 +199,22 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     pk_axis_table(nx, g_stage.tw + 4096 + 8192);
     pk_axis_table(nz, g_stage.tw + 4096 + 8192 + 4096);
     VolDesc v;
-    memset(&v, 0, sizeof(v));
-    v.ny = ny; v.nx = nx; v.nz = nz;
-    v.odd = ny & 1;
-    v.M = M;
-    v.Py = ny / 2 + 1;
-    v.Pp = v.Py + (v.Py & 1);
-    v.nrows = (long long)nx * nz;
-    if (!axis(M, tw_y, &v.ay) || !axis(nx, tw_x, &v.ax) || !axis(nz, tw_z, &v.az))
-        return pk_fail(PK_ERR_UNSUPPORTED, "transform length needs too many radix stages");
+    // a prime factor above 31: the plain engine's sums, which are the register-tiled ones' bit for bit; root matrices
+    // would not fit the array
+    if ((s = pk_geometry(ny, nx, nz, &v, false)) != PK_OK) return s;
+    v.ay.tw = tw_y;
+    v.ax.tw = tw_x;
+    v.az.tw = tw_z;
+    AxisDev* const axes[3] = {&v.ay, &v.ax, &v.az};
+    Mixed& mix = g_stage.mixed;
+    for (int k = 0; k < 3; k++) {
+        AxisDev& a = *axes[k];
+        if (a.engine != AE_MIXED) continue;
+        pk_mixed_tables(a.n, &mix.axis[k].g, mix.axis[k].tw);
+        mix.axis[k].g.tw = dmix->axis[k].tw;
+        a.gen = &dmix->axis[k].g;
+    }
     v.tw_rc = v.odd ? nullptr : tw_rc;
-    const int P = PK_TILE_POINTS;
-    v.Ly = v.ay.plan ? plan_lines_y(M) : (P / M > 1 ? P / M : 1);
-    if ((long long)v.Ly > v.nrows && v.ay.plan == 0) v.Ly = (int)v.nrows;
-    v.Tx = v.ax.plan ? plan_cols_xz(nx) : std::max(1, std::min(P / nx, v.Py));
-    v.Tz = v.az.plan ? plan_cols_xz(nz) : std::max(1, std::min(P / nz, v.Py));
-    v.blocksY = (int)((v.nrows + v.Ly - 1) / v.Ly);
-    v.blocksX = nz * ((v.Py + v.Tx - 1) / v.Tx);
-    v.blocksZ = nx * ((v.Py + v.Tz - 1) / v.Tz);
-    v.bb1[0] = ny - 1; v.bb1[1] = nx - 1; v.bb1[2] = nz - 1;
-    v.scale = 1.f;
     v.S = S;
     v.I = I;
     for (int k = 0; k < 3; k++) v.rdims[k] = (int)dims[k];
@@ -250,10 +239,23 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     h[D_FINN].Jo = J; h[D_FINN].Jn = J;
     set_post(h[D_FIN1], params, 0, d_out);
     set_post(h[D_FINN], params, 0, d_out);
-    int* pf = g_stage.prefix;   // [0, blocksY], [0, blocksX], [0, blocksZ]
-    pf[0] = 0; pf[1] = v.blocksY;
-    pf[2] = 0; pf[3] = v.blocksX;
-    pf[4] = 0; pf[5] = v.blocksZ;
+    // x, z passes on the mixed-radix engine, where the spectra can be described to it
+    bool gen[2];
+    float2* const specs[3] = {S, OF, OB};
+    for (int ax = 1; ax <= 2; ax++) {
+        gen[ax - 1] = axes[ax]->engine == AE_MIXED && g_gen.fn[axes[ax]->gen_big];
+        for (int q = 0; q < 3 && gen[ax - 1]; q++) {
+            VolDesc t = v;
+            t.S = specs[q];
+            gen[ax - 1] = pk_mixed_map(t, ax, &mix.map[ax - 1][q]);
+        }
+    }
+    int* pf = g_stage.prefix;   // [0, blocksY], [0, blocksX], [0, blocksZ], [0, mixed x tiles], [0, mixed z tiles]
+    const int cnt[5] = {v.blocksY, v.blocksX, v.blocksZ, gen[0] ? pk_mixed_tiles(v, 1) : 0, gen[1] ? pk_mixed_tiles(v, 2) : 0};
+    for (int k = 0; k < 5; k++) {
+        pf[2 * k] = 0;
+        pf[2 * k + 1] = cnt[k];
+    }
 
     // ---- uploads (pageable sources are staged before the calls return, so the static staging
     //      area can be rewritten by the next call)
@@ -264,17 +266,25 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     } while (0)
     NA_CUDA(cudaMemcpyAsync(twb, g_stage.tw, kTwBytes, cudaMemcpyHostToDevice, st));
     NA_CUDA(cudaMemcpyAsync(ddesc, g_stage.desc, sizeof(VolDesc) * kDescs, cudaMemcpyHostToDevice, st));
-    NA_CUDA(cudaMemcpyAsync(dprefix, g_stage.prefix, sizeof(int) * 6, cudaMemcpyHostToDevice, st));
+    NA_CUDA(cudaMemcpyAsync(dprefix, g_stage.prefix, sizeof(int) * 10, cudaMemcpyHostToDevice, st));
+    if (v.ay.gen || v.ax.gen || v.az.gen)
+        NA_CUDA(cudaMemcpyAsync(dmix, &g_stage.mixed, sizeof(Mixed), cudaMemcpyHostToDevice, st));
 
     auto launch = [&](int kind, int mode, int di) -> pk_status {
         const VolDesc& hv = h[di];
-        const size_t smem = smem_for(kind, mode, hv);
-        if (kind == PK_STEP_Y)
-            g_kt.y[hv.ay.plan][mode]<<<hv.blocksY, PK_THREADS, smem, st>>>(ddesc + di, dprefix, 1, mode);
-        else if (kind == PK_STEP_X)
-            g_kt.xz[hv.ax.plan]<<<hv.blocksX, PK_THREADS, smem, st>>>(ddesc + di, dprefix + 2, 1, 1, mode);
-        else
-            g_kt.xz[hv.az.plan]<<<hv.blocksZ, PK_THREADS, smem, st>>>(ddesc + di, dprefix + 4, 1, 2, mode);
+        const size_t smem = pk_step_smem(kind, mode, hv);
+        const int plan = pk_step_plan(kind, hv), ax = kind == PK_STEP_X ? 1 : 2;
+        if (kind == PK_STEP_Y) {
+            g_kt.y[plan][mode]<<<hv.blocksY, PK_THREADS, smem, st>>>(ddesc + di, dprefix, 1, mode);
+        } else if (gen[ax - 1]) {
+            const AxisDev& a = *axes[ax];
+            const size_t gs = pkpass::gen_smem(a.gen_land, a.gen_work);
+            const int q = hv.S == S ? 0 : hv.S == OF ? 1 : 2;
+            g_gen.fn[a.gen_big]<<<pk_mixed_grid(cnt[2 + ax], a.gen_big, gs), pkpass::kGenThreads, gs, st>>>(
+                ddesc + di, &dmix->map[ax - 1][q], dprefix + 4 + 2 * ax, 1, ax, mode, a.gen_land, a.gen_work, nullptr);
+        } else {
+            g_kt.xz[plan]<<<ax == 1 ? hv.blocksX : hv.blocksZ, PK_THREADS, smem, st>>>(ddesc + di, dprefix + 2 * ax, 1, ax, mode);
+        }
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return pk_fail(PK_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
         return PK_OK;
@@ -299,14 +309,16 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
 
     // ---- the OMW iterations (decon_lucy_omw_function.m:105-113), as in the context path
     if ((s = launch(PK_STEP_Y, Y_PRE, D_PRE)) != PK_OK) return s;
+    auto conv = [&](int di) -> pk_status {
+        if (nz == 1) return launch(PK_STEP_X, XZ_CONV, di);   // a plane convolves in one x pass
+        if ((s = launch(PK_STEP_X, XZ_FWD, D_BASE)) != PK_OK) return s;
+        if ((s = launch(PK_STEP_Z, XZ_CONV, di)) != PK_OK) return s;
+        return launch(PK_STEP_X, XZ_INV, D_BASE);
+    };
     for (int it = 1; it <= numit; it++) {
-        if ((s = launch(PK_STEP_X, XZ_FWD, D_BASE)) != PK_OK) return s;
-        if ((s = launch(PK_STEP_Z, XZ_CONV, D_ZF)) != PK_OK) return s;
-        if ((s = launch(PK_STEP_X, XZ_INV, D_BASE)) != PK_OK) return s;
+        if ((s = conv(D_ZF)) != PK_OK) return s;
         if ((s = launch(PK_STEP_Y, Y_RATIO, D_BASE)) != PK_OK) return s;
-        if ((s = launch(PK_STEP_X, XZ_FWD, D_BASE)) != PK_OK) return s;
-        if ((s = launch(PK_STEP_Z, XZ_CONV, D_ZB)) != PK_OK) return s;
-        if ((s = launch(PK_STEP_X, XZ_INV, D_BASE)) != PK_OK) return s;
+        if ((s = conv(D_ZB)) != PK_OK) return s;
         if (it < numit) s = launch(PK_STEP_Y, Y_UPDATE, it == 1 ? D_UPD1 : D_UPDN);
         else s = launch(PK_STEP_Y, Y_FINAL, it == 1 ? D_FIN1 : D_FINN);
         if (s != PK_OK) return s;

@@ -90,7 +90,7 @@ static size_t direct_xz_smem(int n, int lines) {
     return sizeof(float2) * (tw_slots(n) + padded_size2(lines * n)) + 16 + sizeof(float4) * (size_t)lines * n;
 }
 
-static size_t step_smem(int kind, int mode, const VolDesc& v) {
+size_t pk_step_smem(int kind, int mode, const VolDesc& v) {
     if (kind == PK_STEP_Y && v.ay.engine == AE_SUMS)
         return sizeof(float2) * (tw_slots(v.M) + (v.odd ? 0 : v.M + 1) + padded_size(v.Ly * v.M) + v.Ly +
                                  (size_t)pkpass::y_aux_arrays(mode) * v.Ly * v.M) + 16 + sizeof(float4) * (size_t)v.Ly * v.M;
@@ -391,7 +391,7 @@ int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& ge
         if (v < 0) {
             for (int r = 0; r < nrep; r++) {
                 pf[r + 1] = pf[r] + (axis == 1 ? dv[r].blocksX : dv[r].blocksZ);
-                smem = std::max(smem, step_smem(s.kind, s.mode, dv[r]));
+                smem = std::max(smem, pk_step_smem(s.kind, s.mode, dv[r]));
             }
             grid = pf[nrep];
         } else {
@@ -658,27 +658,19 @@ static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
     for (int i = 0; i < s.nvol && ok; i++) {
         const VolDesc& d = prog.descs[s.desc_off + i];
         const AxisDev& A = axis == 1 ? d.ax : d.az;
-        ok = encode_spec_box(&prog.maps[s.desc_off + i].s, d.S, d, axis, A.gen_rows, A.genT);
-        if (!ok) break;
+        ok = pk_mixed_map(d, axis, &prog.maps[s.desc_off + i]);
         land = std::max(land, A.gen_land);
         work = std::max(work, A.gen_work);
     }
-    const size_t smem = pkpass::gen_smem(land, work);
-    if (!ok || smem > (size_t)226 * 1024) return;
+    if (!ok) return;
     int* pf = prog.prefix.data() + s.prefix_off;
-    for (int i = 0; i < s.nvol; i++) {
-        const VolDesc& d = prog.descs[s.desc_off + i];
-        const AxisDev& A = axis == 1 ? d.ax : d.az;
-        pf[i + 1] = pf[i] + (axis == 1 ? d.nz : d.nx) * ((d.Py + A.genT - 1) / A.genT);
-    }
+    for (int i = 0; i < s.nvol; i++) pf[i + 1] = pf[i] + pk_mixed_tiles(prog.descs[s.desc_off + i], axis);
     s.grid = pf[s.nvol];
     s.gen = 1 + big;
-    s.tma_smem = smem;
+    s.tma_smem = pkpass::gen_smem(land, work);
     s.gen_land = land;
     s.gen_work = work;
-    // resident CTAs: two or three by registers, fewer where their shared memory (and its 1 KB a CTA) does not fit
-    const int per_sm = std::max(1, std::min(big ? 2 : 3, (int)((size_t)228 * 1024 / (smem + 1024))));
-    s.tma_grid = std::min(s.grid, per_sm * sm_count());
+    s.tma_grid = pk_mixed_grid(s.grid, big, s.tma_smem);
 }
 
 void assign_tma(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
@@ -811,6 +803,23 @@ __global__ void k_lambda(const VolDesc* __restrict__ descs, int nvol) {
 }
 
 }  // namespace
+
+// ---- launch shape of an x / z pass on the mixed-radix engine (pass_gen.cuh)
+bool pk_mixed_map(const VolDesc& d, int axis, XZMaps* m) {
+    const AxisDev& a = axis == 1 ? d.ax : d.az;
+    return encode_spec_box(&m->s, d.S, d, axis, a.gen_rows, a.genT);
+}
+
+int pk_mixed_tiles(const VolDesc& d, int axis) {
+    const AxisDev& a = axis == 1 ? d.ax : d.az;
+    return (axis == 1 ? d.nz : d.nx) * ((d.Py + a.genT - 1) / a.genT);
+}
+
+// resident CTAs: two or three by registers, fewer where their shared memory (and its 1 KB a CTA) does not fit
+int pk_mixed_grid(int tiles, int big, size_t smem) {
+    const int per_sm = std::max(1, std::min(big ? 2 : 3, (int)((size_t)228 * 1024 / (smem + 1024))));
+    return std::min(tiles, per_sm * sm_count());
+}
 
 // One CTA waits on an mbarrier that nothing arrives on: the bounded wait runs out after limit_ns
 // and the failure goes to the context's status word (the self-test of the device waits).
@@ -1006,35 +1015,37 @@ static bool gen_smooth(int n) {
     return n == 1;
 }
 
-// Tables of a plan's stages: the mixed-radix engine's twiddles, or for `direct` the root matrices of the prime-factor
-// stages.  Fills the stages' offsets.
-static std::vector<float2> gen_tables(GenAxis* g) {
-    std::vector<float2> tables;
-    std::vector<float2> root(g->direct ? g->n : 0);
-    if (g->direct) pk_root_table(g->n, root.data());
+// Tables of a plan's stages, in out (null: none written): the mixed-radix engine's twiddles, or for g->direct the root
+// matrices of the prime-factor stages.  Fills the stages' offsets; returns the tables' entries.
+static size_t gen_tables(GenAxis* g, float2* out) {
+    size_t cnt = 0;
+    std::vector<float2> root(g->direct && out ? g->n : 0);
+    if (!root.empty()) pk_root_table(g->n, root.data());
     for (int s = 0; s < g->nst; s++) {
         const int n = g->n, R = g->rad[s], ns = g->ns[s], tstep = n / (ns * R);
         if (!g->direct) {
-            g->off[s] = (int)tables.size();
-            if (ns > 1)
-                for (int k = 0; k < ns; k++)
-                    for (int r = 1; r <= pkgen::tw_row(R); r++)
-                        tables.push_back(root_of((int)((long long)r * k * tstep % n), n));
+            g->off[s] = (int)cnt;
+            if (ns == 1) continue;
+            const int row = pkgen::tw_row(R);
+            for (int k = 0; out && k < ns; k++)
+                for (int r = 1; r <= row; r++) out[cnt + (size_t)k * row + r - 1] = root_of((int)((long long)r * k * tstep % n), n);
+            cnt += (size_t)ns * row;
         } else if (R > 5 && R != 8 && R != 16) {
             const int half = direct_half(R);   // floats; a row is 2 half floats, half float2
-            g->off[s] = (int)tables.size() * 2;
-            tables.resize(tables.size() + (size_t)ns * R * half, make_float2(0.f, 0.f));
-            float* m = (float*)tables.data() + g->off[s];
-            for (int k = 0; k < ns; k++)
+            g->off[s] = (int)cnt * 2;
+            float* m = (float*)(out + cnt);
+            for (int k = 0; out && k < ns; k++)
                 for (int q = 0; q < R; q++, m += 2 * half)
-                    for (int t = 0; t < R; t++) {
-                        const float2 w = root[(size_t)((long long)q * (k + (long long)ns * t) * tstep % n)];
+                    for (int t = 0; t < half; t++) {
+                        const float2 w = t < R ? root[(size_t)((long long)q * (k + (long long)ns * t) * tstep % n)]
+                                               : make_float2(0.f, 0.f);
                         m[t] = w.x;
                         m[half + t] = w.y;
                     }
+            cnt += (size_t)ns * R * half;
         }
     }
-    return tables;
+    return cnt;
 }
 
 static void gen_stages(GenAxis* g, int n, const int* rad, int nst) {
@@ -1070,6 +1081,11 @@ static const GenAxis& mixed_plan(int n) {
     return it->second;
 }
 
+size_t pk_mixed_tables(int n, GenAxis* g, float2* out) {
+    *g = mixed_plan(n);
+    return gen_tables(g, out);
+}
+
 // Lines (32 to 4) per tile of a length with a prime factor above 31, as many as their shared memory smem(lines)
 // allows; the register radices of the in-place engine take 4096 points at most.  0: none, the plain engine (4
 // lines of 999 = 27 * 37 were 5% slower than it).
@@ -1096,7 +1112,8 @@ static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) 
         } else {
             g = mixed_plan(a.n);
         }
-        const std::vector<float2> tables = gen_tables(&g);
+        std::vector<float2> tables(gen_tables(&g, nullptr));
+        gen_tables(&g, tables.data());
         GenAxis* d = nullptr;
         const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
         PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
@@ -1119,7 +1136,7 @@ static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) 
 // Host part of an axis: its engine, stages and tile.  `sums`: the volume has a prime factor above 31; smem(a): shared
 // memory of a tile of a.gen_direct lines.
 template <class F>
-static bool choose_axis(int n, bool sums, AxisDev* a, F&& smem) {
+static bool choose_axis(int n, bool sums, bool matrices, AxisDev* a, F&& smem) {
     AxisPlan p;
     if (!pk_make_axis_plan(n, &p)) return false;
     memset(a, 0, sizeof(*a));
@@ -1132,7 +1149,7 @@ static bool choose_axis(int n, bool sums, AxisDev* a, F&& smem) {
     a->engine = a->plan ? AE_PLAN : AE_PLAIN;
     if (a->plan) return true;
     if (sums) {   // small factors sum as fast on the plain in-place engine
-        if (gen_smooth(n) || n > kDirectMax) return true;
+        if (!matrices || gen_smooth(n) || n > kDirectMax) return true;
         AxisDev t = *a;
         t.engine = AE_SUMS;
         t.gen_direct = direct_lines(*a, [&](int c) {
@@ -1158,7 +1175,7 @@ static bool choose_axis(int n, bool sums, AxisDev* a, F&& smem) {
 static const int kThreads = PK_THREADS;
 
 // Engines, tiles and block counts of a volume, from its extent alone (no device memory, no context).
-static pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d) {
+pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d, bool matrices) {
     memset(d, 0, sizeof(*d));
     if (ny < 1 || nx < 1 || nz < 1) return pk_fail(PK_ERR_INVALID, "volume dimensions must be positive");
     d->ny = ny; d->nx = nx; d->nz = nz;
@@ -1182,19 +1199,19 @@ static pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d) {
         VolDesc t = *d;
         t.ay = a;
         t.Ly = a.gen_direct;
-        return step_smem(PK_STEP_Y, Y_RLUPD, t);
+        return pk_step_smem(PK_STEP_Y, Y_RLUPD, t);
     };
     for (const auto& [n, a] : {std::make_pair(nx, &d->ax), std::make_pair(nz, &d->az)})
-        if (!choose_axis(n, sums, a, xz_smem))
+        if (!choose_axis(n, sums, matrices, a, xz_smem))
             return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
     for (AxisDev* a : {&d->ax, &d->az})
         if (a->engine == AE_MIXED && !a->genT) a->engine = AE_PLAIN;   // no tile fits
-    if (!choose_axis(d->M, sums, &d->ay, y_smem))
+    if (!choose_axis(d->M, sums, matrices, &d->ay, y_smem))
         return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(d->M) + " needs too many radix stages");
     if (d->ay.engine == AE_MIXED) {   // odd rows run in pairs
         d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->M);
         // a line whose engine buffers do not fit shared memory keeps the in-place engine
-        if (step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) d->ay.engine = AE_PLAIN;
+        if (pk_step_smem(PK_STEP_Y, Y_RLUPD, *d) > (size_t)200 * 1024) d->ay.engine = AE_PLAIN;
     }
     if (d->ay.engine == AE_SUMS) d->Ly = d->ay.gen_direct;
     else if (d->ay.engine != AE_MIXED) d->Ly = d->ay.plan ? plan_lines_y(d->M) : std::max(1, P / d->M);
@@ -1244,7 +1261,7 @@ size_t pk_spec_elems(const VolDesc& d) { return (size_t)d.Pp * (size_t)d.nrows; 
 // Kernel-table index of a pass: the axis plan, offset by kNumPlans for the small-tile kernels, or the engine of a
 // length without a plan.  Volumes share a step, hence a kernel, only where this agrees, so a volume's result does not
 // depend on the others of a batch or serving round.
-static int step_plan(int kind, const VolDesc& v) {
+int pk_step_plan(int kind, const VolDesc& v) {
     if (kind == PK_STEP_LAMBDA) return 0;
     const AxisDev& a = kind == PK_STEP_Y ? v.ay : kind == PK_STEP_X ? v.ax : v.az;
     if (a.engine == AE_MIXED) return (kind == PK_STEP_Y ? pkpass::kMixedY : pkpass::kMixedXZ) + a.gen_big;
@@ -1257,7 +1274,7 @@ static int step_plan(int kind, const VolDesc& v) {
 void pk_program_add(PkProgram& prog, int kind, int mode, const std::vector<VolDesc>& vols) {
     std::vector<int> plans;
     for (const VolDesc& v : vols) {
-        const int p = step_plan(kind, v);
+        const int p = pk_step_plan(kind, v);
         if (std::find(plans.begin(), plans.end(), p) == plans.end()) plans.push_back(p);
     }
     for (int plan : plans) {
@@ -1271,9 +1288,9 @@ void pk_program_add(PkProgram& prog, int kind, int mode, const std::vector<VolDe
         size_t smem = 0;
         int nv = 0;
         for (const VolDesc& v : vols) {
-            if (step_plan(kind, v) != plan) continue;
+            if (pk_step_plan(kind, v) != plan) continue;
             int blocks = kind == PK_STEP_Y ? v.blocksY : kind == PK_STEP_X ? v.blocksX : kind == PK_STEP_Z ? v.blocksZ : 1;
-            smem = std::max(smem, step_smem(kind, mode, v));
+            smem = std::max(smem, pk_step_smem(kind, mode, v));
             prog.prefix.push_back(prog.prefix.back() + blocks);
             prog.descs.push_back(v);
             nv++;
@@ -1804,7 +1821,7 @@ extern "C" int32_t pk_plan_read(const int64_t dims[3], char* buf, int32_t cap) {
         const bool tile = kind != PK_STEP_Y && a.engine == AE_MIXED;
         const int* rad = a.engine == AE_PLAN ? kPlans[a.plan].rad : a.engine == AE_MIXED ? mixed_plan(a.n).rad : a.rad;
         const int nst = a.engine == AE_PLAN ? kPlans[a.plan].nst : a.engine == AE_MIXED ? mixed_plan(a.n).nst : a.nst;
-        const size_t smem = tile ? pkpass::gen_smem(a.gen_land, a.gen_work) : step_smem(kind, kind == PK_STEP_Y ? (int)Y_RLUPD : (int)XZ_CONV, d);
+        const size_t smem = tile ? pkpass::gen_smem(a.gen_land, a.gen_work) : pk_step_smem(kind, kind == PK_STEP_Y ? (int)Y_RLUPD : (int)XZ_CONV, d);
         js += std::string(js.size() > 1 ? ", " : "") + "{\"n\": " + std::to_string(a.n) + ", \"engine\": \"" + names[a.engine] +
               "\", \"radices\": [";
         for (int i = 0; i < nst; i++) js += (i ? ", " : "") + std::to_string(rad[i]);

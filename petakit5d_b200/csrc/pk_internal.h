@@ -255,7 +255,18 @@ pk_status pk_fail(pk_status st, const std::string& msg);
 void pk_root_table(int n, float2* out);
 int pk_axis_table(int n, float2* out);   // writes at most n + PK_TW_EXTRA entries, returns the count
 pk_status pk_get_twiddles(pk_ctx* ctx, int twN, const float2** out);
+// engines, tiles and block counts of a volume, from its extent alone (matrices = false: without AE_SUMS, whose root
+// matrices take up to 33 MB); pk_init_desc adds the context's tables
+pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d, bool matrices = true);
 pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d);
+int pk_step_plan(int kind, const VolDesc& v);                        // a pass's kernel-table index
+size_t pk_step_smem(int kind, int mode, const VolDesc& v);           // and its dynamic shared memory
+// mixed-radix engine: the plan of length n and its twiddles (fewer than 2 n; out may be null), and a pass's tensor map,
+// tiles and grid
+size_t pk_mixed_tables(int n, GenAxis* g, float2* out);
+bool pk_mixed_map(const VolDesc& d, int axis, XZMaps* m);
+int pk_mixed_tiles(const VolDesc& d, int axis);
+int pk_mixed_grid(int tiles, int big, size_t smem);
 size_t pk_spec_elems(const VolDesc& d);   // complex elements of the half spectrum
 
 // launch programs (passes.cu)
