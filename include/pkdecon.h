@@ -64,7 +64,7 @@ PK_API void pk_params_default(pk_decon_params* p);
  * decon_lucy_omw_function.m:53-73 with an explicit context bound to one device. */
 PK_API pk_ctx* pk_ctx_create(int device);
 PK_API void pk_ctx_destroy(pk_ctx* ctx);
-/* Drop cached OTFs and work buffers (the demo's reset(gpuDevice), demo_RL_deconvolution.m:164-167). */
+/* Drop cached OTFs, transform plans' tables and work buffers (the demo's reset(gpuDevice), demo_RL_deconvolution.m:164-167). */
 PK_API pk_status pk_ctx_reset(pk_ctx* ctx);
 PK_API const char* pk_last_error(void);
 PK_API const char* pk_version(void);

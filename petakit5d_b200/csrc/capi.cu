@@ -127,6 +127,9 @@ static void release_all(pk_ctx* ctx) {
     ctx->graph_seen.clear();
     for (auto& kv : ctx->otf) cudaFree(kv.second.d);
     ctx->otf.clear();
+    for (auto& kv : ctx->gen) cudaFree(kv.second);
+    ctx->gen.clear();
+    ctx->sums_bytes = 0;
     for (auto& s : ctx->scratch)
         if (s.first) cudaFree(s.first);
     ctx->scratch.clear();
@@ -148,8 +151,6 @@ void pk_ctx_destroy(pk_ctx* ctx) {
         release_all(ctx);
         for (auto& kv : ctx->tw) cudaFree(kv.second.d);
         ctx->tw.clear();
-        for (auto& kv : ctx->gen) cudaFree(kv.second);
-        ctx->gen.clear();
         for (void* p : ctx->host_pinned) cudaFreeHost(p);
     for (auto& r : ctx->prof) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     for (auto e : ctx->ev_pool) cudaEventDestroy(e);

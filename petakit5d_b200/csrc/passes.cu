@@ -1099,8 +1099,17 @@ static int direct_lines(const AxisDev& a, F&& smem) {
     return 0;
 }
 
+// Root matrices a context keeps (8 n^2 bytes for a prime n: 1.7 MB at 467, 33 MB at 2039): regions drawn by hand bring
+// a new length every call.  Lengths past the limit, and ones whose matrices could not be allocated, run
+// the same sums on the plain engine, bit for bit, 1.7 times as long; pk_ctx_reset starts over.
+static size_t sums_limit() {
+    const char* e = getenv("PK_SUMS_MB");   // another limit, in MB
+    return (e && *e ? (size_t)std::max(0, atoi(e)) : (size_t)512) << 20;
+}
+
 // Device copy of the mixed-radix plan of length a.n, or of the plain engine's stages with their root matrices
-// (a.engine says which), made the first time it is asked for.
+// (a.engine says which), made the first time it is asked for; null for matrices that are not kept.  A length's answer
+// stands until pk_ctx_reset: the descriptors that a call makes of one volume agree.
 static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) {
     const int key = a.engine == AE_SUMS ? -a.n : a.n;
     auto it = ctx->gen.find(key);
@@ -1113,10 +1122,19 @@ static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) 
             g = mixed_plan(a.n);
         }
         std::vector<float2> tables(gen_tables(&g, nullptr));
-        gen_tables(&g, tables.data());
         GenAxis* d = nullptr;
-        const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15;
-        PK_CUDA(cudaMalloc(&d, head + sizeof(float2) * tables.size()));
+        const size_t head = (sizeof(GenAxis) + 15) & ~(size_t)15, bytes = head + sizeof(float2) * tables.size();
+        if (g.direct) {
+            if (ctx->sums_bytes + bytes > sums_limit() || cudaMalloc(&d, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                ctx->gen.emplace(key, nullptr);
+                *dev = nullptr;
+                return PK_OK;
+            }
+        } else {
+            PK_CUDA(cudaMalloc(&d, bytes));
+        }
+        gen_tables(&g, tables.data());
         const float2* t = (const float2*)((const char*)d + head);
         g.tw = t;
         g.mat = (const float*)t;
@@ -1127,6 +1145,7 @@ static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) 
             cudaFree(d);
             PK_CUDA(e);
         }
+        if (g.direct) ctx->sums_bytes += bytes;
         it = ctx->gen.emplace(key, d).first;
     }
     *dev = it->second;
@@ -1244,10 +1263,15 @@ pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d, bool matrices) {
 pk_status pk_init_desc(pk_ctx* ctx, int ny, int nx, int nz, VolDesc* d) {
     pk_status st = pk_geometry(ny, nx, nz, d);
     if (st != PK_OK) return st;
+    bool kept = true;
     for (AxisDev* a : {&d->ay, &d->ax, &d->az}) {
-        if ((a->engine == AE_MIXED || a->engine == AE_SUMS) && (st = pk_get_gen(ctx, *a, &a->gen)) != PK_OK) return st;
-        if ((st = pk_get_axis_table(ctx, a->n, &a->tw)) != PK_OK) return st;
+        if (a->engine != AE_MIXED && a->engine != AE_SUMS) continue;
+        if ((st = pk_get_gen(ctx, *a, &a->gen)) != PK_OK) return st;
+        kept = kept && a->gen;
     }
+    if (!kept && (st = pk_geometry(ny, nx, nz, d, false)) != PK_OK) return st;   // beside a large prime none is AE_MIXED
+    for (AxisDev* a : {&d->ay, &d->ax, &d->az})
+        if ((st = pk_get_axis_table(ctx, a->n, &a->tw)) != PK_OK) return st;
     if (!d->odd && (st = pk_get_twiddles(ctx, ny, &d->tw_rc)) != PK_OK) return st;
     return PK_OK;
 }

@@ -184,7 +184,9 @@ struct pk_ctx {
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::map<int, TwTable> tw;                                   // twN -> table
-    std::map<int, GenAxis*> gen;                                 // run-time plans and tables by length (negative: AE_SUMS)
+    std::map<int, GenAxis*> gen;                                 // run-time plans and tables by length (negative: AE_SUMS,
+                                                                 // null where its matrices are not kept)
+    size_t sums_bytes = 0;                                       // AE_SUMS tables
     // OTF cache: key = (psf content hash, ny, nx, nz)
     std::map<std::tuple<uint64_t, int, int, int>, OtfEntry> otf;
     std::vector<std::pair<void*, size_t>> scratch;               // reusable device buffers by slot
