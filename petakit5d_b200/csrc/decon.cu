@@ -351,6 +351,27 @@ pk_status pk_scratch(pk_ctx* ctx, int slot, size_t bytes, void** ptr) {
     return PK_OK;
 }
 
+pk_status pk_dev_table(pk_ctx* ctx, const std::string& key, const std::function<std::vector<char>()>& make, void** ptr) {
+    auto it = ctx->dev_tables.find(key);
+    if (it == ctx->dev_tables.end()) {
+        const std::vector<char> host = make();
+        void* d = nullptr;
+        if (cudaMalloc(&d, std::max<size_t>(1, host.size())) != cudaSuccess) {
+            cudaGetLastError();
+            return pk_fail(PK_ERR_NOMEM, "table allocation failed");
+        }
+        const cudaError_t e = cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(d);
+            return pk_fail(PK_ERR_CUDA, std::string("table upload: ") + cudaGetErrorString(e));
+        }
+        it = ctx->dev_tables.emplace(key, d).first;   // only a filled table is kept
+    }
+    *ptr = it->second;
+    return PK_OK;
+}
+
 enum { SL_ARENA = 0, SL_JB = 2, SL_S = 5, SL_MASK2 = 7, SL_IN = 9, SL_OUT = 10, SL_PSF = 11, SL_SUM = 12,
        SL_ZC = 14 };
 
@@ -358,18 +379,15 @@ enum { SL_ARENA = 0, SL_JB = 2, SL_S = 5, SL_MASK2 = 7, SL_IN = 9, SL_OUT = 10, 
 static pk_status erode_mask(pk_ctx* ctx, uint8_t* mask, int ny, int nx, int nz, int E, const unsigned* zeros,
                             cudaStream_t st) {
     const int R = E - 1;
-    void*& hw = ctx->dev_tables["disk:" + std::to_string(R)];   // the disk's runs, once per radius
-    if (!hw) {
+    const size_t words = (size_t)((ny + 31) / 32) * nx * nz;
+    void *hw, *b;
+    pk_status s;
+    const auto runs = [&] {   // the disk's runs, once per radius
         std::vector<int> h(2 * R + 1, -1);
         for (const int2& o : pk_disk_offsets(R)) h[o.y + R] = std::max(h[o.y + R], o.x);
-        void* d = nullptr;
-        PK_CUDA(cudaMalloc(&d, sizeof(int) * h.size()));
-        hw = d;
-        PK_CUDA(cudaMemcpy(hw, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice));
-    }
-    const size_t words = (size_t)((ny + 31) / 32) * nx * nz;
-    void* b;
-    pk_status s;
+        return std::vector<char>((const char*)h.data(), (const char*)(h.data() + h.size()));
+    };
+    if ((s = pk_dev_table(ctx, "disk:" + std::to_string(R), runs, &hw)) != PK_OK) return s;
     if ((s = pk_scratch(ctx, SL_MASK2, 2 * words * sizeof(unsigned), &b)) != PK_OK) return s;
     unsigned *b0 = (unsigned*)b, *b1 = b0 + words;
     const int gr = grid_for((long long)nx * nz * 32);

@@ -528,20 +528,16 @@ pk_status dsr_run(pk_ctx* ctx, const void* d_in, pk_dtype t, const int64_t dims[
         // the slice tables depend only on the geometry: built and uploaded once per context
         char key[160];
         snprintf(key, sizeof(key), "dsr:%d:%a:%a:%d", nz, P.stepsize, P.xstep, reverse);
-        void*& dtab = ctx->dev_tables[key];
-        if (!dtab) {
+        void* dtab;
+        const auto tables = [&] {
             const size_t tb = sizeof(SkewSlice) * nsl + 4 * zindex.size() + zorig.size();
             std::vector<char> host(tb, 0);
             memcpy(host.data(), sl.data(), sizeof(SkewSlice) * sl.size());
             memcpy(host.data() + sizeof(SkewSlice) * nsl, zindex.data(), 4 * zindex.size());
             memcpy(host.data() + sizeof(SkewSlice) * nsl + 4 * zindex.size(), zorig.data(), zorig.size());
-            if (cudaMalloc(&dtab, tb) != cudaSuccess) {
-                cudaGetLastError();
-                ctx->dev_tables.erase(key);
-                return pk_fail(PK_ERR_NOMEM, "deskew: table allocation failed");
-            }
-            PK_CUDA(cudaMemcpy(dtab, host.data(), tb, cudaMemcpyHostToDevice));
-        }
+            return host;
+        };
+        if ((s = pk_dev_table(ctx, key, tables, &dtab)) != PK_OK) return s;
         char* tp = (char*)dtab;
         SkewSlice* dsl = (SkewSlice*)tp;
         int* dzindex = (int*)(tp + sizeof(SkewSlice) * nsl);

@@ -345,6 +345,8 @@ pk_status pk_dloop_instance(DlRing* d_ring, cudaStream_t st, cudaGraphExec_t* ou
 
 // scratch buffers
 pk_status pk_scratch(pk_ctx* ctx, int slot, size_t bytes, void** ptr);
+// the context's read-only device table `key`, made from the bytes that make() returns the first time it is asked for
+pk_status pk_dev_table(pk_ctx* ctx, const std::string& key, const std::function<std::vector<char>()>& make, void** ptr);
 
 // PSF-size volume helpers (psfvol.cu, decon.cu)
 std::vector<int4> pk_ball_offsets(int r);           // strel('sphere', r): (dy, dx, dz, 0), dy^2+dx^2+dz^2 <= r^2
