@@ -340,8 +340,9 @@ std::string variant_name(int plan, int idx, int v) {
 
 // Times each candidate of step `s` on scratch buffers: one volume per entry of `geo` (the step's
 // own volume, or for a multi-volume step of a batch or a serving round the geometries of its first
-// volumes), each with its own zeroed buffers, descriptor and tensor maps; returns the fastest, or -2
-// when nothing could be timed. ms[i] receives candidate i's time.
+// volumes), each with its own zeroed buffers, descriptor and tensor maps; returns the fastest, -2
+// when none of them ran, or -3 when there was no memory for the scratch, or the stream or an event failed.
+// ms[i] receives candidate i's time.
 int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& geo, int idx, const std::vector<int>& cands,
                     cudaStream_t st, std::vector<float>& ms) {
     const pkpass::TmaTable* t = tma_kernels();
@@ -365,7 +366,7 @@ int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& ge
     char* d = nullptr;   // stream-ordered: a device-wide synchronisation here would wait on a serving dispatcher
     if (cudaMallocAsync((void**)&d, soff + off[nrep], st) != cudaSuccess) {
         cudaGetLastError();
-        return -2;
+        return -3;
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int best = -2;
@@ -442,7 +443,7 @@ int time_candidates(pk_ctx* ctx, const PkStep& s, const std::vector<VolDesc>& ge
     }
     if (!ok) {
         cudaGetLastError();
-        best = -2;
+        best = -3;
     }
     cudaFreeAsync(d, st);
     cudaStreamSynchronize(st);
@@ -532,6 +533,8 @@ int choose_variant(pk_ctx* ctx, const PkProgram& prog, const PkStep& s, int idx,
     const bool capturing = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
     if (capturing) cudaGetLastError();
     if ((off && off[0] == '0') || capturing) return fallback;   // no timing here
+    auto& tries = ctx->tune_tries[key];
+    if (tries.first && tries.second == ctx->tune_program) return fallback;   // this program has tried
     // the timed geometry: the step's volume; for a multi-volume step, its volumes in order (each with
     // its own scratch buffers), up to 16 of them within the scratch limit, so that a batch of mixed
     // shapes is timed on its own mix (copies of one volume ranked the x tiles of a 96-chunk batch the
@@ -567,8 +570,15 @@ int choose_variant(pk_ctx* ctx, const PkProgram& prog, const PkStep& s, int idx,
     std::vector<float> ms;
     PkRange range("pk autotune");
     int best = time_candidates(ctx, s, geo, idx, cands, st, ms);
-    if (best == -2) {   // nothing could be timed: the next call does not try again
+    if (best < 0 && best != -1) {
+        // a moment without memory for the scratch does not fix the choice: later programs try again, twice; a step that
+        // cannot be timed keeps the fallback
+        if (best == -3 && ++tries.first < 3) {
+            tries.second = ctx->tune_program;
+            return fallback;
+        }
         ctx->tune[key] = fallback;
+        record(fallback, "untimed", nullptr, dt);
         return fallback;
     }
     ctx->tune[key] = best;
@@ -674,6 +684,7 @@ static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
 }
 
 void assign_tma(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
+    if (ctx) ctx->tune_program++;
     fuse_conv3(ctx, prog);
     prog.maps.assign(prog.descs.size(), XZMaps());
     const pkpass::YregTable* yt = yreg_kernels();

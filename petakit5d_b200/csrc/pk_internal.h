@@ -240,6 +240,9 @@ struct pk_ctx {
     // autotuner of the x / z passes: chosen variant per (pass, plan, geometry) key (-1 = register-IO
     // kernel, 0.. = TMA variant), and a JSON record of each decision (pk_ctx_tune_read)
     std::map<std::vector<long long>, int> tune;
+    // timings that failed for want of memory: how often, in which program last
+    std::map<std::vector<long long>, std::pair<int, long long>> tune_tries;
+    long long tune_program = 0;
     std::vector<std::string> tune_log;
 };
 
