@@ -76,13 +76,7 @@ __global__ void k_post_from(VolDesc d, const float* __restrict__ src) {
         }
         if (d.scale_mode == 1) J = __fmul_rn(J, d.scale);
         else if (d.scale_mode == 2) {
-            int m = 1;
-            if (d.mask_mode == 1 || d.mask_mode == 3) m = d.mask8[i] != 0;
-            else if (d.mask_mode == 2) {
-                const int E = d.erosion;
-                m = d.mask8[i] != 0 && y >= E && y < d.ny - E && x >= E && x < d.nx - E &&
-                    (d.nz == 1 || (z >= E && z < d.nz - E));      // one plane: MATLAB's 2-D case
-            }
+            const int m = d.mask_mode ? d.mask8[i] != 0 : 1;
             J = __fmul_rn(__fadd_rn(__fmul_rn(J, d.scale), d.offset), (float)m);
         }
         const long long oy = d.bb1[0] - d.bb0[0] + 1, ox = d.bb1[1] - d.bb0[1] + 1;
@@ -486,7 +480,6 @@ void set_post(VolDesc& d, const pk_decon_params* p, int mask_mode, void* d_out) 
     d.damp = (float)p->damp_factor;
     d.scale = (float)p->scale_factor;
     d.offset = (float)p->decon_offset;
-    d.erosion = p->edge_erosion;
     if (p->scale_factor != 1.0 || off || ero) d.scale_mode = (off || ero) ? 2 : 1;
     else d.scale_mode = 0;
     d.mask_mode = d.scale_mode == 2 ? mask_mode : 0;
@@ -502,7 +495,6 @@ void set_post(VolDesc& d, const pk_decon_params* p, int mask_mode, void* d_out) 
     d.crop = 0;
     for (int i = 0; i < 3; i++)
         if (d.bb0[i] != 0 || d.bb1[i] != dims[i] - 1) d.crop = 1;
-    d.need_xz = d.crop || d.mask_mode == 2;
 }
 
 pk_status pk_check_params(const int64_t dims[3], const pk_decon_params* p) {
@@ -667,7 +659,7 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
     }
     PkProgram prog;
     pk_program_add(prog, PK_STEP_Y, Y_PRE, base);
-    const std::vector<int> mask_mode(nj, need_mask ? 1 : 0);
+    const int mask_mode = need_mask ? 1 : 0;
     if (p->edge_erosion > 0) {
         // the masks are eroded behind the pre-pass, which writes them and counts the raw zeros
         if ((s = pk_program_upload(ctx, prog, st)) != PK_OK) return s;
@@ -690,7 +682,7 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
         }
         for (size_t i = 0; i < nj; i++) {
             VolDesc f = base[i];
-            set_post_job(f, p, mask_mode[i], jobs[i]);
+            set_post_job(f, p, mask_mode, jobs[i]);
             k_post_from<<<grid_for((long long)f.nrows * f.ny), 256, 0, st>>>(f, f.I);
             PK_CUDA(cudaGetLastError());
         }
@@ -733,10 +725,10 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
             pk_program_add(prog, PK_STEP_Y, Y_RATIO, base);
             conv(1);
             const bool last = it == numit && !dbg;
-            pk_program_add(prog, PK_STEP_Y, last ? Y_FINAL : Y_UPDATE, with([&](VolDesc& d, DeconJob& j, int i) {
+            pk_program_add(prog, PK_STEP_Y, last ? Y_FINAL : Y_UPDATE, with([&](VolDesc& d, DeconJob& j, int) {
                 d.Jo = it == 1 ? j.I : j.J;
                 d.Jn = j.J;
-                if (last) set_post_job(d, p, mask_mode[i], j);
+                if (last) set_post_job(d, p, mask_mode, j);
             }));
             if (dbg) {
                 if ((s = flush()) != PK_OK) return s;
@@ -772,9 +764,9 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
                     if ((s = dbg->after_iter(k, (k + 1) % 2 ? jobs[0].JB : jobs[0].J, jobs[0].I)) != PK_OK) return s;
                 }
             } else {
-                pk_program_add(prog, PK_STEP_Y, Y_RLFINAL, with([&](VolDesc& d, DeconJob& j, int i) {
+                pk_program_add(prog, PK_STEP_Y, Y_RLFINAL, with([&](VolDesc& d, DeconJob& j, int) {
                     d.Yb = k == 1 ? j.I : j.Yb;
-                    set_post_job(d, p, mask_mode[i], j);
+                    set_post_job(d, p, mask_mode, j);
                 }));
             }
         }
@@ -782,7 +774,7 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
     if (dbg) {   // the last estimate is materialised: post-process it into the output
         if ((s = flush()) != PK_OK) return s;
         VolDesc f = base[0];
-        set_post_job(f, p, mask_mode[0], jobs[0]);
+        set_post_job(f, p, mask_mode, jobs[0]);
         const float* Jlast = method == 1 ? jobs[0].J : ((numit + 1) % 2 ? jobs[0].JB : jobs[0].J);
         k_post_from<<<grid_for((long long)f.nrows * f.ny), 256, 0, st>>>(f, Jlast);
         PK_CUDA(cudaGetLastError());
@@ -799,7 +791,7 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
                     prog.steps[ns - 2].kind == PK_STEP_X && prog.steps[ns - 2].mode == XZ_INV &&
                     prog.steps[ns - 1].kind == PK_STEP_Y &&
                     (prog.steps[ns - 1].mode == Y_FINAL || prog.steps[ns - 1].mode == Y_RLFINAL) &&
-                    !prog.descs[prog.steps[ns - 1].desc_off].need_xz;
+                    !prog.descs[prog.steps[ns - 1].desc_off].crop;
     if (!stream_io) {
         if (io && !io_uploaded) {   // decided late: whole-volume upload before the program
             const size_t N = (size_t)j0.rdims[0] * j0.rdims[1] * j0.rdims[2];

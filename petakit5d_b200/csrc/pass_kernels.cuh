@@ -69,7 +69,7 @@ struct VoxFields {
     float bg_f;
     float *I, *Jn, *Yb, *J4, *J2n, *dst;
     uint8_t* mask8;
-    int write_mask, rl_first, mask_mode, erosion, scale_mode, save16, crop, need_xz;
+    int write_mask, rl_first, mask_mode, scale_mode, save16, crop;
     float damp, scale, offset;
     void* out;
     int bb0[3], bb1[3];
@@ -77,8 +77,8 @@ struct VoxFields {
     __device__ __forceinline__ explicit VoxFields(const VolDesc& d)
         : ny(d.ny), nx(d.nx), nz(d.nz), nrows(d.nrows), raw(d.raw), raw_type(d.raw_type), bg16(d.bg16),
           bg_f(d.bg_f), I(d.I), Jn(d.Jn), Yb(d.Yb), J4(d.J4), J2n(d.J2n), dst(d.dst), mask8(d.mask8),
-          write_mask(d.write_mask), rl_first(d.rl_first), mask_mode(d.mask_mode), erosion(d.erosion),
-          scale_mode(d.scale_mode), save16(d.save16), crop(d.crop), need_xz(d.need_xz), damp(d.damp),
+          write_mask(d.write_mask), rl_first(d.rl_first), mask_mode(d.mask_mode),
+          scale_mode(d.scale_mode), save16(d.save16), crop(d.crop), damp(d.damp),
           scale(d.scale), offset(d.offset), out(d.out), chk(d.chk) {
         for (int i = 0; i < 3; i++) {
             rdims[i] = d.rdims[i];
@@ -89,9 +89,9 @@ struct VoxFields {
 };
 
 // Value of one voxel after the post-processing of decon_lucy_omw_function.m:146-177 (damping, then
-// scaling with offset and mask); x/z only matter to the border-erosion mask.
+// scaling with offset and mask).
 template <class D>
-__device__ __forceinline__ float post_value(const D& d, float J, long long vi, int x, int y, int z) {
+__device__ __forceinline__ float post_value(const D& d, float J, long long vi) {
     if (d.damp > 1.f) {
         const float dI = __fmul_rn(d.damp, d.I[vi]);
         const float a = (J <= dI) ? J : 0.f;
@@ -101,13 +101,7 @@ __device__ __forceinline__ float post_value(const D& d, float J, long long vi, i
     if (d.scale_mode == 1) {
         J = __fmul_rn(J, d.scale);
     } else if (d.scale_mode == 2) {
-        int m = 1;
-        if (d.mask_mode == 1 || d.mask_mode == 3) m = d.mask8[vi] != 0;
-        else if (d.mask_mode == 2) {
-            const int E = d.erosion;
-            m = d.mask8[vi] != 0 && y >= E && y < d.ny - E && x >= E && x < d.nx - E &&
-                (d.nz == 1 || (z >= E && z < d.nz - E));          // one plane: MATLAB's 2-D case
-        }
+        const int m = d.mask_mode ? d.mask8[vi] != 0 : 1;
         J = __fmul_rn(__fadd_rn(__fmul_rn(J, d.scale), d.offset), (float)m);
     }
     return J;
@@ -151,16 +145,16 @@ __device__ __forceinline__ bool rows_meet_box(const VolDesc& d, long long row0, 
 }
 
 // post-processing of one voxel and the cropped store.  x/z of the row are only derived when a crop
-// box or the border-erosion mask needs them.
+// box needs them.
 template <class D>
 __device__ __forceinline__ void post_store(const D& d, float J, long long row, int y) {
     const long long vi = row * d.ny + y;
     int x = 0, z = 0;
-    if (d.need_xz) {
+    if (d.crop) {
         row_xz(d, row, x, z);
         if (!in_box(d, x, y, z)) return;
     }
-    out_store(d, post_value(d, J, vi, x, y, z), vi, x, y, z);
+    out_store(d, post_value(d, J, vi), vi, x, y, z);
 }
 
 __device__ __forceinline__ bool mode_from_spec(int m) {
@@ -576,7 +570,7 @@ __global__ void __launch_bounds__(PK_THREADS, GEN >= 2 ? 2 : 3) k_y(const VolDes
         // per-voxel loop below, so their code is not unrolled into this one
         constexpr bool kPostMode = mode == Y_FINAL || mode == Y_RLFINAL;
         const bool fuse_ok = !odd && !(mode == Y_PRE && raw_sync) &&
-                             !(kPostMode && (d.damp > 1.f || d.scale_mode != 0 || d.need_xz));
+                             !(kPostMode && (d.damp > 1.f || d.scale_mode != 0 || d.crop));
         if (fuse_ok) {
             // The per-voxel phase runs on the registers that the inverse transform's last stage leaves; the
             // forward transform's first stage takes them from there where it has the same radix, else through

@@ -47,7 +47,7 @@ __host__ __device__ constexpr size_t yreg_smem_bytes(int mode) {
     return 128 + sizeof(float2) * ((size_t)y_naux(mode) * 4096 + (size_t)(4096 + 4096 / 16 + 1 + 1) + (256 + 32) + 258) + 16;
 }
 
-// Post-processing here is scaling, offset and a byte mask; damping, crops and the border mask take the
+// Post-processing here is scaling, offset and a byte mask; damping and crops take the
 // rolled kernel (the host's choice).
 template <int P, int MODE>
 __global__ void __launch_bounds__(PK_THREADS, y_naux(MODE) == 2 ? 2 : 3)

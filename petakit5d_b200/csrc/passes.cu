@@ -187,12 +187,12 @@ const pkpass::GenKernel& gen_kernel() {
 
 // A y step's descriptor the register-packing kernel can take: 512-voxel rows on the 4096-point
 // tiles, per-voxel inputs 16-byte aligned (bulk copies), the rolled kernel's fused-path conditions
-// (no padded / float64 raw input, no damping, border mask or crop in the final pass; with a byte mask
+// (no padded / float64 raw input, no damping or crop in the final pass; with a byte mask
 // and offset it takes 0.54 ms on 512x1140x270, the rolled kernel 0.89 ms).
 bool yreg_ok(const VolDesc& d, int mode) {
     auto al = [](const void* p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (d.odd || d.ny != 512 || d.M != 256 || d.tiles_small || !d.tw_rc) return false;
-    const bool post = !(d.damp > 1.f || d.need_xz) && (reinterpret_cast<uintptr_t>(d.mask8) & 1) == 0;
+    const bool post = !(d.damp > 1.f || d.crop) && (reinterpret_cast<uintptr_t>(d.mask8) & 1) == 0;
     switch (mode) {
         case Y_PRE: return !d.padded && (d.raw_type == PK_U16 || d.raw_type == PK_F32) && al(d.raw);
         case Y_R2C: return al(d.src);

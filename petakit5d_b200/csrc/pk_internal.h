@@ -117,13 +117,12 @@ struct VolDesc {
     // pre / post
     float bg_f; int bg16;
     uint8_t* mask8; int write_mask;  // Y_PRE: write raw ~= 0
-    unsigned int* zero_count;        // Y_PRE: number of raw zeros (erosion branch choice)
-    int mask_mode;                   // post: 0 none, 1 mask8 as is, 2 full-mask border erosion, 3 mask8 eroded
-    float damp; float scale; float offset; int erosion; int scale_mode; // scale_mode: 0 none, 1 scale, 2 (J*s+o)*mask
+    unsigned int* zero_count;        // Y_PRE: number of raw zeros (the erosion kernels choose by it)
+    int mask_mode;                   // post: 0 none, 1 mask8 (eroded where EdgeErosion asks for it)
+    float damp; float scale; float offset; int scale_mode; // scale_mode: 0 none, 1 scale, 2 (J*s+o)*mask
     int save16; void* out;
     int bb0[3], bb1[3];              // 0-based inclusive crop box (y, x, z)
     int crop;                        // crop box smaller than the volume
-    int need_xz;                     // post needs x/z of a voxel (crop or border erosion)
     int tiles_small;                 // passes use the 1024-point-tile kernels (small volumes)
     int* chk;                        // bounds-checked build (-DPK_CHECK): where a failed index check is recorded
 };
