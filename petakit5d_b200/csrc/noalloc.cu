@@ -278,10 +278,10 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
             g_kt.y[plan][mode]<<<hv.blocksY, PK_THREADS, smem, st>>>(ddesc + di, dprefix, 1, mode);
         } else if (gen[ax - 1]) {
             const AxisDev& a = *axes[ax];
-            const size_t gs = pkpass::gen_smem(a.gen_land, a.gen_work);
+            const size_t gs = pkpass::gen_smem(a.gen_buf);
             const int q = hv.S == S ? 0 : hv.S == OF ? 1 : 2;
             g_gen.fn[a.gen_big]<<<pk_mixed_grid(cnt[2 + ax], a.gen_big, gs), pkpass::kGenThreads, gs, st>>>(
-                ddesc + di, &dmix->map[ax - 1][q], dprefix + 4 + 2 * ax, 1, ax, mode, a.gen_land, a.gen_work, nullptr);
+                ddesc + di, &dmix->map[ax - 1][q], dprefix + 4 + 2 * ax, 1, ax, mode, a.gen_buf, nullptr);
         } else {
             g_kt.xz[plan]<<<ax == 1 ? hv.blocksX : hv.blocksZ, PK_THREADS, smem, st>>>(ddesc + di, dprefix + 2 * ax, 1, ax, mode);
         }

@@ -21,21 +21,20 @@ namespace pkpass {
 
 constexpr int kGenThreads = 256;
 
-// Elements of a tile's landing buffer and of each of its two stage buffers (whole boxes: the result
+// Elements of each of a tile's three buffers, for landing and for the stages (whole boxes: the result
 // leaves from a stage buffer box by box), in multiples of 128 bytes; a launch takes the largest of its volumes.
-inline int gen_land(const GenAxis& A) { return (A.T * A.rows * A.nbox + 15) & ~15; }
-inline int gen_work(const GenAxis& A) { return (A.T * A.rows * A.nbox + 15) & ~15; }
-inline size_t gen_smem(int land, int work) { return 256 + sizeof(float2) * ((size_t)land + 2 * (size_t)work); }
+inline int gen_buf(const GenAxis& A) { return (A.T * A.rows * A.nbox + 15) & ~15; }
+inline size_t gen_smem(int buf) { return 256 + sizeof(float2) * 3 * (size_t)buf; }
 
 struct GenKernel {   // [0]: radices up to 16, [1]: up to 31
-    void (*fn[2])(const VolDesc*, const XZMaps*, const int*, int, int, int, int, int, int*);
+    void (*fn[2])(const VolDesc*, const XZMaps*, const int*, int, int, int, int, int*);
 };
 
 #ifdef PK_GEN_KERNEL   // instantiated in one file
 template <bool BIG>
 __global__ void __launch_bounds__(kGenThreads, BIG ? 2 : 3)
     k_xzg(const VolDesc* __restrict__ descs, const XZMaps* __restrict__ maps, const int* __restrict__ prefix, int nvol,
-          int axis, int mode, int land, int work, int* err) {
+          int axis, int mode, int buf, int* err) {
     extern __shared__ unsigned char graw[];
     unsigned char* sm = graw + ((128 - (pktma::smem_u32(graw) & 127)) & 127);
     uint64_t* bar = (uint64_t*)sm;
@@ -77,8 +76,8 @@ __global__ void __launch_bounds__(kGenThreads, BIG ? 2 : 3)
     __syncthreads();
 
     float2* const in = (float2*)sm;
-    float2* const w0 = in + land;
-    float2* const w1 = w0 + work;
+    float2* const w0 = in + buf;
+    float2* const w1 = w0 + buf;
     float2* busy = w1;   // the stage buffer that the previous tile's store reads
     uint32_t parity = 0;
     for (int g = blockIdx.x; g < total; g += gridDim.x, parity ^= 1) {

@@ -664,22 +664,19 @@ static void assign_gen(PkProgram& prog, PkStep& s, int axis) {
     s.gen = 0;
     const int big = s.plan - pkpass::kMixedXZ;
     bool ok = gen_kernel().fn[big];
-    int land = 0, work = 0;
+    int buf = 0;
     for (int i = 0; i < s.nvol && ok; i++) {
         const VolDesc& d = prog.descs[s.desc_off + i];
-        const AxisDev& A = axis == 1 ? d.ax : d.az;
         ok = pk_mixed_map(d, axis, &prog.maps[s.desc_off + i]);
-        land = std::max(land, A.gen_land);
-        work = std::max(work, A.gen_work);
+        buf = std::max(buf, (axis == 1 ? d.ax : d.az).gen_buf);
     }
     if (!ok) return;
     int* pf = prog.prefix.data() + s.prefix_off;
     for (int i = 0; i < s.nvol; i++) pf[i + 1] = pf[i] + pk_mixed_tiles(prog.descs[s.desc_off + i], axis);
     s.grid = pf[s.nvol];
     s.gen = 1 + big;
-    s.tma_smem = pkpass::gen_smem(land, work);
-    s.gen_land = land;
-    s.gen_work = work;
+    s.tma_smem = pkpass::gen_smem(buf);
+    s.gen_buf = buf;
     s.tma_grid = pk_mixed_grid(s.grid, big, s.tma_smem);
 }
 
@@ -959,7 +956,7 @@ int gen_tile(int n, GenAxis* g) {
             g->rows = ((n + g->nbox - 1) / g->nbox + gran - 1) / gran * gran;
             if (g->rows <= 256) break;
         }
-        const size_t smem = pkpass::gen_smem(pkpass::gen_land(*g), pkpass::gen_work(*g));
+        const size_t smem = pkpass::gen_smem(pkpass::gen_buf(*g));
         if (smem <= (T > 4 ? (size_t)75 * 1024 : (size_t)226 * 1024)) {
             for (g->lt = 0; (1 << g->lt) < T;) g->lt++;
             return T;
@@ -1195,10 +1192,7 @@ static bool choose_axis(int n, bool sums, bool matrices, AxisDev* a, F&& smem) {
     a->gen_big = g.big;
     a->genT = g.T;
     a->gen_rows = g.rows;
-    if (g.T) {
-        a->gen_land = pkpass::gen_land(g);
-        a->gen_work = pkpass::gen_work(g);
-    }
+    if (g.T) a->gen_buf = pkpass::gen_buf(g);
     return true;
 }
 
@@ -1468,7 +1462,7 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
                 dd, prog.d_maps + s.desc_off, dp, s.nvol, ctx ? ctx->d_err : nullptr);
         } else if (s.gen) {
             gen_kernel().fn[s.gen - 1]<<<s.tma_grid, pkpass::kGenThreads, s.tma_smem, st>>>(
-                dd, prog.d_maps + s.desc_off, dp, s.nvol, s.kind == PK_STEP_X ? 1 : 2, s.mode, s.gen_land, s.gen_work,
+                dd, prog.d_maps + s.desc_off, dp, s.nvol, s.kind == PK_STEP_X ? 1 : 2, s.mode, s.gen_buf,
                 ctx ? ctx->d_err : nullptr);
         } else if (s.yreg) {
             yreg_kernels()->k[s.mode]<<<s.grid, kThreads, s.yreg_smem, st>>>(dd, dp, s.nvol, ctx ? ctx->d_err : nullptr);
@@ -1516,9 +1510,9 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
         void* args2[] = {(void*)&dd, (void*)&nvol};
         void* argst[] = {(void*)&dd, (void*)&dm, (void*)&dp, (void*)&nvol, (void*)&de};
         void* argsy[] = {(void*)&dd, (void*)&dp, (void*)&nvol, (void*)&de};
-        int land = s.gen_land, work = s.gen_work;
-        void* argsg[] = {(void*)&dd, (void*)&dm, (void*)&dp, (void*)&nvol, (void*)&axis, (void*)&mode, (void*)&land,
-                         (void*)&work, (void*)&de};
+        int buf = s.gen_buf;
+        void* argsg[] = {(void*)&dd, (void*)&dm, (void*)&dp, (void*)&nvol, (void*)&axis, (void*)&mode, (void*)&buf,
+                         (void*)&de};
         cudaKernelNodeParams p = {};
         p.blockDim = dim3(kThreads);
         p.gridDim = dim3(s.grid);
@@ -1680,8 +1674,8 @@ pk_status pk_program_launch(pk_ctx* ctx, PkProgram& prog, cudaStream_t st) {
         key.push_back((long long)prog.prefix.size());
         for (const PkStep& s : prog.steps) {
             const long long v[] = {s.kind, s.mode, s.plan, s.nvol, s.grid, (long long)s.smem, s.desc_off, s.prefix_off,
-                                   s.tma, s.tma_var, s.tma_grid, s.yreg, s.conv3, s.gen, s.gen_land, s.gen_work};
-            key.insert(key.end(), v, v + 16);
+                                   s.tma, s.tma_var, s.tma_grid, s.yreg, s.conv3, s.gen, s.gen_buf};
+            key.insert(key.end(), v, v + 15);
         }
         auto it = ctx->graphs.find(key);
         if (it == ctx->graphs.end() && ctx->graph_seen.size() >= 4096) ctx->graph_seen.clear();  // bounded
@@ -1856,7 +1850,7 @@ extern "C" int32_t pk_plan_read(const int64_t dims[3], char* buf, int32_t cap) {
         const bool tile = kind != PK_STEP_Y && a.engine == AE_MIXED;
         const int* rad = a.engine == AE_PLAN ? kPlans[a.plan].rad : a.engine == AE_MIXED ? mixed_plan(a.n).rad : a.rad;
         const int nst = a.engine == AE_PLAN ? kPlans[a.plan].nst : a.engine == AE_MIXED ? mixed_plan(a.n).nst : a.nst;
-        const size_t smem = tile ? pkpass::gen_smem(a.gen_land, a.gen_work) : pk_step_smem(kind, kind == PK_STEP_Y ? (int)Y_RLUPD : (int)XZ_CONV, d);
+        const size_t smem = tile ? pkpass::gen_smem(a.gen_buf) : pk_step_smem(kind, kind == PK_STEP_Y ? (int)Y_RLUPD : (int)XZ_CONV, d);
         js += std::string(js.size() > 1 ? ", " : "") + "{\"n\": " + std::to_string(a.n) + ", \"engine\": \"" + names[a.engine] +
               "\", \"radices\": [";
         for (int i = 0; i < nst; i++) js += (i ? ", " : "") + std::to_string(rad[i]);

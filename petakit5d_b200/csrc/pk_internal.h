@@ -67,7 +67,7 @@ struct AxisDev {
     int engine;       // AxisEngine
     const GenAxis* gen;   // AE_MIXED, AE_SUMS: the length's run-time plan and tables (device)
     int genT, gen_rows;         // its T and rows, and an x / z tile's buffers (pass_gen.cuh)
-    int gen_land, gen_work, gen_big;
+    int gen_buf, gen_big;
     int gen_direct;             // AE_SUMS: lines per tile (32, 16, 8 or 4)
 };
 
@@ -290,8 +290,8 @@ struct PkStep {
     int yreg = 0;
     size_t yreg_smem = 0;
     // set at upload: this x / z step of a length without a plan runs the generic TMA kernel (pass_gen.cuh)
-    // (1: radices up to 16, 2: all) on buffers of these sizes
-    int gen = 0, gen_land = 0, gen_work = 0;
+    // (1: radices up to 16, 2: all) on buffers of this size
+    int gen = 0, gen_buf = 0;
 };
 struct PkProgram {
     std::vector<VolDesc> descs;
