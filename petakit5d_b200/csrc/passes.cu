@@ -1094,17 +1094,43 @@ size_t pk_mixed_tables(int n, GenAxis* g, float2* out) {
     return gen_tables(g, out);
 }
 
-// Lines (32 to 4) per tile of a length with a prime factor above 31, as many as their shared memory smem(lines)
-// allows; the register radices of the in-place engine take 4096 points at most.  0: none, the plain engine (4
-// lines of 999 = 27 * 37 were 5% slower than it).
+// Lines (32, 16, 8 or 4) per tile of a length with a prime factor above 31, or 0 for the plain engine, for `outer` groups
+// of `count` lines (columns of a plane, all rows in y); smem(lines): a tile's shared memory.  Both engines form the same
+// sums.  As many lines as fit win wherever there are twice that many (x 111 of 111 x 56 columns: plain 54 us, 8 a
+// tile 50, 32 a tile 33).  Where there are fewer, a tile's missing lines cost as much as others, and a plain tile holds
+// what there is: the faster is taken, in units of the plain engine's rounds (each of its threads forms one output a
+// round).  A tile of the sums takes 4 + 4.2 I of them, I = its work items over the threads (1.5 more beside a
+// register radix), and no less than about 5 when the GPU has little else.  Measured, plain / sums: x 101 of 1500 planes,
+// 10 columns 138 / 177 us (16 a tile), 24 columns 302 / 246 us (32); x 467, 3 columns 729 / 726 us (4), 8 columns
+// 1856 / 1009 us (8); 2 rows of 467 163 / 228 us, 12 rows 589 / 236 us.  The register radices of the in-place engine
+// take 4096 points at most (4 lines of 999 = 27 * 37 were 5% slower than the plain engine).
 template <class F>
-static int direct_lines(const AxisDev& a, F&& smem) {
+static int direct_lines(const AxisDev& a, long long count, long long outer, F&& smem) {
     bool small = false;
-    for (int s = 0; s < a.nst; s++) small |= a.rad[s] <= 5 || a.rad[s] == 8 || a.rad[s] == 16;
+    int R = 1, most = 0;
+    for (int s = 0; s < a.nst; s++) {
+        small |= a.rad[s] <= 5 || a.rad[s] == 8 || a.rad[s] == 16;
+        R = std::max(R, a.rad[s]);
+    }
+    const int least = small ? 8 : 4;
     for (size_t lim : {(size_t)112 * 1024, (size_t)pkpass::kDirectSmem})   // two CTAs an SM, else one
-        for (int c : {32, 16, 8, 4})
-            if ((!small || (c >= 8 && c * a.n <= PK_TILE_POINTS)) && smem(c) <= lim) return c;
-    return 0;
+        for (int c = 32; c >= least && !most; c /= 2)
+            if ((!small || c * a.n <= PK_TILE_POINTS) && smem(c) <= lim) most = c;
+    if (!most || count >= 2 * most) return most;
+    const double slots = 2.0 * sm_count();
+    auto ceil_div = [](long long x, long long y) { return (x + y - 1) / y; };
+    const long long tp = std::max<long long>(1, std::min<long long>(PK_TILE_POINTS / a.n, count));
+    double best = (double)ceil_div(tp * a.n, PK_THREADS) * std::max(1.0, ceil_div(count, tp) * outer / slots);
+    int lines = 0;
+    for (int c = most; c >= least; c /= 2) {
+        const double items = (double)(a.n / R) * (c / 4) * ((R + 3) / 4) / PK_THREADS;
+        const double t = std::max(4.5 * std::ceil(items) + items, ((small ? 5.5 : 4.0) + 4.2 * items) * ceil_div(count, c) * outer / slots);
+        if (t <= best) {
+            best = t;
+            lines = c;
+        }
+    }
+    return lines;
 }
 
 // Root matrices a context keeps (8 n^2 bytes for a prime n: 1.7 MB at 467, 33 MB at 2039): regions drawn by hand bring
@@ -1160,10 +1186,10 @@ static pk_status pk_get_gen(pk_ctx* ctx, const AxisDev& a, const GenAxis** dev) 
     return PK_OK;
 }
 
-// Host part of an axis: its engine, stages and tile.  `sums`: the volume has a prime factor above 31; smem(a): shared
-// memory of a tile of a.gen_direct lines.
+// Host part of an axis: its engine, stages and tile.  `sums`: the volume has a prime factor above 31; count, outer: its
+// lines (direct_lines); smem(a): shared memory of a tile of a.gen_direct lines.
 template <class F>
-static bool choose_axis(int n, bool sums, bool matrices, AxisDev* a, F&& smem) {
+static bool choose_axis(int n, bool sums, bool matrices, long long count, long long outer, AxisDev* a, F&& smem) {
     AxisPlan p;
     if (!pk_make_axis_plan(n, &p)) return false;
     memset(a, 0, sizeof(*a));
@@ -1179,7 +1205,7 @@ static bool choose_axis(int n, bool sums, bool matrices, AxisDev* a, F&& smem) {
         if (!matrices || gen_smooth(n) || n > kDirectMax) return true;
         AxisDev t = *a;
         t.engine = AE_SUMS;
-        t.gen_direct = direct_lines(*a, [&](int c) {
+        t.gen_direct = direct_lines(*a, count, outer, [&](int c) {
             t.gen_direct = c;
             return smem(t);
         });
@@ -1225,12 +1251,14 @@ pk_status pk_geometry(int ny, int nx, int nz, VolDesc* d, bool matrices) {
         t.Ly = a.gen_direct;
         return pk_step_smem(PK_STEP_Y, Y_RLUPD, t);
     };
-    for (const auto& [n, a] : {std::make_pair(nx, &d->ax), std::make_pair(nz, &d->az)})
-        if (!choose_axis(n, sums, matrices, a, xz_smem))
+    for (AxisDev* a : {&d->ax, &d->az}) {
+        const int n = a == &d->ax ? nx : nz, outer = a == &d->ax ? nz : nx;
+        if (!choose_axis(n, sums, matrices, d->Py, outer, a, xz_smem))
             return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(n) + " needs too many radix stages");
+    }
     for (AxisDev* a : {&d->ax, &d->az})
         if (a->engine == AE_MIXED && !a->genT) a->engine = AE_PLAIN;   // no tile fits
-    if (!choose_axis(d->M, sums, matrices, &d->ay, y_smem))
+    if (!choose_axis(d->M, sums, matrices, d->nrows, 1, &d->ay, y_smem))
         return pk_fail(PK_ERR_UNSUPPORTED, "transform length " + std::to_string(d->M) + " needs too many radix stages");
     if (d->ay.engine == AE_MIXED) {   // odd rows run in pairs
         d->Ly = (d->odd ? 2 : 1) * std::max(1, P / d->M);

@@ -84,6 +84,14 @@ def test_one_engine_for_a_volume():
     assert [a["engine"] for a in plan(512, 37, 256)] == ["plan", "sums", "plan"]
 
 
+def test_few_lines_beside_a_large_prime():
+    # a tile's missing lines cost as much as others: fewer lines a tile where there are few, the plain engine (which has
+    # tiles of what there is) where they are fewer still
+    assert [plan(ny, 126, 233)[2]["engine"] for ny in (3, 400)] == ["plain", "sums"]
+    assert plan(6, 467, 60)[1]["lines"] == 4 and plan(300, 467, 60)[1]["lines"] == 8
+    assert plan(101, 1, 1)[0]["engine"] == "plain" and plan(101, 100, 1)[0]["engine"] == "sums"
+
+
 def test_refused_extents():
     for dims in ((0, 1, 1), (1, 4097, 1), (8194, 1, 1), (4097, 1, 1)):
         assert _lib.lib.pk_plan_read(_lib.i64x3(dims), None, 0) < 0

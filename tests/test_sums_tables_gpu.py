@@ -1,5 +1,8 @@
 """Root matrices of lengths with a prime factor above 31: a context keeps a bounded amount, gives them back on reset, and
 where it keeps none the plain engine forms the same sums."""
+import ctypes as C
+import json
+
 import numpy as np
 import pytest
 
@@ -27,9 +30,21 @@ def _free():
     return torch.cuda.mem_get_info()[0]
 
 
+# tiles of 32, 16, 8 and 4 lines, whole and partly filled, lengths of one and of several prime factors, on each axis
+SHAPES = [(82, 41, 38), (130, 37, 43), (70, 233, 3), (129, 467, 5), (140, 613, 2), (6, 467, 60), (26, 101, 40), (118, 74, 6),
+          (202, 9, 5), (222, 66, 5), (301, 9, 5), (74, 1, 40), (66, 74, 1), (467, 3, 2)]
+
+
+def _engines(shape):
+    buf = C.create_string_buffer(4096)
+    assert _lib.lib.pk_plan_read(_lib.i64x3(shape), buf, len(buf)) > 0
+    return [a["engine"] for a in json.loads(buf.value)]
+
+
 @pytest.mark.parametrize("method,numit", [("omw", 2), ("rl", 4)])
-@pytest.mark.parametrize("shape", [(45, 37, 19), (74, 41, 38), (82, 40, 43), (129, 467, 5), (66, 74, 1), (1006, 20, 9)])
+@pytest.mark.parametrize("shape", SHAPES)
 def test_same_results_without_the_matrices(shape, method, numit, monkeypatch):
+    assert "sums" in _engines(shape)
     ctx = _lib.Context(0)
     ref = _decon(method, shape, ctx, numit)
     ctx.close()
