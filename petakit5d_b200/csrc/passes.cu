@@ -1514,6 +1514,26 @@ static pk_status launch_steps(pk_ctx* ctx, const PkProgram& prog, cudaStream_t s
     return PK_OK;
 }
 
+// Whether pass `s` starts while pass `p` before it runs (a programmatic edge), so that its start hides behind it.  Its
+// early CTAs take the slots that are free, so a grid of less than a wave ends up three to an SM beside empty SMs:
+// between long passes that costs more than the gap.  Compile-time plans: below 128 MB of algorithmic traffic, about 20 us
+// (128x128x64 RL 1.11 -> 0.96 ms, a 2048x2048 plane 4.13 -> 3.88 ms; 1024x1024x512 OMW 23.9 -> 26.6 ms).  Mixed
+// radices take longer for their bytes: 6 MB (99x88x27 OMW 157 -> 151 us, 120x77x184 228 -> 234 us, 512x1140x270 10.3 ->
+// 11.4 ms).  Plain sums are bound by arithmetic: where both grids fit one CTA to an SM (101x1x1 RL 176 -> 161 us; else
+// 250x250x37 OMW 630 -> 810 us, 41x512x256 1.21 -> 1.49 ms).
+static bool early_start(const PkProgram& prog, const PkStep& p, const PkStep& s) {
+    bool sums = false, brief = true;
+    for (const PkStep* q : {&p, &s}) {
+        if (q->kind == PK_STEP_CONV3) return false;
+        if (q->kind == PK_STEP_LAMBDA) continue;
+        const VolDesc* d = prog.descs.data() + q->desc_off;
+        const int engine = (q->kind == PK_STEP_Y ? d->ay : q->kind == PK_STEP_X ? d->ax : d->az).engine;   // one a step
+        sums = sums || engine == AE_PLAIN || engine == AE_SUMS;
+        brief = brief && pk_step_bytes(*q, d) < (engine == AE_MIXED ? 6e6 : 128e6);
+    }
+    return sums ? p.grid + s.grid <= sm_count() : brief;
+}
+
 // The program's launches as a graph of kernel nodes in launch order, built node by node (no stream
 // capture, so other threads' CUDA calls cannot disturb it).
 
@@ -1525,7 +1545,8 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
     cudaGraph_t g = nullptr;
     if (cudaGraphCreate(&g, 0) != cudaSuccess) { cudaGetLastError(); return false; }
     cudaGraphNode_t prev = nullptr;
-    bool ok = true, prev_brief = false;
+    bool ok = true;
+    const PkStep* before = nullptr;
     for (const PkStep& s : prog.steps) {
         if (s.grid == 0) continue;
         const VolDesc* dd = d_desc + s.desc_off;
@@ -1583,13 +1604,8 @@ static bool build_graph(const PkProgram& prog, const VolDesc* d_desc, const int*
             p.kernelParams = args2;
         }
         cudaGraphNode_t node = nullptr;
-        // between two short passes only (128 MB of algorithmic traffic, about 20 us, each): there the next one's
-        // start hides behind this one (128x128x64 RL 1.11 -> 0.96 ms, a 2048x2048 plane 4.13 -> 3.88 ms); on
-        // long ones the early CTAs cost more than the gap (1024x1024x512 OMW 23.9 -> 26.6 ms, 512x1140x270
-        // 10.3 -> 11.4 ms)
-        const bool brief = s.kind != PK_STEP_CONV3 && pk_step_bytes(s, prog.descs.data() + s.desc_off) < 128e6;
-        const bool edge = pdl && prev && brief && prev_brief;
-        prev_brief = brief;
+        const bool edge = pdl && prev && early_start(prog, *before, s);
+        before = &s;
         cudaError_t ea = cudaGraphAddKernelNode(&node, g, prev && !edge ? &prev : nullptr, prev && !edge ? 1 : 0, &p);
         if (ea == cudaSuccess && edge) {
             cudaGraphEdgeData ed = {};
