@@ -700,13 +700,21 @@ pk_status pk_decon_multi(pk_ctx* ctx, int method, std::vector<DeconJob>& jobs, p
     // passes took 75 us on a 2048 x 2048 plane, the z pass of length 1 the longest of them; this one takes 30),
     // whatever volumes the call holds beside them
     auto conv = [&](int which) {
-        std::vector<VolDesc> planes, vols;
-        for (const VolDesc& v : with([&](VolDesc& d, DeconJob& j, int) {
-                 if (method == 1) { d.otf = which ? j.otf_b : j.otf_f; d.conj = 0; }
-                 else { d.otf = j.otf_f; d.conj = which; }
-             }))
-            (v.nz == 1 ? planes : vols).push_back(v);
-        pk_program_add(prog, PK_STEP_X, XZ_CONV, planes);
+        std::vector<VolDesc> vols = with([&](VolDesc& d, DeconJob& j, int) {
+            if (method == 1) { d.otf = which ? j.otf_b : j.otf_f; d.conj = 0; }
+            else { d.otf = j.otf_f; d.conj = which; }
+        });
+        const auto plane = [](const VolDesc& d) { return d.nz == 1; };
+        const size_t np = std::count_if(vols.begin(), vols.end(), plane);
+        if (np == nj) {
+            pk_program_add(prog, PK_STEP_X, XZ_CONV, vols);
+            return;
+        }
+        if (np) {
+            const auto rest = std::stable_partition(vols.begin(), vols.end(), plane);
+            pk_program_add(prog, PK_STEP_X, XZ_CONV, std::vector<VolDesc>(vols.begin(), rest));
+            vols.erase(vols.begin(), rest);
+        }
         pk_program_add(prog, PK_STEP_X, XZ_FWD, vols);
         pk_program_add(prog, PK_STEP_Z, XZ_CONV, vols);
         pk_program_add(prog, PK_STEP_X, XZ_INV, vols);

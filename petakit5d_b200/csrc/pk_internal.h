@@ -86,7 +86,7 @@ enum YMode : int {
 
 enum XZMode : int { XZ_FWD = 0, XZ_INV = 1, XZ_CONV = 2, XZ_FWD_SCALE = 3 };
 
-struct VolDesc {
+struct alignas(64) VolDesc {   // a program's descriptors start on whole sectors
     // geometry
     int ny, nx, nz;
     int M;            // y-pass complex length: ny/2 (even ny) or ny (odd ny)
