@@ -1100,7 +1100,8 @@ size_t pk_mixed_tables(int n, GenAxis* g, float2* out) {
 // tile 50, 32 a tile 33).  Where there are fewer, a tile's missing lines cost as much as others, and a plain tile holds
 // what there is: the faster is taken, in units of the plain engine's rounds (each of its threads forms one output a
 // round).  A tile of the sums takes 4 + 4.2 I of them, I = its work items over the threads (1.5 more beside a
-// register radix), and no less than about 5 when the GPU has little else.  Measured, plain / sums: x 101 of 1500 planes,
+// register radix), and when the GPU has little else one round of its items takes 0.24 R us, 3 (R = 37) to 6 of the plain
+// engine's rounds of 0.0375 R + 1.3 us.  Measured, plain / sums: x 101 of 1500 planes,
 // 10 columns 138 / 177 us (16 a tile), 24 columns 302 / 246 us (32); x 467, 3 columns 729 / 726 us (4), 8 columns
 // 1856 / 1009 us (8); 2 rows of 467 163 / 228 us, 12 rows 589 / 236 us.  The register radices of the in-place engine
 // take 4096 points at most (4 lines of 999 = 27 * 37 were 5% slower than the plain engine).
@@ -1124,7 +1125,7 @@ static int direct_lines(const AxisDev& a, long long count, long long outer, F&& 
     int lines = 0;
     for (int c = most; c >= least; c /= 2) {
         const double items = (double)(a.n / R) * (c / 4) * ((R + 3) / 4) / PK_THREADS;
-        const double t = std::max(4.5 * std::ceil(items) + items, ((small ? 5.5 : 4.0) + 4.2 * items) * ceil_div(count, c) * outer / slots);
+        const double t = std::max(6.4 * R / (R + 35) * std::ceil(items) + items, ((small ? 5.5 : 4.0) + 4.2 * items) * ceil_div(count, c) * outer / slots);
         if (t <= best) {
             best = t;
             lines = c;
