@@ -1,7 +1,8 @@
 // Compile-time transform plans.  Each entry is a transform length and its radix sequence; the pass
 // kernels are instantiated once per entry, so every stage runs with constant radix, stride and
-// twiddle step (straight-line code, no register spills).  Lengths without an entry use plan 0,
-// the runtime-radix engine (any length, slower).
+// twiddle step (straight-line code, no register spills).  Lengths without an entry have plan 0 and run on
+// one of the run-time engines: mixed radices (gen_engine.cuh, prime factors up to 31), or the in-place engine with or
+// without register-tiled sums (fft_engine.cuh); AxisDev::engine says which.
 #pragma once
 
 #define PK_THREADS 256        // threads per pass CTA
