@@ -13,7 +13,7 @@
 //
 // Limits and sharing:
 //   * at most PK_NOALLOC_MAX_VOXELS voxels per volume (1,048,576, e.g. 128 x 128 x 64); larger
-//     volumes are rejected with PK_ERR_UNSUPPORTED.  The array (about 32.6 MB) is held on every
+//     volumes are rejected with PK_ERR_UNSUPPORTED.  The array (about 32.4 MB) is held on every
 //     GPU that loads the library until the process exits;
 //   * deconOffset and EdgeErosion (which need a mask volume) and NUMIT = 0 are rejected with
 //     PK_ERR_UNSUPPORTED; dampFactor, scaleFactor, save16bit and bbox are supported;
@@ -25,7 +25,9 @@
 //     the array's device address (cudaGetSymbolAddress, once per device, with that device
 //     current) and sets the kernels' shared-memory limits.  Both are kept for the life of the
 //     process: a program that resets a device (cudaDeviceReset) must not call this entry point on
-//     that device afterwards.
+//     that device afterwards;
+//   * lengths on the mixed-radix engine wait on their own TMA copies, each for a second at most; where
+//     one runs out, the output is filled with NaN (uint16: 65535).
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -103,6 +105,16 @@ __global__ void k_na_psf_scatter(const float* __restrict__ psf, int py, int px, 
         int tx = x - px / 2; if (tx < 0) tx += nx;
         int tz = z - pz / 2; if (tz < 0) tz += nz;
         vol[(long long)ty + (long long)ny * (tx + (long long)nx * tz)] = (float)((double)psf[i] / s);
+    }
+}
+
+// A bounded device wait that ran out (tma.cuh) leaves *failed set: there is no context to report it, so the output is
+// overwritten with NaN or 65535.
+__global__ void k_na_failed(const int* failed, void* out, long long n, int u16) {
+    if (*(const volatile int*)failed == 0) return;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        if (u16) ((uint16_t*)out)[i] = 65535;
+        else ((float*)out)[i] = __int_as_float(0x7fffffff);
     }
 }
 
@@ -256,6 +268,7 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
         pf[2 * k] = 0;
         pf[2 * k + 1] = cnt[k];
     }
+    pf[10] = 0;   // a device wait ran out
 
     // ---- uploads (pageable sources are staged before the calls return, so the static staging
     //      area can be rewritten by the next call)
@@ -266,7 +279,7 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
     } while (0)
     NA_CUDA(cudaMemcpyAsync(twb, g_stage.tw, kTwBytes, cudaMemcpyHostToDevice, st));
     NA_CUDA(cudaMemcpyAsync(ddesc, g_stage.desc, sizeof(VolDesc) * kDescs, cudaMemcpyHostToDevice, st));
-    NA_CUDA(cudaMemcpyAsync(dprefix, g_stage.prefix, sizeof(int) * 10, cudaMemcpyHostToDevice, st));
+    NA_CUDA(cudaMemcpyAsync(dprefix, g_stage.prefix, sizeof(int) * 11, cudaMemcpyHostToDevice, st));
     if (v.ay.gen || v.ax.gen || v.az.gen)
         NA_CUDA(cudaMemcpyAsync(dmix, &g_stage.mixed, sizeof(Mixed), cudaMemcpyHostToDevice, st));
 
@@ -281,7 +294,7 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
             const size_t gs = pkpass::gen_smem(a.gen_buf);
             const int q = hv.S == S ? 0 : hv.S == OF ? 1 : 2;
             g_gen.fn[a.gen_big]<<<pk_mixed_grid(cnt[2 + ax], a.gen_big, gs), pkpass::kGenThreads, gs, st>>>(
-                ddesc + di, &dmix->map[ax - 1][q], dprefix + 4 + 2 * ax, 1, ax, mode, a.gen_buf, nullptr);
+                ddesc + di, &dmix->map[ax - 1][q], dprefix + 4 + 2 * ax, 1, ax, mode, a.gen_buf, dprefix + 10);
         } else {
             g_kt.xz[plan]<<<ax == 1 ? hv.blocksX : hv.blocksZ, PK_THREADS, smem, st>>>(ddesc + di, dprefix + 2 * ax, 1, ax, mode);
         }
@@ -322,6 +335,12 @@ extern "C" pk_status pk_decon_lucy_omw_noalloc(const void* d_in, pk_dtype in_typ
         if (it < numit) s = launch(PK_STEP_Y, Y_UPDATE, it == 1 ? D_UPD1 : D_UPDN);
         else s = launch(PK_STEP_Y, Y_FINAL, it == 1 ? D_FIN1 : D_FINN);
         if (s != PK_OK) return s;
+    }
+    if (gen[0] || gen[1]) {
+        const VolDesc& f = h[D_FINN];
+        const long long n = (long long)(f.bb1[0] - f.bb0[0] + 1) * (f.bb1[1] - f.bb0[1] + 1) * (f.bb1[2] - f.bb0[2] + 1);
+        k_na_failed<<<(int)std::min<long long>((n + 255) / 256, 148LL * 4), 256, 0, st>>>(dprefix + 10, d_out, n, f.save16);
+        NA_CUDA(cudaGetLastError());
     }
 #undef NA_CUDA
     return PK_OK;
